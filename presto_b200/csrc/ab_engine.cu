@@ -99,7 +99,7 @@ struct ab_ctx {
     DevBuf<int> bidx;                       // bank lists of the grouped preparation launches
     DevBuf<int> dd_cd, dd_off;              // dedispersion delays
     long long blu_M = 0;                    // the length blu_b was built for
-    DevBuf<int2> dered_blocks;
+    DevBuf<int4> dered_runs;                 // runs of equal de-reddening blocks
     DevBuf<float> dered_means;
     DevBuf<TcItem> titems;
     float2 *tmpl_p = nullptr;
@@ -1151,7 +1151,7 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->bidx.release();
     ctx->dd_cd.release();
     ctx->dd_off.release();
-    ctx->dered_blocks.release();
+    ctx->dered_runs.release();
     ctx->dered_means.release();
     ctx->titems.release();
     ctx->norms.release();
@@ -1395,18 +1395,16 @@ static int realfft_dev(ab_ctx *ctx, const float *series, long long n, int series
     if (pow2_fft_supported(M)) {
         CK(ctx->ser_scr.ensure((size_t) M));
         CK(launch_realfft(din, dout, ctx->ser_scr.p, n, ctx->stream));
-        ctx->launches += 6;
+        ctx->launches += M <= 8192 ? 2 : 3;
         return AB_OK;
     }
     const long long L = bluestein_len(M);
-    CK(ctx->ser_scr.ensure((size_t) L));
     CK(ctx->blu_a.ensure((size_t) L));
     const bool fresh = ctx->blu_M != M || ctx->blu_b.n < (size_t) L;
     CK(ctx->blu_b.ensure((size_t) L));
-    CK(launch_realfft_bluestein(din, dout, ctx->blu_a.p, ctx->ser_scr.p, ctx->blu_b.p, fresh, n,
-                                ctx->stream));
+    CK(launch_realfft_bluestein(din, dout, ctx->blu_a.p, ctx->blu_b.p, fresh, n, ctx->stream));
     ctx->blu_M = M;
-    ctx->launches += fresh ? 24 : 17;
+    ctx->launches += (L <= 8192 ? 2 : 4) + (fresh ? 2 : 0);
     return AB_OK;
 }
 
@@ -1415,20 +1413,24 @@ static int deredden_dev(ab_ctx *ctx, float2 *dfft, long long numbins, int startw
 {
     if (endwidth > AB_DERED_MAXW)
         return fail(ctx, AB_ERR_ARG, "deredden endwidth %d above %d", endwidth, AB_DERED_MAXW);
+    // at most one run per length up to AB_DERED_MAXW, the first two blocks, the
+    // cut-off last one and the sentinel
+    constexpr int kMaxRuns = AB_DERED_MAXW + 8;
+    std::vector<int4> runs(kMaxRuns);
     long long nb = 0;
-    int rc = ab_dered_plan(numbins, startwidth, endwidth, endfreq, T, nullptr, 0, &nb);
+    int nruns = 0, maxlen = 0;
+    int rc = ab_dered_runs(numbins, startwidth, endwidth, endfreq, T, &runs[0].x, kMaxRuns, &nruns, &nb,
+                           &maxlen);
     if (rc) return fail(ctx, rc, "deredden: spectrum of %lld bins too short", numbins);
     if (nb > (1LL << 30)) return fail(ctx, AB_ERR_ARG, "deredden: too many blocks");
-    std::vector<int> plan((size_t) (2 * nb));
-    ab_dered_plan(numbins, startwidth, endwidth, endfreq, T, plan.data(), nb, &nb);
-    CK(ctx->dered_blocks.ensure((size_t) nb));
+    CK(ctx->dered_runs.ensure(kMaxRuns));
     CK(ctx->dered_means.ensure((size_t) nb));
-    CK(cudaMemcpyAsync(ctx->dered_blocks.p, plan.data(), sizeof(int) * 2 * nb, cudaMemcpyHostToDevice,
+    // a pageable upload of a few KB: the copy has left the vector on return
+    CK(cudaMemcpyAsync(ctx->dered_runs.p, runs.data(), sizeof(int4) * (size_t) (nruns + 1),
+                       cudaMemcpyHostToDevice, ctx->stream));
+    CK(launch_deredden(dfft, ctx->dered_runs.p, nruns, (int) nb, maxlen, numbins, ctx->dered_means.p,
                        ctx->stream));
-    CK(launch_deredden(dfft, ctx->dered_blocks.p, (int) nb, ctx->dered_means.p, ctx->stream));
     ctx->launches += 2;
-    // the plan upload is pageable: wait before the vector goes away
-    CK(cudaStreamSynchronize(ctx->stream));
     return AB_OK;
 }
 

@@ -170,37 +170,48 @@ template <int L, int S> struct FftTw {
     float2 b2[4];                                   // pass 2: w = exp(S 2 pi i k / 256)
     float2 b3[SH::NB3 > 0 ? SH::NB3 : 1][NBASE3];   // pass 3: w = exp(S 2 pi i k / (256 R3))
     float2 b4[SH::NB4 > 0 ? SH::NB4 : 1];           // pass 4 (radix 2): w = exp(S 2 pi i k / L)
+    // w, w^2, w^4, ... from one FP64 root per butterfly and its squares (each
+    // squaring adds 1e-16, far below the FP32 rounding): sincospi costs as much
+    // as ten squarings, and a thread that runs one transform only would spend
+    // longer on ten roots than on its butterflies
+    static __device__ __forceinline__ void powers(double arg, float2 *out, int n)
+    {
+        double s, c;
+        sincospi(arg, &s, &c);
+#pragma unroll
+        for (int e = 0; e < n; e++) {
+            out[e] = make_float2((float) c, (float) (S * s));
+            const double c2 = (c - s) * (c + s);
+            s = 2.0 * c * s;
+            c = c2;
+        }
+    }
     __device__ __forceinline__ void init(int t)
     {
-        int k = t & 15;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            double s, c;
-            sincospi(2.0 * (double) (k << e) / 256.0, &s, &c);
-            b2[e] = make_float2((float) c, (float) (S * s));
-        }
+        powers(2.0 * (double) (t & 15) / 256.0, b2, 4);
         if constexpr (SH::R3 > 1) {
 #pragma unroll
-            for (int b = 0; b < SH::NB3; b++) {
-                int kk = (t + SH::NT * b) & 255;
-#pragma unroll
-                for (int e = 0; e < NBASE3; e++) {
-                    double s, c;
-                    sincospi(2.0 * (double) (kk << e) / (double) (256 * SH::R3), &s, &c);
-                    b3[b][e] = make_float2((float) c, (float) (S * s));
-                }
-            }
+            for (int b = 0; b < SH::NB3; b++)
+                powers(2.0 * (double) ((t + SH::NT * b) & 255) / (double) (256 * SH::R3), b3[b], NBASE3);
         }
         if constexpr (SH::R4 > 1) {
             static_assert(SH::R4 == 2, "fourth pass is radix 2");
 #pragma unroll
-            for (int b = 0; b < SH::NB4; b++) {
-                int kk = (t + SH::NT * b) & 4095;
-                double s, c;
-                sincospi(2.0 * (double) kk / (double) L, &s, &c);
-                b4[b] = make_float2((float) c, (float) (S * s));
-            }
+            for (int b = 0; b < SH::NB4; b++)
+                powers(2.0 * (double) ((t + SH::NT * b) & 4095) / (double) L, &b4[b], 1);
         }
+    }
+    // the twiddles of the transform in the other direction
+    __device__ __forceinline__ void conj_of(const FftTw<L, -S> &o)
+    {
+#pragma unroll
+        for (int e = 0; e < 4; e++) b2[e] = make_float2(o.b2[e].x, -o.b2[e].y);
+#pragma unroll
+        for (int b = 0; b < SH::NB3; b++)
+#pragma unroll
+            for (int e = 0; e < NBASE3; e++) b3[b][e] = make_float2(o.b3[b][e].x, -o.b3[b][e].y);
+#pragma unroll
+        for (int b = 0; b < SH::NB4; b++) b4[b] = make_float2(o.b4[b].x, -o.b4[b].y);
     }
 };
 

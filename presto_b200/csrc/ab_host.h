@@ -63,6 +63,8 @@ long long ab_num_preblocks(const ab_obs *obs);
 int  ab_w_resp_halfwidth(double z, double w);
 int  ab_dered_plan(long long numbins, int startwidth, int endwidth, double endfreq, double T,
                    int *blocks, long long maxblocks, long long *nblocks);
+int  ab_dered_runs(long long numbins, int startwidth, int endwidth, double endfreq, double T, int *runs,
+                   int maxruns, int *nruns, long long *nblocks, int *maxlen);
 int  ab_next_good_fftlen(int n);
 int  ab_fftlen_from_kernwidth(int kw);
 

@@ -7,16 +7,16 @@
 // untangling pass into n/2 bins with bin 0 = (DC, Nyquist).  For a
 // power-of-two M = n/2 the complex FFT is one radix-16 Stockham transform in
 // shared memory up to 8192 points, and above that a four-step transform
-// M = M1 M2: transpose, M2 transforms of length M1 multiplied by
-// exp(-2 pi i n2 k1 / M), transpose, M1 transforms of length M2, transpose
-// (each step one pass over HBM).  Any other even n (dedispersed series are
-// usually 2^a 3^b 5^c 7^d samples long) goes through Bluestein's chirp-z
-// transform on three power-of-two transforms of length >= 2M - 1.
+// M = M1 M2 in two passes over memory: strided columns with the inter-step
+// twiddles, then rows written in their transposed places.  Any other even n
+// (dedispersed series are usually 2^a 3^b 5^c 7^d samples long) goes through
+// Bluestein's chirp-z transform on power-of-two transforms of length
+// >= 2M - 1, fused into three passes.
 //
 // deredden: the block partition depends only on bin indices (lengths
-// startwidth ln(bin) up to endwidth), so the host plans it; one CTA per block
-// takes the exact median of its powers, then one CTA per segment between
-// block midpoints scales the bins by the reference's interpolated
+// startwidth ln(bin) up to endwidth), so the host plans it as runs of equal
+// blocks (some hundred); one warp per block takes the exact median of its
+// powers, then every bin is scaled by the reference's interpolated
 // normalisation with its fast inverse square root, in float with explicit
 // rounding, so the same input gives the reference's bits.
 #include <cuda_runtime.h>
@@ -25,57 +25,231 @@
 #include "ab_fft.cuh"
 #include "ab_kernels.h"
 #include "ab_norm.cuh"
-#include "ab_select.cuh"
 
 namespace ab {
 namespace {
 
+// W_M^{S j} for 0 <= j < M
+template <int S> __device__ __forceinline__ double2 root(long long j, double invM)
+{
+    double s, c;
+    sincospi(2.0 * S * ((double) j * invM), &s, &c);
+    return make_double2(c, s);
+}
+
+// v[m] *= W_M^{S a (t + NT m)}, m = 0..15 (a, t + NT m < 2^13, M a power of
+// two: a (t + NT m) / M is exact): two FP64 roots and their products instead
+// of sixteen roots; fifteen FP64 products stay far below the FP32 rounding.
+template <int S>
+__device__ __forceinline__ void step_twiddles(float2 (&v)[16], int a, int t, int NT, long long M)
+{
+    const double inv = 1.0 / (double) M;
+    double2 w = root<S>((long long) a * t, inv);
+    const double2 q = root<S>((long long) a * NT, inv);
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const float cr = (float) w.x, ci = (float) w.y;
+        v[m] = make_float2(v[m].x * cr - v[m].y * ci, v[m].x * ci + v[m].y * cr);
+        w = dmul(w, q);
+    }
+}
+
+// Bluestein's chirp-z transform for any length M: with c_j = exp(i pi j^2 / M),
+// X_k = conj(c_k) sum_j (x_j conj(c_j)) c_{k-j}, a linear convolution done as
+// a circular one of power-of-two length L >= 2M - 1.  Chirps are evaluated in
+// FP64 from j^2 mod 2M (exact: j < 2^25, so j^2 and the multiple of 2M taken
+// from it stay below 2^53), the products with them in FP64; the transforms of
+// length L are the FP32 power-of-two FFT.
+struct Chirp {
+    long long M, L;
+    double twoM, inv2M;
+};
+
+Chirp make_chirp(long long M, long long L)
+{
+    return Chirp{M, L, 2.0 * (double) M, 1.0 / (2.0 * (double) M)};
+}
+
+__device__ __forceinline__ double2 chirp(long long j, const Chirp &c)
+{
+    const double sq = (double) j * (double) j;
+    double r = fma(-floor(sq * c.inv2M), c.twoM, sq);      // the quotient is off by one at most
+    if (r < 0.0) r += c.twoM;
+    if (r >= c.twoM) r -= c.twoM;
+    double s, co;
+    sincospi(r / (double) c.M, &s, &co);
+    return make_double2(co, s);
+}
+
+// x_j conj(c_j), zero from M on
+__device__ __forceinline__ float2 blu_in(const float2 *z, long long j, const Chirp &c)
+{
+    if (j >= c.M) return make_float2(0.f, 0.f);
+    const double2 h = chirp(j, c);
+    const double xr = z[j].x, xi = z[j].y;
+    return make_float2((float) (xr * h.x + xi * h.y), (float) (xi * h.x - xr * h.y));
+}
+
+// the convolution's kernel c_{|j|}, circular in L
+__device__ __forceinline__ float2 blu_kernel(long long j, const Chirp &c)
+{
+    const long long m = j < c.M ? j : (j > c.L - c.M ? c.L - j : -1);
+    if (m < 0) return make_float2(0.f, 0.f);
+    const double2 h = chirp(m, c);
+    return make_float2((float) h.x, (float) h.y);
+}
+
+// conj(c_k) v_k / L
+__device__ __forceinline__ float2 blu_out(float2 v, long long k, const Chirp &c)
+{
+    const double2 h = chirp(k, c);
+    const double inv = 1.0 / (double) c.L;
+    const double yr = (double) v.x * inv, yi = (double) v.y * inv;
+    return make_float2((float) (yr * h.x + yi * h.y), (float) (yi * h.x - yr * h.y));
+}
+
+// Transforms of more than 8192 points go as M = M1 M2 in two passes over
+// memory, points n = n1 M2 + n2, bins k = k1 + M1 k2:
+//   columns   the M2 transforms over n1 (stride M2), times W_M^{n2 k1}, in
+//             the same places;
+//   rows      the M1 transforms over n2 (contiguous).
+// A column CTA takes C neighbouring columns, so that its reads and writes
+// are whole C float2 runs; its threads are ordered column fastest, and the
+// C shared-memory buffers lie 16 / C float2 off each other's banks.  512
+// threads (16 points each, 128 registers) whatever the length: C = 4 at 2048
+// points fills 32-byte sectors, C = 2 at 4096 half of one (the neighbouring
+// CTA's half comes from L2).  At M = 2^22 the two passes take 30 + 27 us; three
+// transposes, two row passes with a root per point and a copy took 120 us.
+template <int L> struct ColShape {
+    static constexpr int NT = L / 16;
+    static constexpr int CTA = NT >= 512 ? 1024 : 512;
+    static constexpr int C = CTA / NT;
+    static constexpr int STRIDE = FftShape<L>::SMEM + (C >= 16 ? 1 : 16 / C);
+    static constexpr size_t SMEM = (size_t) C * STRIDE * sizeof(float2);
+};
+
+enum { COL_PLAIN, COL_BLU_IN, COL_BLU_KERNEL, COL_BLU_OUT };
+
+// MODE: where the points come from (an array, Bluestein's chirped input or
+// its kernel) or, COL_BLU_OUT, the inverse transform over k1 of rows that are
+// twiddled already, whose output is the chirped result.
+template <int L, int MODE>
+__global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_cols(const float2 *in, float2 *out, int M2,
+                                                               long long M, Chirp ch)
+{
+    using CS = ColShape<L>;
+    constexpr int S = MODE == COL_BLU_OUT ? 1 : -1;
+    extern __shared__ float2 fsm[];
+    const int c = threadIdx.x % CS::C, t = threadIdx.x / CS::C;
+    const int n2 = blockIdx.x * CS::C + c;
+    float2 v[16];
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const long long j = (long long) (t + CS::NT * m) * M2 + n2;
+        if constexpr (MODE == COL_BLU_IN) v[m] = blu_in(in, j, ch);
+        else if constexpr (MODE == COL_BLU_KERNEL) v[m] = blu_kernel(j, ch);
+        else v[m] = in[j];
+    }
+    FftTw<L, S> tw;
+    tw.init(t);
+    fft_run<L, S>(v, fsm + c * CS::STRIDE, t, tw);
+    if constexpr (MODE != COL_BLU_OUT) step_twiddles<-1>(v, n2, t, CS::NT, M);
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const long long j = (long long) (t + CS::NT * m) * M2 + n2;
+        if constexpr (MODE == COL_BLU_OUT) {
+            if (j < ch.M) out[j] = blu_out(v[m], j, ch);
+        } else {
+            out[j] = v[m];
+        }
+    }
+}
+
+// The rows' transforms with bin k1 + M1 k2 written to its natural place: the
+// same shape, a CTA's C rows giving runs of C bins.
 template <int L>
-__global__ void __launch_bounds__(FftShape<L>::CTA) k_fft_rows(const float2 *in, float2 *out,
-                                                             long long rows, long long twM)
+__global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_rows_out(const float2 *in, float2 *out, int M1)
+{
+    using CS = ColShape<L>;
+    extern __shared__ float2 fsm[];
+    const int r0 = blockIdx.x * CS::C;
+    float2 v[16];
+    {
+        // read along the rows, hand over in shared memory to the threads that
+        // are ordered row fastest for the writes
+        const int c = threadIdx.x / CS::NT, t = threadIdx.x % CS::NT;
+#pragma unroll
+        for (int m = 0; m < 16; m++) v[m] = in[(long long) (r0 + c) * L + t + CS::NT * m];
+#pragma unroll
+        for (int m = 0; m < 16; m++) fsm[c * CS::STRIDE + pad16(t + CS::NT * m)] = v[m];
+    }
+    __syncthreads();
+    const int c = threadIdx.x % CS::C, t = threadIdx.x / CS::C;
+    float2 *sm = fsm + c * CS::STRIDE;
+#pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = sm[pad16(t + CS::NT * m)];
+    FftTw<L, -1> tw;
+    tw.init(t);
+    __syncthreads();
+    fft_run<L, -1>(v, sm, t, tw);
+#pragma unroll
+    for (int m = 0; m < 16; m++) out[(long long) (t + CS::NT * m) * M1 + r0 + c] = v[m];
+}
+
+enum { ROW_PLAIN, ROW_CONV, ROW_BLU };
+
+// Row transforms in place of the rows (grid: rows / G).
+//   ROW_PLAIN  the forward transform
+//   ROW_CONV   forward, times the row of B (whose bins are in the same
+//              order), inverse, times W_M^{-k1 n2}: the middle of a
+//              convolution of M = rows L points in one pass
+//   ROW_BLU    a whole chirp-z transform of at most L points in one row
+template <int L, int MODE>
+__global__ void __launch_bounds__(FftShape<L>::CTA) k_fft_rows(const float2 *in, float2 *out, long long rows,
+                                                             const float2 *B, long long M, Chirp ch)
 {
     using SH = FftShape<L>;
     extern __shared__ float2 fsm[];
     const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
     const long long row = (long long) blockIdx.x * SH::G + grp;
     float2 *sm = fsm + grp * SH::SMEM;
-    FftTw<L, -1> tw;
-    tw.init(t);
     const bool ok = row < rows;
     float2 v[16];
 #pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = ok ? in[row * L + t + SH::NT * m] : make_float2(0.f, 0.f);
+    for (int m = 0; m < 16; m++) {
+        const int k = t + SH::NT * m;
+        if constexpr (MODE == ROW_BLU) v[m] = ok ? blu_in(in, k, ch) : make_float2(0.f, 0.f);
+        else v[m] = ok ? in[row * L + k] : make_float2(0.f, 0.f);
+    }
+    FftTw<L, -1> tw;
+    tw.init(t);
     fft_run<L, -1>(v, sm, t, tw);
+    if constexpr (MODE != ROW_PLAIN) {
+#pragma unroll
+        for (int m = 0; m < 16; m++)
+            if (ok) v[m] = cmul(v[m], B[row * L + t + SH::NT * m]);
+        FftTw<L, 1> twi;
+        twi.conj_of(tw);
+        fft_run<L, 1>(v, sm, t, twi);
+        if constexpr (MODE == ROW_CONV) step_twiddles<1>(v, (int) row, t, SH::NT, M);
+    }
     if (!ok) return;
 #pragma unroll
     for (int m = 0; m < 16; m++) {
-        const long long k = t + SH::NT * m;
-        float2 y = v[m];
-        if (twM) {
-            // W_M^{row k} = exp(-2 pi i row k / M), argument reduced mod M
-            double s, c;
-            sincospi(-2.0 * (double) ((row * k) % twM) / (double) twM, &s, &c);
-            const float cr = (float) c, ci = (float) s;
-            y = make_float2(y.x * cr - y.y * ci, y.x * ci + y.y * cr);
+        const int k = t + SH::NT * m;
+        if constexpr (MODE == ROW_BLU) {
+            if (k < ch.M) out[k] = blu_out(v[m], k, ch);
+        } else {
+            out[row * L + k] = v[m];
         }
-        out[row * L + k] = y;
     }
 }
 
-// out (C x R) = transpose of in (R x C), 32 x 32 tiles
-__global__ void __launch_bounds__(256) k_transpose(const float2 *in, float2 *out, int R, int C)
+// Bluestein's kernel in one row's points
+__global__ void k_blu_kernel(float2 *b, Chirp ch)
 {
-    __shared__ float2 tile[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += 8) {
-        const int r = by + j, c = bx + threadIdx.x;
-        if (r < R && c < C) tile[j][threadIdx.x] = in[(long long) r * C + c];
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += 8) {
-        const int c = bx + j, r = by + threadIdx.x;
-        if (r < R && c < C) out[(long long) c * R + r] = tile[threadIdx.x][j];
-    }
+    const long long j = (long long) blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < ch.L) b[j] = blu_kernel(j, ch);
 }
 
 // realfft's untangling (src/fastffts.c:195-229, forward): pair (il, n/2 - il)
@@ -108,170 +282,214 @@ __global__ void k_untangle(float2 *c, long long n)
 }
 
 
-// Median of each block's powers / ln 2 (the block "mean" of deredden), one
-// 32-thread CTA per block.
-__global__ void __launch_bounds__(32) k_dered_means(const float2 *fft, const int2 *blocks, float *means)
+// Run i of the block partition (equal blocks one behind the other): first
+// bin, block length, index of the first block, block count.  runs[nruns] is
+// a sentinel: the bin and the block behind the last.
+__device__ __forceinline__ int run_of_block(const int4 *runs, int nruns, int block)
 {
-    __shared__ float pw[AB_DERED_MAXW];
-    __shared__ unsigned hist[256], res[2];
-    const int2 b = blocks[blockIdx.x];
-    for (int i = threadIdx.x; i < b.y; i += blockDim.x) {
-        const float2 v = fft[b.x + i];
-        pw[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
+    int lo = 0, hi = nruns - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (runs[mid].z <= block) lo = mid;
+        else hi = mid - 1;
     }
-    __syncthreads();
-    const float lo = select_rank(pw, b.y, (b.y - 1) / 2, hist, res);
-    const float hi = (b.y & 1) ? lo : select_rank(pw, b.y, b.y / 2, hist, res);
-    if (threadIdx.x == 0) {
-        const float med = (b.y & 1) ? lo : (float) (0.5 * ((double) lo + (double) hi));
-        means[blockIdx.x] = (float) ((double) med / 0.69314718055994530942);
-    }
+    return lo;
 }
 
-// Segment s of the output (one CTA each): s = 0 is the first half of block 0
-// (no slope); s = 1..nb-1 runs from the midpoint of block s-1 to the midpoint
-// of block s with the slope between their means; s = nb is the second half
-// of the last block with the last slope (1 when there is one block).  Bin 0
-// becomes (1, 0).
-__global__ void __launch_bounds__(256) k_dered_apply(float2 *fft, const int2 *blocks, const float *means,
-                                                    int nb)
+// Median of each block's powers / ln 2 (the block "mean" of deredden), one
+// warp per block of at most 32 NV bins, held in registers: the k-th smallest
+// by building its bits from the top (one warp-wide count a bit; powers are
+// not negative, so their bits order as they do), and the (k+1)-th as the
+// smallest above it unless it is equal.  2^22 bins in 49645 blocks: 160 us as
+// 32-thread CTAs with 4-pass radix selects through shared memory, 42 us so
+// (some 350 warp instructions a block; issue-bound).
+template <int NV>
+__global__ void __launch_bounds__(256) k_dered_means(const float2 *fft, const int4 *runs, int nruns, int nb,
+                                                     float *means)
 {
-    const int s = blockIdx.x;
-    long long start, end;
-    float mean_old, dslope = 1.0f;
-    if (s == 0) {
-        start = blocks[0].x;
-        end = start + blocks[0].y / 2;
-        mean_old = means[0];
-        if (threadIdx.x == 0) fft[0] = make_float2(1.0f, 0.0f);
-    } else {
-        const int k = s < nb ? s : nb - 1;              // slope of blocks k-1, k
-        if (k >= 1) {
-            const int2 b0 = blocks[k - 1], b1 = blocks[k];
-            dslope = (float) ((double) __fsub_rn(means[k], means[k - 1]) / (0.5 * (double) (b0.y + b1.y)));
+    const int block = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (block >= nb) return;
+    const int4 r = runs[run_of_block(runs, nruns, block)];
+    const int n = r.y;
+    const float2 *x = fft + r.x + (long long) (block - r.z) * n;
+    unsigned u[NV];
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        u[q] = 0xFFFFFFFFu;                                 // above every power
+        if (lane + 32 * q < n) {
+            const float2 v = x[lane + 32 * q];
+            u[q] = __float_as_uint(__fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)));
         }
-        const int2 bo = blocks[s - 1];
-        start = bo.x + bo.y / 2;
-        end = (s < nb) ? blocks[s].x + blocks[s].y / 2 : bo.x + bo.y;
-        mean_old = means[s - 1];
     }
-    for (long long bin = start + threadIdx.x; bin < end; bin += blockDim.x) {
-        const float ii = (float) (bin - start);
-        const float norm = (s == 0) ? fast_invsqrtf(mean_old)
-                                    : fast_invsqrtf(__fadd_rn(mean_old, __fmul_rn(dslope, ii)));
+    const unsigned k = (unsigned) (n - 1) / 2;
+    unsigned pre = 0;
+    for (int bit = 30; bit >= 0; bit--) {
+        const unsigned trial = pre | (1u << bit);
+        unsigned below = 0;
+#pragma unroll
+        for (int q = 0; q < NV; q++) below += u[q] < trial;
+        if (__reduce_add_sync(0xffffffffu, below) <= k) pre = trial;
+    }
+    float med = __uint_as_float(pre);
+    if (!(n & 1)) {
+        unsigned upto = 0, next = 0xFFFFFFFFu;
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            upto += u[q] <= pre;
+            if (u[q] > pre) next = min(next, u[q]);
+        }
+        upto = __reduce_add_sync(0xffffffffu, upto);
+        next = __reduce_min_sync(0xffffffffu, next);
+        const float hi = upto > k + 1 ? med : __uint_as_float(next);
+        med = (float) (0.5 * ((double) med + (double) hi));
+    }
+    if (lane == 0) means[block] = (float) ((double) med / 0.69314718055994530942);
+}
+
+// Every bin by its own thread: from the middle of block b - 1 to the middle
+// of block b the line between their means, the first half of block 0 its own
+// mean, the second half of the last block the line before it carried on
+// (slope 1 when there is one block).  Bin 0 becomes (1, 0).  (One CTA per
+// segment of some 90 bins took 62 us at 2^22 bins, this 31 us.)
+__global__ void __launch_bounds__(256) k_dered_apply(float2 *fft, const int4 *runs, int nruns, int nb,
+                                                    const float *means)
+{
+    const int last = runs[nruns].x;                         // first bin behind the blocks
+    const long long bin0 = (long long) blockIdx.x * 1024;
+    // the run of the CTA's first bin, then forward
+    int ri;
+    {
+        int lo = 0, hi = nruns - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (runs[mid].x <= bin0) lo = mid;
+            else hi = mid - 1;
+        }
+        ri = lo;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const long long bin = bin0 + threadIdx.x + 256 * q;
+        if (bin == 0) fft[0] = make_float2(1.0f, 0.0f);
+        if (bin == 0 || bin >= last) continue;
+        while (bin >= runs[ri + 1].x) ri++;
+        const int4 r = runs[ri];
+        const int in = (int) bin - r.x, k = in / r.y, off = in - k * r.y;
+        const int b = r.z + k;                              // the bin's block
+        // segment s = 0: before block 0's middle; else behind block s - 1's
+        const int s = off < r.y / 2 ? b : b + 1;
+        float norm;
+        if (s == 0) {
+            norm = fast_invsqrtf(means[0]);
+        } else {
+            const int kk = s < nb ? s : nb - 1;             // slope of blocks kk - 1, kk
+            // lengths of block b and of the neighbours the segment involves
+            const int4 rp = (k == 0 && ri > 0) ? runs[ri - 1] : r;
+            const int4 rn = (k == r.w - 1 && ri + 1 < nruns) ? runs[ri + 1] : r;
+            const int len_prev = rp.y, len_next = rn.y;     // of blocks b - 1 and b + 1
+            long long start;
+            if (s == b) start = (long long) r.x + (long long) k * r.y - len_prev + len_prev / 2;
+            else start = (long long) r.x + (long long) k * r.y + r.y / 2;
+            float dslope = 1.0f;
+            if (kk >= 1) {
+                const int sum = kk == b ? len_prev + r.y : r.y + len_next;
+                dslope = (float) ((double) __fsub_rn(means[kk], means[kk - 1]) / (0.5 * (double) sum));
+            }
+            const float ii = (float) (bin - start);
+            norm = fast_invsqrtf(__fadd_rn(means[s - 1], __fmul_rn(dslope, ii)));
+        }
         const float2 v = fft[bin];
         fft[bin] = make_float2(__fmul_rn(v.x, norm), __fmul_rn(v.y, norm));
     }
 }
 
-template <int L>
-cudaError_t fft_rows_L(const float2 *in, float2 *out, long long rows, long long twM, cudaStream_t st)
+template <int L, int MODE>
+cudaError_t cols_L(const float2 *in, float2 *out, int M2, long long M, const Chirp &ch, cudaStream_t st)
 {
-    using SH = FftShape<L>;
-    const size_t smem = (size_t) SH::G * SH::SMEM * sizeof(float2);
-    cudaFuncSetAttribute(k_fft_rows<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const long long grid = (rows + SH::G - 1) / SH::G;
-    k_fft_rows<L><<<(unsigned) grid, SH::CTA, smem, st>>>(in, out, rows, twM);
+    using CS = ColShape<L>;
+    cudaError_t e = cudaFuncSetAttribute(k_fft_cols<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) CS::SMEM);
+    if (e != cudaSuccess) return e;
+    k_fft_cols<L, MODE><<<(unsigned) (M2 / CS::C), CS::CTA, CS::SMEM, st>>>(in, out, M2, M, ch);
     return cudaGetLastError();
 }
 
-cudaError_t fft_rows(int L, const float2 *in, float2 *out, long long rows, long long twM, cudaStream_t st)
+template <int MODE>
+cudaError_t cols(int L, const float2 *in, float2 *out, int M2, long long M, const Chirp &ch, cudaStream_t st)
 {
     switch (L) {
-        case 256: return fft_rows_L<256>(in, out, rows, twM, st);
-        case 512: return fft_rows_L<512>(in, out, rows, twM, st);
-        case 1024: return fft_rows_L<1024>(in, out, rows, twM, st);
-        case 2048: return fft_rows_L<2048>(in, out, rows, twM, st);
-        case 4096: return fft_rows_L<4096>(in, out, rows, twM, st);
-        case 8192: return fft_rows_L<8192>(in, out, rows, twM, st);
+        case 256: return cols_L<256, MODE>(in, out, M2, M, ch, st);
+        case 512: return cols_L<512, MODE>(in, out, M2, M, ch, st);
+        case 1024: return cols_L<1024, MODE>(in, out, M2, M, ch, st);
+        case 2048: return cols_L<2048, MODE>(in, out, M2, M, ch, st);
+        case 4096: return cols_L<4096, MODE>(in, out, M2, M, ch, st);
+        case 8192: return cols_L<8192, MODE>(in, out, M2, M, ch, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t transpose(const float2 *in, float2 *out, int R, int C, cudaStream_t st)
+template <int L> cudaError_t rows_out_L(const float2 *in, float2 *out, int M1, cudaStream_t st)
 {
-    dim3 grid((C + 31) / 32, (R + 31) / 32), block(32, 8);
-    k_transpose<<<grid, block, 0, st>>>(in, out, R, C);
+    using CS = ColShape<L>;
+    cudaError_t e = cudaFuncSetAttribute(k_fft_rows_out<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) CS::SMEM);
+    if (e != cudaSuccess) return e;
+    k_fft_rows_out<L><<<(unsigned) (M1 / CS::C), CS::CTA, CS::SMEM, st>>>(in, out, M1);
     return cudaGetLastError();
 }
 
-// Forward complex FFT of M points, M a power of two in 512..8192 or 2^16..2^26;
-// out may be in, scratch (M points) may not.
-cudaError_t cfft_pow2(const float2 *in, float2 *out, float2 *scratch, long long M, cudaStream_t st)
+cudaError_t rows_out(int L, const float2 *in, float2 *out, int M1, cudaStream_t st)
 {
-    if (M <= 8192) return fft_rows((int) M, in, out, 1, 0, st);
+    switch (L) {
+        case 256: return rows_out_L<256>(in, out, M1, st);
+        case 512: return rows_out_L<512>(in, out, M1, st);
+        case 1024: return rows_out_L<1024>(in, out, M1, st);
+        case 2048: return rows_out_L<2048>(in, out, M1, st);
+        case 4096: return rows_out_L<4096>(in, out, M1, st);
+        case 8192: return rows_out_L<8192>(in, out, M1, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int L, int MODE>
+cudaError_t rows_L(const float2 *in, float2 *out, long long rows, const float2 *B, long long M,
+                   const Chirp &ch, cudaStream_t st)
+{
+    using SH = FftShape<L>;
+    const size_t smem = (size_t) SH::G * SH::SMEM * sizeof(float2);
+    cudaError_t e = cudaFuncSetAttribute(k_fft_rows<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) smem);
+    if (e != cudaSuccess) return e;
+    const long long grid = (rows + SH::G - 1) / SH::G;
+    k_fft_rows<L, MODE><<<(unsigned) grid, SH::CTA, smem, st>>>(in, out, rows, B, M, ch);
+    return cudaGetLastError();
+}
+
+template <int MODE>
+cudaError_t fft_rows(int L, const float2 *in, float2 *out, long long rows, const float2 *B, long long M,
+                     const Chirp &ch, cudaStream_t st)
+{
+    switch (L) {
+        case 256: return rows_L<256, MODE>(in, out, rows, B, M, ch, st);
+        case 512: return rows_L<512, MODE>(in, out, rows, B, M, ch, st);
+        case 1024: return rows_L<1024, MODE>(in, out, rows, B, M, ch, st);
+        case 2048: return rows_L<2048, MODE>(in, out, rows, B, M, ch, st);
+        case 4096: return rows_L<4096, MODE>(in, out, rows, B, M, ch, st);
+        case 8192: return rows_L<8192, MODE>(in, out, rows, B, M, ch, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+// M = M1 M2 of a transform above 8192 points: M1 (the columns) at most 2048,
+// where C = 4 columns fill whole sectors, as long as M2 <= cap
+void split_len(long long M, int cap, int *M1, int *M2)
+{
     int m = 0;
     while ((1LL << m) < M) m++;
-    const int M1 = 1 << (m / 2), M2 = (int) (M / M1);
-    // x[n1][n2] (M1 x M2) -> scratch[n2][n1]; rows of length M1 with the
-    // twiddle; -> out[k1][n2]; rows of length M2; -> scratch[k2][k1]; copy
-    cudaError_t e = transpose(in, scratch, M1, M2, st);
-    if (e == cudaSuccess) e = fft_rows(M1, scratch, scratch, M2, M, st);
-    if (e == cudaSuccess) e = transpose(scratch, out, M2, M1, st);
-    if (e == cudaSuccess) e = fft_rows(M2, out, out, M1, 0, st);
-    if (e == cudaSuccess) e = transpose(out, scratch, M1, M2, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, scratch, sizeof(float2) * M, cudaMemcpyDeviceToDevice, st);
-    return e;
-}
-
-// Bluestein's chirp-z transform for any length M: with c_j = exp(i pi j^2 / M),
-// X_k = conj(c_k) sum_j (x_j conj(c_j)) c_{k-j}, a linear convolution done as
-// a circular one of power-of-two length L >= 2M - 1.  Chirps are evaluated in
-// FP64 from j^2 mod 2M (exact in 64-bit integers), the products with them in
-// FP64; the three length-L transforms are the FP32 power-of-two FFT above.
-__device__ __forceinline__ void chirp(long long j, long long M, double &c, double &s)
-{
-    const long long r = (j * j) % (2 * M);
-    sincospi((double) r / (double) M, &s, &c);
-}
-
-__global__ void k_blu_pre(const float2 *z, float2 *a, long long M, long long L)
-{
-    const long long j = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= L) return;
-    if (j >= M) {
-        a[j] = make_float2(0.f, 0.f);
-        return;
-    }
-    double c, s;
-    chirp(j, M, c, s);
-    const double xr = z[j].x, xi = z[j].y;           // x conj(c)
-    a[j] = make_float2((float) (xr * c + xi * s), (float) (xi * c - xr * s));
-}
-
-__global__ void k_blu_kernel(float2 *b, long long M, long long L)
-{
-    const long long j = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= L) return;
-    const long long m = j < M ? j : (j > L - M ? L - j : -1);
-    if (m < 0) {
-        b[j] = make_float2(0.f, 0.f);
-        return;
-    }
-    double c, s;
-    chirp(m, M, c, s);
-    b[j] = make_float2((float) c, (float) s);
-}
-
-// a = conj(a B): the inverse transform as a forward one of the conjugate
-__global__ void k_blu_mul(float2 *a, const float2 *B, long long L)
-{
-    const long long j = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= L) return;
-    const float2 x = a[j], y = B[j];
-    a[j] = make_float2(x.x * y.x - x.y * y.y, -(x.x * y.y + x.y * y.x));
-}
-
-__global__ void k_blu_post(const float2 *v, float2 *out, long long M, long long L)
-{
-    const long long k = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= M) return;
-    double c, s;
-    chirp(k, M, c, s);
-    const double inv = 1.0 / (double) L;
-    const double yr = (double) v[k].x * inv, yi = -(double) v[k].y * inv;   // conj(v) / L
-    out[k] = make_float2((float) (yr * c + yi * s), (float) (yi * c - yr * s));
+    int a = m / 2;
+    while (a > 11 && (M >> (a - 1)) <= cap) a--;
+    *M1 = 1 << a;
+    *M2 = (int) (M >> a);
 }
 
 }  // namespace
@@ -302,42 +520,68 @@ cudaError_t launch_realfft(const float *series, float2 *out, float2 *scratch, lo
 {
     const long long M = n / 2;
     if (n % 2 || !pow2_fft_supported(M)) return cudaErrorInvalidValue;
-    cudaError_t e = cfft_pow2(reinterpret_cast<const float2 *>(series), out, scratch, M, st);
+    const float2 *x = reinterpret_cast<const float2 *>(series);
+    cudaError_t e;
+    if (M <= 8192) {
+        e = fft_rows<ROW_PLAIN>((int) M, x, out, 1, nullptr, M, Chirp{}, st);
+    } else {
+        int M1, M2;
+        split_len(M, 4096, &M1, &M2);
+        e = cols<COL_PLAIN>(M1, x, scratch, M2, M, Chirp{}, st);
+        if (e == cudaSuccess) e = rows_out(M2, scratch, out, M1, st);
+    }
     if (e != cudaSuccess) return e;
     const long long nthr = M / 2 + 1;
     k_untangle<<<(unsigned) ((nthr + 255) / 256), 256, 0, st>>>(out, n);
     return cudaGetLastError();
 }
 
-cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *scratch,
-                                     float2 *B, bool build_B, long long n, cudaStream_t st)
+// Three passes over memory: the chirped input's columns, the rows with the
+// convolution's product in the middle (the bins stay in the order the first
+// transform leaves them in, and B's with them), the columns back.  (Three
+// whole transforms with their transposes and the products between them took
+// 480 us and two copies at M = 3024000, L = 2^23; the three passes 181 us:
+// 73 + 60 + 49, the first bound by its FP64 chirps and inter-step roots.)
+cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *B, bool build_B,
+                                     long long n, cudaStream_t st)
 {
     const long long M = n / 2, L = bluestein_len(M);
     if (n % 2 || n < 1024 || M > (1LL << 25)) return cudaErrorInvalidValue;
-    const unsigned gL = (unsigned) ((L + 255) / 256), gM = (unsigned) ((M + 255) / 256);
+    const Chirp ch = make_chirp(M, L);
+    const float2 *x = reinterpret_cast<const float2 *>(series);
     cudaError_t e = cudaSuccess;
-    if (build_B) {                                   // FFT of the chirp kernel, kept per M
-        k_blu_kernel<<<gL, 256, 0, st>>>(B, M, L);
-        e = cfft_pow2(B, B, scratch, L, st);
-        if (e != cudaSuccess) return e;
+    if (L <= 8192) {
+        if (build_B) {                               // FFT of the chirp kernel, kept per M
+            k_blu_kernel<<<(unsigned) ((L + 255) / 256), 256, 0, st>>>(B, ch);
+            e = fft_rows<ROW_PLAIN>((int) L, B, B, 1, nullptr, L, ch, st);
+        }
+        if (e == cudaSuccess) e = fft_rows<ROW_BLU>((int) L, x, out, 1, B, L, ch, st);
+    } else {
+        int M1, M2;
+        split_len(L, 8192, &M1, &M2);
+        if (build_B) {
+            e = cols<COL_BLU_KERNEL>(M1, nullptr, B, M2, L, ch, st);
+            if (e == cudaSuccess) e = fft_rows<ROW_PLAIN>(M2, B, B, M1, nullptr, L, ch, st);
+        }
+        if (e == cudaSuccess) e = cols<COL_BLU_IN>(M1, x, a, M2, L, ch, st);
+        if (e == cudaSuccess) e = fft_rows<ROW_CONV>(M2, a, a, M1, B, L, ch, st);
+        if (e == cudaSuccess) e = cols<COL_BLU_OUT>(M1, a, out, M2, L, ch, st);
     }
-    k_blu_pre<<<gL, 256, 0, st>>>(reinterpret_cast<const float2 *>(series), a, M, L);
-    e = cfft_pow2(a, a, scratch, L, st);
     if (e != cudaSuccess) return e;
-    k_blu_mul<<<gL, 256, 0, st>>>(a, B, L);
-    e = cfft_pow2(a, a, scratch, L, st);
-    if (e != cudaSuccess) return e;
-    k_blu_post<<<gM, 256, 0, st>>>(a, out, M, L);
     const long long nthr = M / 2 + 1;
     k_untangle<<<(unsigned) ((nthr + 255) / 256), 256, 0, st>>>(out, n);
     return cudaGetLastError();
 }
 
-cudaError_t launch_deredden(float2 *fft, const int2 *blocks, int nb, float *means, cudaStream_t st)
+cudaError_t launch_deredden(float2 *fft, const int4 *runs, int nruns, int nb, int maxlen, long long numbins,
+                            float *means, cudaStream_t st)
 {
-    if (nb <= 0) return cudaErrorInvalidValue;
-    k_dered_means<<<nb, 32, 0, st>>>(fft, blocks, means);
-    k_dered_apply<<<nb + 1, 256, 0, st>>>(fft, blocks, means, nb);
+    if (nb <= 0 || nruns <= 0 || maxlen > AB_DERED_MAXW) return cudaErrorInvalidValue;
+    const unsigned grid = (unsigned) ((nb + 7) / 8);
+    if (maxlen <= 128) k_dered_means<4><<<grid, 256, 0, st>>>(fft, runs, nruns, nb, means);
+    else if (maxlen <= 256) k_dered_means<8><<<grid, 256, 0, st>>>(fft, runs, nruns, nb, means);
+    else k_dered_means<AB_DERED_MAXW / 32><<<grid, 256, 0, st>>>(fft, runs, nruns, nb, means);
+    k_dered_apply<<<(unsigned) ((numbins + 1023) / 1024), 256, 0, st>>>(fft, runs, nruns, nb, means);
     return cudaGetLastError();
 }
 

@@ -53,3 +53,31 @@ def test_dered_plan_partitions_the_spectrum(ablib):
     want = np.minimum((6 * np.log(binnum[:-1].astype(np.float64))).astype(int), 200)
     assert np.array_equal(blocks[1:-1, 1], want[:-1])
     assert f(5, 6, 200, 1e300, 1.0, None, 0, C.byref(nb)) == -1
+
+
+@pytest.mark.parametrize("numbins,sw,ew,endfreq,T", [
+    (7, 6, 200, 1e300, 1.0), (8, 6, 200, 1e300, 1.0), (100, 6, 200, 1e300, 1.0), (12345, 6, 200, 7812.5, 8.0),
+    (1 << 20, 6, 200, 1e300, 1.0), ((1 << 22) + 1, 6, 200, 7812.5, 537.0), (1 << 18, 6, 200, 20.0, 1000.0),
+    (1 << 18, 6, 200, 1e-9, 1000.0), (5000, 1, 3, 1e300, 1.0), (5000, 2, 2, 1e300, 1.0),
+    (1 << 19, 100, 1024, 1e300, 1.0), (300000, 37, 1000, 100.0, 33.0)])
+def test_dered_runs_are_the_plan(ablib, numbins, sw, ew, endfreq, T):
+    """The runs of equal blocks spell out the block list, block by block."""
+    L = ablib.lib()
+    nb, nr, ml = C.c_longlong(), C.c_int(), C.c_int()
+    L.ab_dered_plan.argtypes = [C.c_longlong, C.c_int, C.c_int, C.c_double, C.c_double, C.c_void_p,
+                                C.c_longlong, C.POINTER(C.c_longlong)]
+    assert L.ab_dered_plan(numbins, sw, ew, endfreq, T, None, 0, C.byref(nb)) == 0
+    blocks = np.zeros((nb.value, 2), np.int32)
+    assert L.ab_dered_plan(numbins, sw, ew, endfreq, T, blocks.ctypes.data, nb.value, C.byref(nb)) == 0
+    f = L.ab_dered_runs
+    f.argtypes = [C.c_longlong, C.c_int, C.c_int, C.c_double, C.c_double, C.c_void_p, C.c_int,
+                  C.POINTER(C.c_int), C.POINTER(C.c_longlong), C.POINTER(C.c_int)]
+    runs = np.zeros((1032, 4), np.int32)
+    n2 = C.c_longlong()
+    assert f(numbins, sw, ew, endfreq, T, runs.ctypes.data, 1032, C.byref(nr), C.byref(n2), C.byref(ml)) == 0
+    assert n2.value == nb.value and ml.value == blocks[:, 1].max()
+    got = [(first + k * length, length) for first, length, _, count in runs[:nr.value] for k in range(count)]
+    assert np.array_equal(np.array(got), blocks)
+    starts = np.concatenate([[0], np.cumsum(runs[:nr.value, 3])])
+    assert np.array_equal(runs[:nr.value + 1, 2], starts)
+    assert tuple(runs[nr.value]) == (blocks[-1].sum(), 1, nb.value, 0)

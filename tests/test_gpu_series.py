@@ -140,3 +140,33 @@ def test_device_pointers_off_their_boundary(ctx, ablib):
     with pytest.raises(ablib.AccelError):
         ctx.search(obs, None, device_ptr=out.data_ptr() + 4)
     assert len(ctx.search(obs, None, device_ptr=out.data_ptr())) == len(ctx.search(obs, want))
+
+
+@pytest.mark.parametrize("n", [1 << 18, 1 << 20, 1 << 24, 1 << 25, 1 << 26,      # both splits' edges
+                               1024 * 3, 16000, 24578, 262218, 3000000, 9000018, 40000014])
+def test_device_realfft_every_split(ctx, n):
+    """The two-pass transform at every pair of lengths and the chirp-z transform at row
+    lengths 512 to 8192, one-row and three-pass, against the FP64 transform on the device."""
+    import torch
+
+    x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
+    out = torch.empty(n // 2, dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):                                   # the second call reuses the chirp's transform
+        assert ctx.L.ab_realfft(ctx.ptr, x.data_ptr(), n, 1, out.data_ptr(), 1) == 0
+        X = torch.fft.rfft(x.double())
+        want = X[:n // 2].clone()
+        want[0] = torch.complex(X[0].real, X[n // 2].real)
+        assert float((out - want).abs().max()) <= 3e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("numbins,sw,ew,endfreq", [(40, 6, 200, 1e300), (5000, 1, 3, 1e300), (70001, 6, 200, 900.0),
+                                                  (70000, 20, 150, 1e300), (300001, 100, 1024, 1e300)])
+def test_device_deredden_block_lengths(ctx, oracle, numbins, sw, ew, endfreq):
+    """Blocks of up to 128, 256 and 1024 bins, cut-off last blocks, a plan that ends early and
+    the jump to endwidth past endfreq: the oracle's bits."""
+    rng = np.random.default_rng(numbins)
+    spec = (rng.standard_normal(numbins) + 1j * rng.standard_normal(numbins)).astype(np.complex64)
+    dev = ctx.deredden(spec, sw, ew, endfreq, 64.0)
+    orc = oracle.deredden(spec, sw, ew, endfreq, 64.0)
+    assert np.array_equal(dev.view(np.uint32), orc.view(np.uint32))
