@@ -1399,12 +1399,14 @@ static int realfft_dev(ab_ctx *ctx, const float *series, long long n, int series
         return AB_OK;
     }
     const long long L = bluestein_len(M);
+    CK(ctx->ser_scr.ensure((size_t) L));
     CK(ctx->blu_a.ensure((size_t) L));
     const bool fresh = ctx->blu_M != M || ctx->blu_b.n < (size_t) L;
     CK(ctx->blu_b.ensure((size_t) L));
-    CK(launch_realfft_bluestein(din, dout, ctx->blu_a.p, ctx->blu_b.p, fresh, n, ctx->stream));
+    CK(launch_realfft_bluestein(din, dout, ctx->blu_a.p, ctx->ser_scr.p, ctx->blu_b.p, fresh, n,
+                                ctx->stream));
     ctx->blu_M = M;
-    ctx->launches += (L <= 8192 ? 2 : 4) + (fresh ? 2 : 0);
+    ctx->launches += (L <= 8192 ? 3 : 5) + (fresh ? 2 : 0);
     return AB_OK;
 }
 

@@ -201,18 +201,6 @@ template <int L, int S> struct FftTw {
                 powers(2.0 * (double) ((t + SH::NT * b) & 4095) / (double) L, &b4[b], 1);
         }
     }
-    // the twiddles of the transform in the other direction
-    __device__ __forceinline__ void conj_of(const FftTw<L, -S> &o)
-    {
-#pragma unroll
-        for (int e = 0; e < 4; e++) b2[e] = make_float2(o.b2[e].x, -o.b2[e].y);
-#pragma unroll
-        for (int b = 0; b < SH::NB3; b++)
-#pragma unroll
-            for (int e = 0; e < NBASE3; e++) b3[b][e] = make_float2(o.b3[b][e].x, -o.b3[b][e].y);
-#pragma unroll
-        for (int b = 0; b < SH::NB4; b++) b4[b] = make_float2(o.b4[b].x, -o.b4[b].y);
-    }
 };
 
 // x[q] *= w^q for q = 1..R-1, w^q built from the base powers.

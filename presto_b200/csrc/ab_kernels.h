@@ -205,10 +205,10 @@ bool realfft_supported(long long n);
 bool pow2_fft_supported(long long M);
 long long bluestein_len(long long M);
 cudaError_t launch_realfft(const float *series, float2 *out, float2 *scratch, long long n, cudaStream_t st);
-// any even n (1024 <= n <= 2^26): a: bluestein_len(n/2) points of work, B the
-// cached transform of the chirp kernel (rebuilt when build_B)
-cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *B, bool build_B,
-                                     long long n, cudaStream_t st);
+// any even n (1024 <= n <= 2^26): a: bluestein_len(n/2) points of work, scratch
+// as many, B the cached transform of the chirp kernel (rebuilt when build_B)
+cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *scratch, float2 *B,
+                                     bool build_B, long long n, cudaStream_t st);
 // runs of equal blocks {first bin, length, first block, blocks}, nruns of them
 // and a sentinel {bin behind the last, 1, nb, 0}; nb blocks of at most maxlen bins
 cudaError_t launch_deredden(float2 *fft, const int4 *runs, int nruns, int nb, int maxlen, long long numbins,

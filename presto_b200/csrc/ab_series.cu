@@ -11,7 +11,7 @@
 // twiddles, then rows written in their transposed places.  Any other even n
 // (dedispersed series are usually 2^a 3^b 5^c 7^d samples long) goes through
 // Bluestein's chirp-z transform on power-of-two transforms of length
-// >= 2M - 1, fused into three passes.
+// >= 2M - 1, its products fused into their four passes.
 //
 // deredden: the block partition depends only on bin indices (lengths
 // startwidth ln(bin) up to endwidth), so the host plans it as runs of equal
@@ -29,23 +29,22 @@
 namespace ab {
 namespace {
 
-// W_M^{S j} for 0 <= j < M
-template <int S> __device__ __forceinline__ double2 root(long long j, double invM)
+// W_M^j = exp(-2 pi i j / M), 0 <= j < M
+__device__ __forceinline__ double2 root(long long j, double invM)
 {
     double s, c;
-    sincospi(2.0 * S * ((double) j * invM), &s, &c);
+    sincospi(-2.0 * ((double) j * invM), &s, &c);
     return make_double2(c, s);
 }
 
-// v[m] *= W_M^{S a (t + NT m)}, m = 0..15 (a, t + NT m < 2^13, M a power of
+// v[m] *= W_M^{a (t + NT m)}, m = 0..15 (a, t + NT m < 2^13, M a power of
 // two: a (t + NT m) / M is exact): two FP64 roots and their products instead
 // of sixteen roots; fifteen FP64 products stay far below the FP32 rounding.
-template <int S>
 __device__ __forceinline__ void step_twiddles(float2 (&v)[16], int a, int t, int NT, long long M)
 {
     const double inv = 1.0 / (double) M;
-    double2 w = root<S>((long long) a * t, inv);
-    const double2 q = root<S>((long long) a * NT, inv);
+    double2 w = root((long long) a * t, inv);
+    const double2 q = root((long long) a * NT, inv);
 #pragma unroll
     for (int m = 0; m < 16; m++) {
         const float cr = (float) w.x, ci = (float) w.y;
@@ -99,12 +98,13 @@ __device__ __forceinline__ float2 blu_kernel(long long j, const Chirp &c)
     return make_float2((float) h.x, (float) h.y);
 }
 
-// conj(c_k) v_k / L
+// conj(c_k) conj(v_k) / L: the inverse transform is taken as a forward one of
+// the conjugate
 __device__ __forceinline__ float2 blu_out(float2 v, long long k, const Chirp &c)
 {
     const double2 h = chirp(k, c);
     const double inv = 1.0 / (double) c.L;
-    const double yr = (double) v.x * inv, yi = (double) v.y * inv;
+    const double yr = (double) v.x * inv, yi = -(double) v.y * inv;
     return make_float2((float) (yr * h.x + yi * h.y), (float) (yi * h.x - yr * h.y));
 }
 
@@ -128,17 +128,15 @@ template <int L> struct ColShape {
     static constexpr size_t SMEM = (size_t) C * STRIDE * sizeof(float2);
 };
 
-enum { COL_PLAIN, COL_BLU_IN, COL_BLU_KERNEL, COL_BLU_OUT };
+enum { COL_PLAIN, COL_BLU_IN, COL_BLU_KERNEL };
 
 // MODE: where the points come from (an array, Bluestein's chirped input or
-// its kernel) or, COL_BLU_OUT, the inverse transform over k1 of rows that are
-// twiddled already, whose output is the chirped result.
+// its kernel).
 template <int L, int MODE>
 __global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_cols(const float2 *in, float2 *out, int M2,
                                                                long long M, Chirp ch)
 {
     using CS = ColShape<L>;
-    constexpr int S = MODE == COL_BLU_OUT ? 1 : -1;
     extern __shared__ float2 fsm[];
     const int c = threadIdx.x % CS::C, t = threadIdx.x / CS::C;
     const int n2 = blockIdx.x * CS::C + c;
@@ -150,25 +148,36 @@ __global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_cols(const float2 *in,
         else if constexpr (MODE == COL_BLU_KERNEL) v[m] = blu_kernel(j, ch);
         else v[m] = in[j];
     }
-    FftTw<L, S> tw;
+    FftTw<L, -1> tw;
     tw.init(t);
-    fft_run<L, S>(v, fsm + c * CS::STRIDE, t, tw);
-    if constexpr (MODE != COL_BLU_OUT) step_twiddles<-1>(v, n2, t, CS::NT, M);
+    fft_run<L, -1>(v, fsm + c * CS::STRIDE, t, tw);
+    step_twiddles(v, n2, t, CS::NT, M);
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
-        const long long j = (long long) (t + CS::NT * m) * M2 + n2;
-        if constexpr (MODE == COL_BLU_OUT) {
-            if (j < ch.M) out[j] = blu_out(v[m], j, ch);
-        } else {
-            out[j] = v[m];
-        }
+    for (int m = 0; m < 16; m++) out[(long long) (t + CS::NT * m) * M2 + n2] = v[m];
+}
+
+enum { ROW_PLAIN, ROW_CONV, ROW_BLU_OUT };
+
+// What becomes of bin k of a transform: kept, the convolution's product
+// conj(v B[k]) (the next transform's input), or the chirped result.
+template <int MODE>
+__device__ __forceinline__ void put_bin(float2 *out, long long k, float2 v, const float2 *B, const Chirp &ch)
+{
+    if constexpr (MODE == ROW_CONV) {
+        const float2 y = B[k];
+        out[k] = make_float2(v.x * y.x - v.y * y.y, -(v.x * y.y + v.y * y.x));
+    } else if constexpr (MODE == ROW_BLU_OUT) {
+        if (k < ch.M) out[k] = blu_out(v, k, ch);
+    } else {
+        out[k] = v;
     }
 }
 
 // The rows' transforms with bin k1 + M1 k2 written to its natural place: the
 // same shape, a CTA's C rows giving runs of C bins.
-template <int L>
-__global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_rows_out(const float2 *in, float2 *out, int M1)
+template <int L, int MODE>
+__global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_rows_out(const float2 *in, float2 *out, int M1,
+                                                                   const float2 *B, Chirp ch)
 {
     using CS = ColShape<L>;
     extern __shared__ float2 fsm[];
@@ -193,59 +202,33 @@ __global__ void __launch_bounds__(ColShape<L>::CTA) k_fft_rows_out(const float2 
     __syncthreads();
     fft_run<L, -1>(v, sm, t, tw);
 #pragma unroll
-    for (int m = 0; m < 16; m++) out[(long long) (t + CS::NT * m) * M1 + r0 + c] = v[m];
+    for (int m = 0; m < 16; m++)
+        put_bin<MODE>(out, (long long) (t + CS::NT * m) * M1 + r0 + c, v[m], B, ch);
 }
 
-enum { ROW_PLAIN, ROW_CONV, ROW_BLU };
-
-// Row transforms in place of the rows (grid: rows / G).
-//   ROW_PLAIN  the forward transform
-//   ROW_CONV   forward, times the row of B (whose bins are in the same
-//              order), inverse, times W_M^{-k1 n2}: the middle of a
-//              convolution of M = rows L points in one pass
-//   ROW_BLU    a whole chirp-z transform of at most L points in one row
-template <int L, int MODE>
-__global__ void __launch_bounds__(FftShape<L>::CTA) k_fft_rows(const float2 *in, float2 *out, long long rows,
-                                                             const float2 *B, long long M, Chirp ch)
+// A transform of L <= 8192 points in one CTA.
+template <int L, bool BLU_IN, int MODE>
+__global__ void __launch_bounds__(FftShape<L>::CTA) k_fft_one(const float2 *in, float2 *out, const float2 *B, Chirp ch)
 {
     using SH = FftShape<L>;
     extern __shared__ float2 fsm[];
     const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
-    const long long row = (long long) blockIdx.x * SH::G + grp;
-    float2 *sm = fsm + grp * SH::SMEM;
-    const bool ok = row < rows;
     float2 v[16];
 #pragma unroll
     for (int m = 0; m < 16; m++) {
         const int k = t + SH::NT * m;
-        if constexpr (MODE == ROW_BLU) v[m] = ok ? blu_in(in, k, ch) : make_float2(0.f, 0.f);
-        else v[m] = ok ? in[row * L + k] : make_float2(0.f, 0.f);
+        v[m] = BLU_IN ? blu_in(in, k, ch) : in[k];
     }
     FftTw<L, -1> tw;
     tw.init(t);
-    fft_run<L, -1>(v, sm, t, tw);
-    if constexpr (MODE != ROW_PLAIN) {
+    __syncthreads();                        // out may be in: every group has read it
+    fft_run<L, -1>(v, fsm + grp * SH::SMEM, t, tw);
+    if (grp) return;                        // the CTA's other groups did the same
 #pragma unroll
-        for (int m = 0; m < 16; m++)
-            if (ok) v[m] = cmul(v[m], B[row * L + t + SH::NT * m]);
-        FftTw<L, 1> twi;
-        twi.conj_of(tw);
-        fft_run<L, 1>(v, sm, t, twi);
-        if constexpr (MODE == ROW_CONV) step_twiddles<1>(v, (int) row, t, SH::NT, M);
-    }
-    if (!ok) return;
-#pragma unroll
-    for (int m = 0; m < 16; m++) {
-        const int k = t + SH::NT * m;
-        if constexpr (MODE == ROW_BLU) {
-            if (k < ch.M) out[k] = blu_out(v[m], k, ch);
-        } else {
-            out[row * L + k] = v[m];
-        }
-    }
+    for (int m = 0; m < 16; m++) put_bin<MODE>(out, t + SH::NT * m, v[m], B, ch);
 }
 
-// Bluestein's kernel in one row's points
+// Bluestein's kernel for a transform in one CTA
 __global__ void k_blu_kernel(float2 *b, Chirp ch)
 {
     const long long j = (long long) blockIdx.x * blockDim.x + threadIdx.x;
@@ -428,68 +411,64 @@ cudaError_t cols(int L, const float2 *in, float2 *out, int M2, long long M, cons
     }
 }
 
-template <int L> cudaError_t rows_out_L(const float2 *in, float2 *out, int M1, cudaStream_t st)
+template <int L, int MODE>
+cudaError_t rows_out_L(const float2 *in, float2 *out, int M1, const float2 *B, const Chirp &ch, cudaStream_t st)
 {
     using CS = ColShape<L>;
-    cudaError_t e = cudaFuncSetAttribute(k_fft_rows_out<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_fft_rows_out<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int) CS::SMEM);
     if (e != cudaSuccess) return e;
-    k_fft_rows_out<L><<<(unsigned) (M1 / CS::C), CS::CTA, CS::SMEM, st>>>(in, out, M1);
-    return cudaGetLastError();
-}
-
-cudaError_t rows_out(int L, const float2 *in, float2 *out, int M1, cudaStream_t st)
-{
-    switch (L) {
-        case 256: return rows_out_L<256>(in, out, M1, st);
-        case 512: return rows_out_L<512>(in, out, M1, st);
-        case 1024: return rows_out_L<1024>(in, out, M1, st);
-        case 2048: return rows_out_L<2048>(in, out, M1, st);
-        case 4096: return rows_out_L<4096>(in, out, M1, st);
-        case 8192: return rows_out_L<8192>(in, out, M1, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <int L, int MODE>
-cudaError_t rows_L(const float2 *in, float2 *out, long long rows, const float2 *B, long long M,
-                   const Chirp &ch, cudaStream_t st)
-{
-    using SH = FftShape<L>;
-    const size_t smem = (size_t) SH::G * SH::SMEM * sizeof(float2);
-    cudaError_t e = cudaFuncSetAttribute(k_fft_rows<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int) smem);
-    if (e != cudaSuccess) return e;
-    const long long grid = (rows + SH::G - 1) / SH::G;
-    k_fft_rows<L, MODE><<<(unsigned) grid, SH::CTA, smem, st>>>(in, out, rows, B, M, ch);
+    k_fft_rows_out<L, MODE><<<(unsigned) (M1 / CS::C), CS::CTA, CS::SMEM, st>>>(in, out, M1, B, ch);
     return cudaGetLastError();
 }
 
 template <int MODE>
-cudaError_t fft_rows(int L, const float2 *in, float2 *out, long long rows, const float2 *B, long long M,
-                     const Chirp &ch, cudaStream_t st)
+cudaError_t rows_out(int L, const float2 *in, float2 *out, int M1, const float2 *B, const Chirp &ch,
+                     cudaStream_t st)
 {
     switch (L) {
-        case 256: return rows_L<256, MODE>(in, out, rows, B, M, ch, st);
-        case 512: return rows_L<512, MODE>(in, out, rows, B, M, ch, st);
-        case 1024: return rows_L<1024, MODE>(in, out, rows, B, M, ch, st);
-        case 2048: return rows_L<2048, MODE>(in, out, rows, B, M, ch, st);
-        case 4096: return rows_L<4096, MODE>(in, out, rows, B, M, ch, st);
-        case 8192: return rows_L<8192, MODE>(in, out, rows, B, M, ch, st);
+        case 256: return rows_out_L<256, MODE>(in, out, M1, B, ch, st);
+        case 512: return rows_out_L<512, MODE>(in, out, M1, B, ch, st);
+        case 1024: return rows_out_L<1024, MODE>(in, out, M1, B, ch, st);
+        case 2048: return rows_out_L<2048, MODE>(in, out, M1, B, ch, st);
+        case 4096: return rows_out_L<4096, MODE>(in, out, M1, B, ch, st);
+        case 8192: return rows_out_L<8192, MODE>(in, out, M1, B, ch, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
-// M = M1 M2 of a transform above 8192 points: M1 (the columns) at most 2048,
-// where C = 4 columns fill whole sectors, as long as M2 <= cap
-void split_len(long long M, int cap, int *M1, int *M2)
+template <int L, bool BLU_IN, int MODE>
+cudaError_t one_L(const float2 *in, float2 *out, const float2 *B, const Chirp &ch, cudaStream_t st)
+{
+    using SH = FftShape<L>;
+    const size_t smem = (size_t) SH::G * SH::SMEM * sizeof(float2);
+    cudaError_t e = cudaFuncSetAttribute(k_fft_one<L, BLU_IN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) smem);
+    if (e != cudaSuccess) return e;
+    k_fft_one<L, BLU_IN, MODE><<<1, SH::CTA, smem, st>>>(in, out, B, ch);
+    return cudaGetLastError();
+}
+
+template <bool BLU_IN, int MODE>
+cudaError_t fft_one(int L, const float2 *in, float2 *out, const float2 *B, const Chirp &ch, cudaStream_t st)
+{
+    switch (L) {
+        case 512: return one_L<512, BLU_IN, MODE>(in, out, B, ch, st);
+        case 1024: return one_L<1024, BLU_IN, MODE>(in, out, B, ch, st);
+        case 2048: return one_L<2048, BLU_IN, MODE>(in, out, B, ch, st);
+        case 4096: return one_L<4096, BLU_IN, MODE>(in, out, B, ch, st);
+        case 8192: return one_L<8192, BLU_IN, MODE>(in, out, B, ch, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+// M = M1 M2 of a transform above 8192 points
+void split_len(long long M, int *M1, int *M2)
 {
     int m = 0;
     while ((1LL << m) < M) m++;
-    int a = m / 2;
-    while (a > 11 && (M >> (a - 1)) <= cap) a--;
-    *M1 = 1 << a;
-    *M2 = (int) (M >> a);
+    *M1 = 1 << (m / 2);
+    *M2 = (int) (M / *M1);
 }
 
 }  // namespace
@@ -523,12 +502,12 @@ cudaError_t launch_realfft(const float *series, float2 *out, float2 *scratch, lo
     const float2 *x = reinterpret_cast<const float2 *>(series);
     cudaError_t e;
     if (M <= 8192) {
-        e = fft_rows<ROW_PLAIN>((int) M, x, out, 1, nullptr, M, Chirp{}, st);
+        e = fft_one<false, ROW_PLAIN>((int) M, x, out, nullptr, Chirp{}, st);
     } else {
         int M1, M2;
-        split_len(M, 4096, &M1, &M2);
+        split_len(M, &M1, &M2);
         e = cols<COL_PLAIN>(M1, x, scratch, M2, M, Chirp{}, st);
-        if (e == cudaSuccess) e = rows_out(M2, scratch, out, M1, st);
+        if (e == cudaSuccess) e = rows_out<ROW_PLAIN>(M2, scratch, out, M1, nullptr, Chirp{}, st);
     }
     if (e != cudaSuccess) return e;
     const long long nthr = M / 2 + 1;
@@ -536,14 +515,16 @@ cudaError_t launch_realfft(const float *series, float2 *out, float2 *scratch, lo
     return cudaGetLastError();
 }
 
-// Three passes over memory: the chirped input's columns, the rows with the
-// convolution's product in the middle (the bins stay in the order the first
-// transform leaves them in, and B's with them), the columns back.  (Three
-// whole transforms with their transposes and the products between them took
-// 480 us and two copies at M = 3024000, L = 2^23; the three passes 181 us:
-// 73 + 60 + 49, the first bound by its FP64 chirps and inter-step roots.)
-cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *B, bool build_B,
-                                     long long n, cudaStream_t st)
+// Four passes over memory: the chirped input's columns, the rows with the
+// convolution's product, the second transform's columns, its rows with the
+// chirped output.  (As separate transforms with their transposes and products
+// they were 27 passes: 480 us and two copies at M = 3024000, L = 2^23.
+// Leaving the bins in the first transform's order and going back by rows,
+// then columns, saves a pass and 70 us more, but sums the second transform in
+// another order: where a large mean dominates the series, as in counts off a
+// filterbank, that alone moves the other bins by 1e-5.)
+cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a, float2 *scratch, float2 *B,
+                                     bool build_B, long long n, cudaStream_t st)
 {
     const long long M = n / 2, L = bluestein_len(M);
     if (n % 2 || n < 1024 || M > (1LL << 25)) return cudaErrorInvalidValue;
@@ -553,19 +534,21 @@ cudaError_t launch_realfft_bluestein(const float *series, float2 *out, float2 *a
     if (L <= 8192) {
         if (build_B) {                               // FFT of the chirp kernel, kept per M
             k_blu_kernel<<<(unsigned) ((L + 255) / 256), 256, 0, st>>>(B, ch);
-            e = fft_rows<ROW_PLAIN>((int) L, B, B, 1, nullptr, L, ch, st);
+            e = fft_one<false, ROW_PLAIN>((int) L, B, B, nullptr, ch, st);
         }
-        if (e == cudaSuccess) e = fft_rows<ROW_BLU>((int) L, x, out, 1, B, L, ch, st);
+        if (e == cudaSuccess) e = fft_one<true, ROW_CONV>((int) L, x, a, B, ch, st);
+        if (e == cudaSuccess) e = fft_one<false, ROW_BLU_OUT>((int) L, a, out, nullptr, ch, st);
     } else {
         int M1, M2;
-        split_len(L, 8192, &M1, &M2);
+        split_len(L, &M1, &M2);
         if (build_B) {
-            e = cols<COL_BLU_KERNEL>(M1, nullptr, B, M2, L, ch, st);
-            if (e == cudaSuccess) e = fft_rows<ROW_PLAIN>(M2, B, B, M1, nullptr, L, ch, st);
+            e = cols<COL_BLU_KERNEL>(M1, nullptr, scratch, M2, L, ch, st);
+            if (e == cudaSuccess) e = rows_out<ROW_PLAIN>(M2, scratch, B, M1, nullptr, ch, st);
         }
-        if (e == cudaSuccess) e = cols<COL_BLU_IN>(M1, x, a, M2, L, ch, st);
-        if (e == cudaSuccess) e = fft_rows<ROW_CONV>(M2, a, a, M1, B, L, ch, st);
-        if (e == cudaSuccess) e = cols<COL_BLU_OUT>(M1, a, out, M2, L, ch, st);
+        if (e == cudaSuccess) e = cols<COL_BLU_IN>(M1, x, scratch, M2, L, ch, st);
+        if (e == cudaSuccess) e = rows_out<ROW_CONV>(M2, scratch, a, M1, B, ch, st);
+        if (e == cudaSuccess) e = cols<COL_PLAIN>(M1, a, scratch, M2, L, ch, st);
+        if (e == cudaSuccess) e = rows_out<ROW_BLU_OUT>(M2, scratch, out, M1, nullptr, ch, st);
     }
     if (e != cudaSuccess) return e;
     const long long nthr = M / 2 + 1;

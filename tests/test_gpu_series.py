@@ -145,8 +145,8 @@ def test_device_pointers_off_their_boundary(ctx, ablib):
 @pytest.mark.parametrize("n", [1 << 18, 1 << 20, 1 << 24, 1 << 25, 1 << 26,      # both splits' edges
                                1024 * 3, 16000, 24578, 262218, 3000000, 9000018, 40000014])
 def test_device_realfft_every_split(ctx, n):
-    """The two-pass transform at every pair of lengths and the chirp-z transform at row
-    lengths 512 to 8192, one-row and three-pass, against the FP64 transform on the device."""
+    """The two-pass transform and the chirp-z transform at the pairs of lengths 256 to 8192,
+    and in one CTA, against the FP64 transform on the device."""
     import torch
 
     x = torch.randn(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n))
