@@ -106,6 +106,7 @@ struct ab_ctx {
     DevBuf<ab_bank> dbanks;
     DevBuf<double2> tw64;
     DevBuf<double2> tw_rzw;                 // exp(-2 pi i m / 2^RZW_NMAX_LOG2), jerk polishing
+    DevBuf<double2> fresnel_tab;            // auxiliary Fresnel functions, acceleration polishing
     DevBuf<float2> resp;
 
     // spectrum, scratch, planes
@@ -1127,6 +1128,7 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->dbanks.release();
     ctx->tw64.release();
     ctx->tw_rzw.release();
+    ctx->fresnel_tab.release();
     ctx->resp.release();
     ctx->fft.release();
     ctx->xhat.release();
@@ -1341,6 +1343,14 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
     if (nin > (1 << 24)) return fail(ctx, AB_ERR_ARG, "too many harmonics to polish");
     std::vector<ab_polished> single(each ? (size_t) nin : 0);
     ab_polished *hout = each ? single.data() : out;
+    if (ctx->fresnel_tab.n == 0) {
+        std::vector<double2> tab(POLISH_FRESNEL_TAB);
+        fresnel_table(tab.data());
+        CK(ctx->fresnel_tab.ensure(tab.size()));
+        CK(cudaMemcpyAsync(ctx->fresnel_tab.p, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice,
+                           ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));           // tab is a host vector
+    }
     DevBuf<PolishIn> din;
     DevBuf<ab_polished> dout;
     cudaError_t e = din.ensure((size_t) nin);
@@ -1348,7 +1358,8 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(din.p, in.data(), sizeof(PolishIn) * nin, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess)
-        e = launch_polish(dfft, obs->numbins, obs->lobin, din.p, (int) nin, dout.p, ctx->stream);
+        e = launch_polish(dfft, obs->numbins, obs->lobin, in.data(), din.p, (int) nin, ctx->fresnel_tab.p, dout.p,
+                          ctx->stream);
     if (e == cudaSuccess) ctx->launches++;
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hout, dout.p, sizeof(ab_polished) * nin, cudaMemcpyDeviceToHost, ctx->stream);

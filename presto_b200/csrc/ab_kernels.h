@@ -142,8 +142,11 @@ struct PolishIn {
     int numharm;
     int mode;                   // 0: max_rz_arr_harmonics, 1: max_rz_arr (one harmonic)
 };
-cudaError_t launch_polish(const float2 *data, long long numdata, long long lobin, const PolishIn *in,
-                          int n, ab_polished *out, cudaStream_t st);
+// fresnel_tab: fresnel_table's points on the device
+constexpr int POLISH_FRESNEL_TAB = 353;
+void fresnel_table(double2 *out);
+cudaError_t launch_polish(const float2 *data, long long numdata, long long lobin, const PolishIn *in_host,
+                          const PolishIn *in, int n, const double2 *fresnel_tab, ab_polished *out, cudaStream_t st);
 
 // Jerk-search polishing: one job = one response (gen_z_response or
 // gen_w_response at roffset, numbetween nb, numkern points) and the

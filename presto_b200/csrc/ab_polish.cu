@@ -2,24 +2,27 @@
 // (src/accel_utils.c:552-626) for acceleration searches with harmonic
 // polishing, the reference's default, every candidate of a search at once.
 //
-// One CTA of 256 threads per candidate runs max_rz_arr_harmonics
-// (src/maximize_rz.c:173-228): local powers of the harmonics, two
-// Nelder-Mead stages over (r, z / 4) maximising the sum of the harmonics'
-// locally normalised powers (LOWACC kernels, step 0.4, size tolerance 1e-4;
-// then HIGHACC kernels, step 0.01, 1e-7), then each harmonic's power, local
-// power and derivatives (get_localpower3d, get_derivs3d,
+// A cluster of 1 to 8 CTAs of 512 threads per candidate runs
+// max_rz_arr_harmonics (src/maximize_rz.c:173-228): local powers of the
+// harmonics, two Nelder-Mead stages over (r, z / 4) maximising the sum of the
+// harmonics' locally normalised powers (LOWACC kernels, step 0.4, size
+// tolerance 1e-4; then HIGHACC kernels, step 0.01, 1e-7), then each harmonic's
+// power, local power and derivatives (get_localpower3d, get_derivs3d,
 // src/characteristics.c:79-193).  Complex amplitudes at fractional (r, z)
 // come from rz_interp (src/rzinterp.c:144-232): a warp correlates the data
 // with the FP64 response generated at the fractional offset, lanes splitting
 // the kernel points.  The simplex bookkeeping runs identically in every
-// thread; each function value is reduced by thread 0 in the reference's
+// thread; each function value is summed by one warp in the reference's
 // harmonic order and broadcast through shared memory, so control flow stays
 // uniform.  Iterations are bounded (5000 per stage, as the reference).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include "ab_kernels.h"
 #include "ab_resp.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ab {
 namespace {
@@ -37,12 +40,19 @@ __device__ __forceinline__ int z_halfwidth(double z, bool highacc)   // src/resp
     return (int) (0.5 * 1.1 * fabs(z)) + (highacc ? 48 : 16);
 }
 
+// |z| below the fast points' range (out of line: its registers are not the
+// loop's)
+__device__ __noinline__ double2 slow_point(double frac, double z, int numkern, int c)
+{
+    return z_resp_point(frac, 1, z, numkern, c);
+}
+
 // rz_interp (src/rzinterp.c:144-232) at (r, z) with kernel half-width hw,
 // shared by P warps: this lane of warp part sums kernel points lane + 32 (part
 // + P k) in FP64.  The lanes' and parts' sums add up to the amplitude; the
 // exact-bin cases come from lane 0 of part 0 alone.
-__device__ double2 rz_interp_part(const float2 *data, long long numdata, double r, double z, int hw,
-                                  int part, int P, int lane)
+__device__ __noinline__ double2 rz_interp_part(const float2 *data, long long numdata, double r, double z, int hw,
+                                  int part, int P, int lane, const double2 *tab)
 {
     if (r > numdata - 1.0 || r < 0.0) return make_double2(0.0, 0.0);
     double dint;
@@ -69,8 +79,12 @@ __device__ double2 rz_interp_part(const float2 *data, long long numdata, double 
     const long long hiresp = (hidata > numdata - 1) ? numkern - hidata + numdata - 1 : numkern;
     const long long nsum = hiresp - loresp;
     double ar = 0.0, ai = 0.0;
+    const bool fast = fabs(z) >= 1e-3;
+    ZResp zr;
+    if (fast) zr.init(frac, z, numkern);
     for (long long ii = lane + 32 * part; ii < nsum; ii += 32 * P) {
-        const double2 pv = z_resp_point(frac, 1, z, numkern, (int) (loresp + ii));
+        const double2 pv = fast ? zr.point((int) (loresp + ii), tab)
+                                : slow_point(frac, z, numkern, (int) (loresp + ii));
         const float pr = (float) pv.x, pim = (float) pv.y;      // the reference's response is float
         const float2 d = data[lodata + ii];
         ar += (double) d.x * (double) pr + (double) __fmul_rn(d.y, pim);
@@ -91,41 +105,80 @@ __device__ __forceinline__ double2 warp_sum(double2 v)
 
 // rz_interp by one warp.
 __device__ float2 warp_rz_interp(const float2 *data, long long numdata, double r, double z, int hw,
-                                 int lane)
+                                 int lane, const double2 *tab)
 {
-    const double2 v = warp_sum(rz_interp_part(data, numdata, r, z, hw, 0, 1, lane));
+    const double2 v = warp_sum(rz_interp_part(data, numdata, r, z, hw, 0, 1, lane, tab));
     return make_float2((float) v.x, (float) v.y);
 }
 
 __device__ __forceinline__ double powerf2(float2 a) { return (double) a.x * a.x + (double) a.y * a.y; }
 
+constexpr int PL_MAXK = 8;                    // CTAs (one cluster) per candidate at most
+constexpr int PL_PARTS = PL_MAXK * PL_WARPS;
+
 struct PolishSmem {
+    double2 tab[FRESNEL_TAB];
     double r[PL_ITEMS], z[PL_ITEMS];
     int hw[PL_ITEMS];
     float2 amp[PL_ITEMS];
     int cnt[PL_MAXH];
-    double term[PL_MAXH];
     float locpow[PL_MAXH];
-    double2 part[PL_MAXH];      // per-warp partial amplitudes of one evaluation
+    double2 part[2][PL_PARTS];  // partial amplitudes of one evaluation, by turns
     double val;
+    int nitem;
     int raw;                    // max_rz_arr: one harmonic, raw power (-noharmpolish)
 };
 
-// Amplitudes of items [0, n) (all threads).
-__device__ void interp_items(const float2 *data, long long numdata, int n, PolishSmem &s)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int it = warp; it < n; it += PL_WARPS) {
-        const float2 a = warp_rz_interp(data, numdata, s.r[it], s.z[it], s.hw[it], lane);
-        if (lane == 0) s.amp[it] = a;
+// The cluster's CTAs run the same simplex: each keeps all the partial sums
+// and amplitudes, its own and those that the others' warps store into its
+// shared memory, adds them in the same order and so takes the same turns.  One
+// cluster barrier per evaluation: the partial sums alternate between two
+// buffers, and a CTA passes the barrier behind evaluation n + 1 only after
+// every CTA has read those of evaluation n.
+struct Team {
+    int k, rank, gwarp, nwarps, lane, turn;
+    __device__ __forceinline__ void init()
+    {
+        k = (int) cg::this_cluster().num_blocks();
+        rank = (int) cg::this_cluster().block_rank();
+        gwarp = rank * PL_WARPS + (threadIdx.x >> 5);
+        nwarps = k * PL_WARPS;
+        lane = threadIdx.x & 31;
+        turn = 0;
     }
-    __syncthreads();
+    __device__ __forceinline__ void sync() const
+    {
+        if (k > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    }
+    // *at = v in every CTA's shared memory (lanes of the warp, one CTA each)
+    template <class T> __device__ __forceinline__ void store(T *at, T v) const
+    {
+        if (k == 1) {
+            if (lane == 0) *at = v;
+        } else if (lane < k) {
+            *cg::this_cluster().map_shared_rank(at, lane) = v;
+        }
+    }
+};
+
+// Amplitudes of items [0, n) but those in [skip0, skip1) (all threads of the
+// cluster).
+__device__ void interp_items(const float2 *data, long long numdata, int n, int skip0, int skip1, PolishSmem &s,
+                             const Team &tm)
+{
+    for (int it = tm.gwarp; it < n; it += tm.nwarps) {
+        if (it >= skip0 && it < skip1) continue;
+        const float2 a = warp_rz_interp(data, numdata, s.r[it], s.z[it], s.hw[it], tm.lane, s.tab);
+        tm.store(&s.amp[it], a);
+    }
+    tm.sync();
 }
 
 // get_localpower3d (w = 0) of harmonic n = 1..nh at (r n, z n) into s.locpow
 // (float, as max_rz_arr_harmonics keeps them).
 __device__ void local_powers(const float2 *data, long long numdata, double r, double z, int nh,
-                             PolishSmem &s)
+                             PolishSmem &s, const Team &tm)
 {
     if (threadIdx.x == 0) {
         int k = 0;
@@ -152,12 +205,10 @@ __device__ void local_powers(const float2 *data, long long numdata, double r, do
             }
             s.cnt[ii] = c;
         }
-        s.val = (double) k;
+        s.nitem = k;
     }
-    __syncthreads();
-    const int n = (int) s.val;
-    __syncthreads();
-    interp_items(data, numdata, n, s);
+    tm.sync();                                  // and every CTA is done with its last amplitudes
+    interp_items(data, numdata, s.nitem, 0, 0, s, tm);
     if (threadIdx.x == 0) {
         int k = 0;
         for (int ii = 0; ii < nh; ii++) {
@@ -171,33 +222,36 @@ __device__ void local_powers(const float2 *data, long long numdata, double r, do
 
 // Minus the summed normalised power of the harmonics at (r, zs * ZSCALE)
 // (power_call_rz_harmonics_gsl, src/maximize_rz.c:42-62); all threads.
-__device__ double eval_harmonics(const float2 *data, long long numdata, int nh, int kernhw, double r,
-                                 double zs, PolishSmem &s)
+__device__ __noinline__ double eval_harmonics(const float2 *data, long long numdata, int nh, int kernhw, double r,
+                                 double zs, PolishSmem &s, Team &tm)
 {
-    // P warps per harmonic (all warps busy for few harmonics)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int P = nh >= PL_WARPS ? 1 : PL_WARPS / nh;
-    for (int w = warp; w < nh * P; w += PL_WARPS) {
+    // P warps per harmonic (all warps of the cluster busy for few harmonics)
+    const int P = nh >= tm.nwarps ? 1 : tm.nwarps / nh;
+    double2 *part = s.part[tm.turn];
+    tm.turn ^= 1;
+    for (int w = tm.gwarp; w < nh * P; w += tm.nwarps) {
         const int ii = w / P, n = ii + 1;
         const double2 v = warp_sum(rz_interp_part(data, numdata, r * n, zs * PL_ZSCALE * n, kernhw,
-                                                  w - ii * P, P, lane));
-        if (lane == 0) s.part[w] = v;
+                                                  w - ii * P, P, tm.lane, s.tab));
+        tm.store(&part[w], v);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double total = 0.0;
-        for (int ii = 0; ii < nh; ii++) {
+    tm.sync();
+    // one warp: a lane per harmonic, the sum over harmonics in order
+    if (threadIdx.x < 32) {
+        double term = 0.0;
+        if (tm.lane < nh) {
             double ar = 0.0, ai = 0.0;
             for (int q = 0; q < P; q++) {
-                ar += s.part[ii * P + q].x;
-                ai += s.part[ii * P + q].y;
+                ar += part[tm.lane * P + q].x;
+                ai += part[tm.lane * P + q].y;
             }
             const float2 a = make_float2((float) ar, (float) ai);
-            s.term[ii] = s.raw ? powerf2(a) : powerf2(a) / (double) s.locpow[ii];
-            total += s.term[ii];
+            term = s.raw ? powerf2(a) : powerf2(a) / (double) s.locpow[tm.lane];
         }
+        double total = 0.0;
+        for (int ii = 0; ii < nh; ii++) total += __shfl_sync(0xffffffffu, term, ii);
         // power_call_rz (src/maximize_rz.c:10-23) for one raw power
-        s.val = s.raw ? -total : (isfinite(total) ? -total : 0.0);
+        if (tm.lane == 0) s.val = s.raw ? -total : (isfinite(total) ? -total : 0.0);
     }
     __syncthreads();
     const double v = s.val;
@@ -207,14 +261,14 @@ __device__ double eval_harmonics(const float2 *data, long long numdata, int nh, 
 
 // Nelder-Mead over (r, zs), the oracle's orc_nm_minimize step for step.
 __device__ double nm_minimize(const float2 *data, long long numdata, int nh, int kernhw, double *x,
-                              double step, double tol, PolishSmem &s)
+                              double step, double tol, PolishSmem &s, Team &tm)
 {
     double v[3][2], fv[3], xt[2], xt2[2];
     for (int i = 0; i < 3; i++) {
         v[i][0] = x[0];
         v[i][1] = x[1];
         if (i > 0) v[i][i - 1] += step;
-        fv[i] = eval_harmonics(data, numdata, nh, kernhw, v[i][0], v[i][1], s);
+        fv[i] = eval_harmonics(data, numdata, nh, kernhw, v[i][0], v[i][1], s, tm);
     }
     for (int iter = 0; iter < 5000; iter++) {
         int hi = 0, lo = 0;
@@ -236,11 +290,11 @@ __device__ double nm_minimize(const float2 *data, long long numdata, int nh, int
         // x(t) = (1 - t) c + t x_worst
         xt[0] = 2.0 * c[0] - v[hi][0];
         xt[1] = 2.0 * c[1] - v[hi][1];
-        const double fr = eval_harmonics(data, numdata, nh, kernhw, xt[0], xt[1], s);
+        const double fr = eval_harmonics(data, numdata, nh, kernhw, xt[0], xt[1], s, tm);
         if (fr < fv[lo]) {
             xt2[0] = 3.0 * c[0] - 2.0 * v[hi][0];
             xt2[1] = 3.0 * c[1] - 2.0 * v[hi][1];
-            const double fe = eval_harmonics(data, numdata, nh, kernhw, xt2[0], xt2[1], s);
+            const double fe = eval_harmonics(data, numdata, nh, kernhw, xt2[0], xt2[1], s, tm);
             if (fe < fv[lo]) {
                 v[hi][0] = xt2[0];
                 v[hi][1] = xt2[1];
@@ -258,7 +312,7 @@ __device__ double nm_minimize(const float2 *data, long long numdata, int nh, int
             }
             xt2[0] = 0.5 * c[0] + 0.5 * v[hi][0];
             xt2[1] = 0.5 * c[1] + 0.5 * v[hi][1];
-            const double fc = eval_harmonics(data, numdata, nh, kernhw, xt2[0], xt2[1], s);
+            const double fc = eval_harmonics(data, numdata, nh, kernhw, xt2[0], xt2[1], s, tm);
             if (fc <= fv[hi]) {
                 v[hi][0] = xt2[0];
                 v[hi][1] = xt2[1];
@@ -268,7 +322,7 @@ __device__ double nm_minimize(const float2 *data, long long numdata, int nh, int
                     if (i == lo) continue;
                     v[i][0] = 0.5 * (v[i][0] + v[lo][0]);
                     v[i][1] = 0.5 * (v[i][1] + v[lo][1]);
-                    fv[i] = eval_harmonics(data, numdata, nh, kernhw, v[i][0], v[i][1], s);
+                    fv[i] = eval_harmonics(data, numdata, nh, kernhw, v[i][0], v[i][1], s, tm);
                 }
             }
         } else {
@@ -297,22 +351,25 @@ __device__ double nm_minimize(const float2 *data, long long numdata, int nh, int
 
 __global__ void __launch_bounds__(PL_THREADS) k_polish_rz(const float2 *data, long long numdata,
                                                           long long lobin, const PolishIn *in,
-                                                          ab_polished *out)
+                                                          const double2 *fresnel_tab, ab_polished *out)
 {
     __shared__ PolishSmem s;
-    const PolishIn c = in[blockIdx.x];
-    ab_polished &o = out[blockIdx.x];
+    Team tm;
+    tm.init();
+    const PolishIn c = in[blockIdx.x / tm.k];
+    ab_polished &o = out[blockIdx.x / tm.k];
+    for (int i = threadIdx.x; i < FRESNEL_TAB; i += blockDim.x) s.tab[i] = fresnel_tab[i];
     const int nh = c.mode == 1 ? 1 : (c.numharm < 1 ? 1 : (c.numharm > PL_MAXH ? PL_MAXH : c.numharm));
     if (threadIdx.x == 0) s.raw = c.mode == 1;
     const double rin = c.r - (double) lobin, zin = c.z;
-    local_powers(data, numdata, rin, zin, nh, s);
+    local_powers(data, numdata, rin, zin, nh, s, tm);
     double x[2] = {rin, zin / PL_ZSCALE};
     int kernhw = z_halfwidth(fabs(zin * nh) + 4.0, false);
-    nm_minimize(data, numdata, nh, kernhw, x, 0.4, 1.0e-4, s);
+    nm_minimize(data, numdata, nh, kernhw, x, 0.4, 1.0e-4, s, tm);
     kernhw = z_halfwidth(fabs(x[1] * nh) + 4.0, true);
-    nm_minimize(data, numdata, nh, kernhw, x, 0.01, 1.0e-7, s);
+    nm_minimize(data, numdata, nh, kernhw, x, 0.01, 1.0e-7, s, tm);
     const double rout = x[0], zout = x[1] * PL_ZSCALE;
-    local_powers(data, numdata, rout, zout, nh, s);
+    local_powers(data, numdata, rout, zout, nh, s, tm);
     // harmonic powers (HIGHACC kernel of the second stage) and the five
     // derivative points r n - 0.006 .. + 0.006 (get_derivs3d) per harmonic
     if (threadIdx.x == 0) {
@@ -332,18 +389,11 @@ __global__ void __launch_bounds__(PL_THREADS) k_polish_rz(const float2 *data, lo
             }
         }
     }
-    __syncthreads();
+    tm.sync();
     // items: [0, nh) powers, [PL_MAXH, PL_MAXH + 5 nh) derivative points
-    {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        for (int it = warp; it < PL_MAXH + 5 * nh; it += PL_WARPS) {
-            if (it >= nh && it < PL_MAXH) continue;
-            const float2 a = warp_rz_interp(data, numdata, s.r[it], s.z[it], s.hw[it], lane);
-            if (lane == 0) s.amp[it] = a;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
+    interp_items(data, numdata, PL_MAXH + 5 * nh, nh, PL_MAXH, s, tm);
+    tm.sync();                                  // no CTA leaves while another may store into it
+    if (threadIdx.x == 0 && tm.rank == 0) {
         const double pi = 3.14159265358979323846, twopi = 6.28318530717958647692;
         o.numharm = nh;
         for (int ii = 0; ii < nh; ii++) {
@@ -375,12 +425,75 @@ __global__ void __launch_bounds__(PL_THREADS) k_polish_rz(const float2 *data, lo
 
 }  // namespace
 
-cudaError_t launch_polish(const float2 *data, long long numdata, long long lobin, const PolishIn *in,
-                          int n, ab_polished *out, cudaStream_t st)
+static_assert(FRESNEL_TAB == POLISH_FRESNEL_TAB, "table length");
+
+// f and g at k / FRESNEL_STEPS: the system f' = -pi x g, g' = pi x f - 1 is
+// neutrally stable, so Taylor steps in extended precision carry the asymptotic
+// values at x = 9 (terms below 1e-21) down to 0 with their accuracy.
+void fresnel_table(double2 *out)
+{
+    const long double pi = 3.14159265358979323846264338327950288L;
+    const int k0 = 9 * FRESNEL_STEPS;
+    long double x = 9.0L, h = 1.0L / (pi * x * x), f = 1.0L, g = 1.0L;
+    for (int m = 14; m >= 1; m--) {
+        f = 1.0L - (long double) ((4 * m - 3) * (4 * m - 1)) * h * h * f;
+        g = 1.0L - (long double) ((4 * m - 1) * (4 * m + 1)) * h * h * g;
+    }
+    f *= h * x;
+    g *= h * h * x;
+    const long double d = -1.0L / FRESNEL_STEPS;
+    for (int k = k0; k >= 0; k--) {
+        if (k < FRESNEL_TAB) out[k] = make_double2((double) f, (double) g);
+        x = (long double) k / FRESNEL_STEPS;
+        long double a0 = f, b0 = g, a1 = -pi * x * g, b1 = pi * x * f - 1.0L, p = d;
+        f += a1 * p;
+        g += b1 * p;
+        for (int n = 1; n < 24; n++) {
+            const long double a2 = -pi * (x * b1 + b0) / (n + 1), b2 = pi * (x * a1 + a0) / (n + 1);
+            p *= d;
+            f += a2 * p;
+            g += b2 * p;
+            a0 = a1;
+            b0 = b1;
+            a1 = a2;
+            b1 = b2;
+        }
+    }
+}
+
+// CTAs per candidate.  Its evaluations follow one another, so a candidate's
+// time is a chain: a cluster of up to 8 CTAs (one per SM) shares each evaluation's
+// kernel points while that leaves a thread four of them, which also evens
+// out lists whose candidates differ in length; very long lists fill the SMs
+// on their own.
+static int polish_cluster(const PolishIn *in, int n)
+{
+    double most = 0.0;
+    for (int i = 0; i < n; i++) {
+        const int nh = in[i].mode == 1 ? 1 : in[i].numharm;
+        most = fmax(most, nh * 2.0 * (0.55 * (fabs(in[i].z * nh) + 4.0) + 48.0));
+    }
+    int k = 1;
+    while (k < PL_MAXK && most >= 4.0 * PL_THREADS * k && 2LL * k * n <= 16 * 148) k *= 2;
+    return k;
+}
+
+cudaError_t launch_polish(const float2 *data, long long numdata, long long lobin, const PolishIn *in_host,
+                          const PolishIn *in, int n, const double2 *fresnel_tab, ab_polished *out, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    k_polish_rz<<<n, PL_THREADS, 0, st>>>(data, numdata, lobin, in, out);
-    return cudaGetLastError();
+    const int k = polish_cluster(in_host, n);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned) n * k);
+    cfg.blockDim = dim3(PL_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned) k;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_polish_rz, data, numdata, lobin, in, fresnel_tab, out);
 }
 
 }  // namespace ab

@@ -141,4 +141,106 @@ __device__ __forceinline__ double2 z_resp_point(double roffset, int numbetween, 
     return v;
 }
 
+// ======================================================================
+// Fast response points (candidate polishing).  With the auxiliary functions
+// f and g (Abramowitz & Stegun 7.3.5-6), C + iS at x > 0 is
+//   (1 + i) / 2 - (g + i f) exp(i pi x^2 / 2),
+// and along a response both Fresnel arguments have the phase of the point's
+// own factor exp(-i pi r^2 / z), up to a constant: only the points between the
+// two ends of the drift need a sine and a cosine at all, and f and g vary
+// slowly.  About 170 FP64 operations a point; three sines and cosines, two
+// series term by term and, for 1.8 < x < 5.5, continued fractions of some
+// thirty divisions each took several times that (with up to 8 CTAs a
+// candidate, 160 candidates of a zmax = 600 search with 16 harmonics went from
+// 104 to 39 ms and from 302 to 64 ms; B200).
+// ======================================================================
+constexpr int FRESNEL_STEPS = 64;               // table points per unit of x
+constexpr int FRESNEL_TAB = 353;                // x = 0 .. 5.5
+
+// f and g at x >= 0.  Up to 5.5 the Taylor series about the nearest table
+// point, |d| <= 1/128, its coefficients from f' = -pi x g and g' = pi x f - 1:
+// the first left out is below 1e-18 (f and g are smooth: coefficient n falls
+// like x^-n, and like pi^(n/2) / (n/2)! at 0).  Above, the asymptotic series
+// (7.3.27-28) to m = 11, whose next term is below 1e-18 at 5.5.
+__device__ __forceinline__ void fresnel_fg(double x, const double2 *tab, double &f, double &g)
+{
+    if (x < 5.5) {
+        const int k = __double2int_rn(x * FRESNEL_STEPS);
+        const double x0 = (double) k * (1.0 / FRESNEL_STEPS), d = x - x0;
+        const double2 t = tab[k];
+        double a0 = t.x, b0 = t.y, p = d;
+        double a1 = -M_PI * (x0 * b0), b1 = fma(M_PI, x0 * a0, -1.0);
+        f = fma(a1, p, a0);
+        g = fma(b1, p, b0);
+#pragma unroll
+        for (int n = 1; n < 9; n++) {
+            const double c = M_PI / (n + 1);
+            const double a2 = -c * fma(x0, b1, b0), b2 = c * fma(x0, a1, a0);
+            p *= d;
+            f = fma(a2, p, f);
+            g = fma(b2, p, g);
+            a0 = a1;
+            b0 = b1;
+            a1 = a2;
+            b1 = b2;
+        }
+    } else {
+        const double h = 1.0 / (M_PI * x * x), t = h * h;
+        // f: 1 - 1.3 t + 1.3.5.7 t^2 - ..., g: 1 - 3.5 t + 3.5.7.9 t^2 - ...
+        f = 1.0;
+        g = 1.0;
+#pragma unroll
+        for (int m = 11; m >= 1; m--) {
+            f = fma(-(double) ((4 * m - 3) * (4 * m - 1)) * t, f, 1.0);
+            g = fma(-(double) ((4 * m - 1) * (4 * m + 1)) * t, g, 1.0);
+        }
+        f *= h * x;
+        g *= t * x;
+    }
+}
+
+// What the points of one z response share: gen_z_response at roffset, one
+// point per bin, numkern (even) points.
+struct ZResp {
+    double start, z, zd, cons, pibyz, ec, es;
+    double sgn;
+    __device__ __forceinline__ void init(double roffset, double zz, int numkern)
+    {
+        z = zz;
+        sgn = z < 0.0 ? -1.0 : 1.0;
+        zd = sgn * M_SQRT2 / sqrt(fabs(z));
+        cons = 0.5 * fabs(zd);
+        pibyz = M_PI / z;
+        start = roffset - 0.5 * z + 0.5 * numkern;
+        // the second argument's phase over the first's: 2 pi r + pi z, r = start - c
+        sincospi(2.0 * roffset, &es, &ec);
+    }
+    // |z| >= 1e-3; agrees with z_resp_point to the rounding of its phases
+    __device__ __forceinline__ double2 point(int c, const double2 *tab) const
+    {
+        const double r = start - c, yy = r * zd, zz = yy + z * zd;
+        double fy, gy, fz, gz;
+        fresnel_fg(fabs(yy), tab, fy, gy);
+        fresnel_fg(fabs(zz), tab, fz, gz);
+        fy *= sgn;
+        fz *= sgn;
+        const double wr = gz * ec - fz * es, wi = gz * es + fz * ec;
+        double vr = yy < 0.0 ? -gy : gy, vi = yy < 0.0 ? -fy : fy;
+        if (zz < 0.0) {
+            vr += wr;
+            vi += wi;
+        } else {
+            vr -= wr;
+            vi -= wi;
+        }
+        if (yy < 0.0 && zz >= 0.0) {
+            double sx, cx;
+            sincos(pibyz * r * r, &sx, &cx);
+            vr += cx + sgn * sx;
+            vi += sgn * cx - sx;
+        }
+        return make_double2(cons * vr, cons * vi);
+    }
+};
+
 }  // namespace ab

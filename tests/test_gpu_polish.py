@@ -119,3 +119,24 @@ def test_device_noharmpolish_accel(ctx, ablib, oracle):
                              f"pow {dev['pows'][ii]!r} {p!r} locpow {dev['derivs'][ii][6]!r} "
                              f"{rd.locpow!r}")
     assert not fails, fails
+
+
+def test_device_polish_teams(ctx, ablib, oracle):
+    """One to eight CTAs per candidate (short, long and very long lists of light and heavy
+    candidates), one harmonic or sixteen, drifts on both sides of the fast response's limit:
+    the oracle's optima, and the same numbers wherever a candidate stands in its list."""
+    ft = harmonic_signal(R_HARM, 5.0, 4, 1.0, 99)
+    obs = _obs(ablib, ft.size)
+    light = [(0.0, 0.0, 1, R_HARM + 0.1, z, 0.0) for z in (0.0, 5e-4, 9e-4, -2e-3, 4.0)]
+    heavy = [(0.0, 0.0, 4, R_HARM + 0.1, 4.6, 0.0), (0.0, 0.0, 4, R_HARM - 0.1, 150.0, 0.0)]
+    for base in (light, heavy, light + heavy):
+        orc = oracle.optimize_cands(ft, 0, [(c[2], c[3], c[4]) for c in base], nthreads=8)
+        for n in (1, len(base), 90, 700):
+            cands = [base[k % len(base)] for k in range(n)]
+            dev = ctx.optimize_cands(obs, ft, cands)
+            # a start 145 bins of drift away is a climb over noise: its end is not the oracle's to the bin
+            pick = [k for k in range(min(n, len(base))) if abs(base[k][4]) < 100]
+            _agree([dev[k] for k in pick], [orc[k] for k in pick], ("team", n))
+            for k in range(len(base), n):
+                for key in ("pows", "hirs", "hizs"):
+                    np.testing.assert_array_equal(dev[k][key], dev[k % len(base)][key])
