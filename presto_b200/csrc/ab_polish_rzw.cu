@@ -14,10 +14,11 @@
 //    is computed phase by phase: with N = M P (P <= 4096) and t = M a + b,
 //      X[nb k + s] = sum_b W_N^{k b} W_{nb N}^{s b}
 //                      FFT_P( x[M a + b] W_{nb P}^{s a} )[k mod P],
-//    one FP64 radix-2 FFT of P points in shared memory per (b, s), the
-//    chirp samples of one b kept in shared memory across the nb phases;
-//    only the numkern outputs the reference keeps are formed, rounded to
-//    float as the reference stores its response;
+//    one FP64 radix-16 transform of P points in registers per (b, s), the
+//    chirp samples of one b kept in shared memory across the phases; half
+//    of the phases are conjugates of the others.  Only the numkern outputs
+//    the reference keeps are formed, rounded to float as the reference
+//    stores its response;
 //  * the job's correlation outputs (the 24 r cells of a volume row, or an
 //    rzw_interp point) are FP64 dot products, one warp each.
 // k_rzw_sum then forms the summed, locally normalised powers in float in the
@@ -38,7 +39,8 @@ namespace ab {
 
 namespace {
 
-constexpr int RZW_THREADS = 512;
+constexpr int RZW_THREADS = 256;
+constexpr int RZW_PMIN = 512;               // shortest chirp (next2 of at least 328 samples)
 constexpr long long RZW_NMAX = 1LL << RZW_NMAX_LOG2;
 
 // exp(-2 pi i m / RZW_NMAX) from the half-circle table tw[m] (m < NMAX / 2)
@@ -54,41 +56,203 @@ __device__ __forceinline__ double2 cmul64(double2 a, double2 b)
 {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__device__ __forceinline__ double2 add64(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 sub64(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
-// Forward FP64 FFT of n = 2^log2n points in shared memory (radix 2,
-// decimation in time after a bit reversal).  All threads of the CTA call it;
-// it ends with a barrier.
-__device__ void fft_pow2(double2 *x, int n, int log2n, const double2 *tw)
+// a exp(-2 pi i M / 16)
+template <int M> __device__ __forceinline__ double2 tw16d(double2 a)
 {
-    const long long tstride = RZW_NMAX / n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int j = (int) (__brev((unsigned) i) >> (32 - log2n));
-        if (j > i) {
-            const double2 a = x[i];
-            x[i] = x[j];
-            x[j] = a;
+    constexpr double C = 0.92387953251128675613, S = 0.38268343236508977173, H = 0.70710678118654752440;
+    constexpr int m = M & 15;
+    if constexpr (m == 0) return a;
+    else if constexpr (m == 1) return cmul64(a, make_double2(C, -S));
+    else if constexpr (m == 2) return make_double2(H * (a.x + a.y), H * (a.y - a.x));
+    else if constexpr (m == 3) return cmul64(a, make_double2(S, -C));
+    else if constexpr (m == 4) return make_double2(a.y, -a.x);
+    else if constexpr (m == 6) return make_double2(H * (a.y - a.x), -H * (a.x + a.y));
+    else return cmul64(a, make_double2(-C, S));                     // 9, the last used
+}
+
+__device__ __forceinline__ void dft4d(double2 &a0, double2 &a1, double2 &a2, double2 &a3)
+{
+    const double2 t0 = add64(a0, a2), t1 = sub64(a0, a2), t2 = add64(a1, a3), d = sub64(a1, a3);
+    a0 = add64(t0, t2);
+    a2 = sub64(t0, t2);
+    a1 = make_double2(t1.x + d.y, t1.y - d.x);
+    a3 = make_double2(t1.x - d.y, t1.y + d.x);
+}
+
+// Forward DFT of R points in place, bin k in x[bind<R>(k)].
+template <int R> __device__ __forceinline__ void dftd(double2 *x)
+{
+    if constexpr (R == 2) {
+        const double2 t = x[0];
+        x[0] = add64(t, x[1]);
+        x[1] = sub64(t, x[1]);
+    } else if constexpr (R == 4) {
+        dft4d(x[0], x[1], x[2], x[3]);
+    } else if constexpr (R == 8) {
+        dft4d(x[0], x[2], x[4], x[6]);
+        dft4d(x[1], x[3], x[5], x[7]);
+        const double2 o[4] = {x[1], tw16d<2>(x[3]), tw16d<4>(x[5]), tw16d<6>(x[7])};
+        const double2 e[4] = {x[0], x[2], x[4], x[6]};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            x[k] = add64(e[k], o[k]);
+            x[k + 4] = sub64(e[k], o[k]);
         }
+    } else {
+        // n = 4 n1 + n2, k = k1 + 4 k2, bin k in x[4 k1 + k2]
+#pragma unroll
+        for (int n2 = 0; n2 < 4; n2++) dft4d(x[n2], x[4 + n2], x[8 + n2], x[12 + n2]);
+        x[5] = tw16d<1>(x[5]);
+        x[9] = tw16d<2>(x[9]);
+        x[13] = tw16d<3>(x[13]);
+        x[6] = tw16d<2>(x[6]);
+        x[10] = tw16d<4>(x[10]);
+        x[14] = tw16d<6>(x[14]);
+        x[7] = tw16d<3>(x[7]);
+        x[11] = tw16d<6>(x[11]);
+        x[15] = tw16d<9>(x[15]);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; k1++) dft4d(x[4 * k1], x[4 * k1 + 1], x[4 * k1 + 2], x[4 * k1 + 3]);
     }
-    __syncthreads();
-    for (int lh = 0; lh < log2n; lh++) {
-        const int half = 1 << lh;
-        const long long st = (long long) (n >> (lh + 1)) * tstride;
-        for (int b = threadIdx.x; b < n / 2; b += blockDim.x) {
-            const int k = b & (half - 1);
-            const int i0 = ((b >> lh) << (lh + 1)) + k, i1 = i0 + half;
-            const double2 w = tw[k * st];
-            const double2 u = x[i0], v = cmul64(x[i1], w);
-            x[i0] = make_double2(u.x + v.x, u.y + v.y);
-            x[i1] = make_double2(u.x - v.x, u.y - v.y);
-        }
-        __syncthreads();
+}
+template <int R> __host__ __device__ constexpr int bind(int k) { return R == 16 ? 4 * (k & 3) + (k >> 2) : k; }
+
+// x[q] *= w^q, q = 1..R-1, from w by products (each adds some 1e-16)
+template <int R> __device__ __forceinline__ void twiddle_d(double2 *x, double2 w)
+{
+    double2 p = w;
+#pragma unroll
+    for (int q = 1; q < R; q++) {
+        x[q] = cmul64(x[q], p);
+        if (q + 1 < R) p = cmul64(p, w);
     }
 }
 
-__global__ void __launch_bounds__(RZW_THREADS) k_rzw_jobs(const RzwJob *jobs, const float2 *data,
-                                                          long long numdata, const double2 *tw,
-                                                          float2 *resp_all, double2 *acc_all,
-                                                          const long long *out_j, float2 *out_amp)
+__device__ __forceinline__ int pad16d(int i) { return i + (i >> 4); }
+
+// Forward FP64 transform of P points by P / 16 threads (Stockham, radix 16,
+// 16 and P / 256), point t + (P / 16) m in v[m] before and after.  sm: P +
+// P / 16 points of this transform's own.  All threads of the CTA call it.
+template <int P> __device__ __forceinline__ void fft_d(double2 (&v)[16], double2 *sm, int t, const double2 *tw)
+{
+    constexpr int NT = P / 16, R3 = P / 256, NB3 = 16 / R3;
+    dftd<16>(v);
+#pragma unroll
+    for (int s = 0; s < 16; s++) sm[pad16d(16 * t + s)] = v[bind<16>(s)];
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = sm[pad16d(t + NT * m)];
+    __syncthreads();
+    {
+        const int k = t & 15;
+        twiddle_d<16>(v, tw_at(tw, k * (RZW_NMAX / 256)));
+        dftd<16>(v);
+        const int base = (t - k) * 16 + k;
+#pragma unroll
+        for (int s = 0; s < 16; s++) sm[pad16d(base + 16 * s)] = v[bind<16>(s)];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 16; m++) v[m] = sm[pad16d(t + NT * m)];
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < NB3; b++) {
+        double2 x[R3];
+#pragma unroll
+        for (int q = 0; q < R3; q++) x[q] = v[b + q * NB3];
+        twiddle_d<R3>(x, tw_at(tw, ((t + NT * b) & 255) * (RZW_NMAX / (256 * R3))));
+        dftd<R3>(x);
+#pragma unroll
+        for (int q = 0; q < R3; q++) v[b + q * NB3] = x[bind<R3>(q)];
+    }
+}
+
+// The response of a w job (gen_w_response, src/responses.c:333-418), into
+// resp laid out by phase: output c = nb q + s at resp[s nq + q], nq = numkern
+// / nb.  The chirp is real, so phase nb - s is the conjugate of phase s at
+// bin N - 1 - k: with nb = 8 the transforms of phases 0..4 give all eight.
+// P < 4096 leaves threads for 4096 / P phases at a time.
+template <int P>
+__device__ void chirp_response(const RzwJob &jb, const double2 *tw, double2 *sm, float2 *resp, double2 *acc)
+{
+    constexpr int NT = P / 16, G = RZW_THREADS / NT;
+    const int nb = jb.nb, nq = jb.numkern / nb, N = jb.npts, M = N / P;
+    double *xb = reinterpret_cast<double *>(sm + G * (P + P / 16));        // [P]
+    const double dt = 1.0 / (double) N, amp = 2.0 * dt;
+    const int fbar = N / 4;
+    const double f = ((double) fbar + jb.roffset) - 0.5 * jb.z + jb.w / 12.0;
+    const double fd = (jb.z - 0.5 * jb.w) / 2.0, fdd = jb.w / 6.0;
+    // first kept output g0 = fbar nb - numkern / 2, a multiple of nb
+    const int kbase = fbar - nq / 2;
+    const int nphase = nb / 2 + 1;                              // phases 0 .. nb / 2
+    const long long sP = RZW_NMAX / ((long long) nb * P), sN = RZW_NMAX / N;
+    const int grp = threadIdx.x / NT, t = threadIdx.x - grp * NT;
+    for (int b = 0; b < M; b++) {
+        for (int q = threadIdx.x; q < P; q += RZW_THREADS) {
+            const double u = (double) (q * M + b) * dt;
+            xb[q] = amp * cospi(2.0 * (u * (u * (u * fdd + fd) + f)));
+        }
+        __syncthreads();
+        for (int s0 = 0; s0 < nphase; s0 += G) {
+            const int s = s0 + grp;
+            const bool on = s < nphase;
+            double2 v[16];
+            {
+                // x W_{nb P}^{s q}, q = t + NT m: one root of t and products of another
+                double2 w = tw_at(tw, (long long) s * t * sP);
+                const double2 step = tw_at(tw, (long long) s * NT * sP);
+#pragma unroll
+                for (int m = 0; m < 16; m++) {
+                    const double x = on ? xb[t + NT * m] : 0.0;
+                    v[m] = make_double2(x * w.x, x * w.y);
+                    w = cmul64(w, step);
+                }
+            }
+            fft_d<P>(v, sm + grp * (P + P / 16), t, tw);
+            if (!on) continue;
+            // the phase's own bins, and (mirrored) those of phase nb - s
+            const int smir = (s > 0 && 2 * s < nb) ? nb - s : 0;
+            double2 wsb = make_double2(1.0, 0.0);
+            if (M > 1 && s * b != 0) {
+                double sn, cs;
+                sincospi(-2.0 * (double) (s * b) / ((double) nb * (double) N), &sn, &cs);
+                wsb = make_double2(cs, sn);
+            }
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+                const int k0 = t + NT * m;
+                for (int mir = 0; mir < (smir ? 2 : 1); mir++) {
+                    // q with kbase + q = k0, or N - 1 - (kbase + q) = k0, mod P
+                    int q = mir ? (N - 1 - k0 - kbase) & (P - 1) : (k0 - kbase) & (P - 1);
+                    for (; q < nq; q += P) {
+                        const int k = mir ? N - 1 - (kbase + q) : kbase + q;
+                        double2 y = v[m];
+                        const int c = (mir ? smir : s) * nq + q;
+                        if (M > 1) y = cmul64(y, cmul64(tw_at(tw, (((long long) k * b) & (N - 1)) * sN), wsb));
+                        if (mir) y.y = -y.y;
+                        if (M > 1 && b > 0) y = add64(acc[c], y);
+                        if (b == M - 1) resp[c] = make_float2((float) y.x, (float) y.y);
+                        else acc[c] = y;
+                    }
+                }
+            }
+        }
+        __syncthreads();                    // xb is rewritten next
+    }
+}
+
+// One CTA per response: at most 69 KB of exchange and 32 KB of chirp samples, two
+// CTAs per SM.  Three radix-16 passes in registers move a 4096-point
+// transform through shared memory twice; twelve radix-2 passes in shared
+// memory were bound by its bandwidth (94 % of it).  48 candidates of a zmax = 200,
+// wmax = 300 search with up to 8 harmonics: 22.8 ms before, 10.0 ms so (B200).
+__global__ void __launch_bounds__(RZW_THREADS, 2) k_rzw_jobs(const RzwJob *jobs, const float2 *data,
+                                                             long long numdata, const double2 *tw,
+                                                             float2 *resp_all, double2 *acc_all,
+                                                             const long long *out_j, float2 *out_amp)
 {
     extern __shared__ double2 sm[];
     const RzwJob jb = jobs[blockIdx.x];
@@ -99,73 +263,33 @@ __global__ void __launch_bounds__(RZW_THREADS) k_rzw_jobs(const RzwJob *jobs, co
         }
         return;
     }
-    const int nb = jb.nb, numkern = jb.numkern;
+    const int nb = jb.nb, numkern = jb.numkern, nq = numkern / nb;
     float2 *resp = resp_all + jb.resp_off;
     if (jb.mode == 0) {
         for (int c = threadIdx.x; c < numkern; c += blockDim.x) {
             const double2 v = z_resp_point(jb.roffset, nb, jb.z, numkern, c);
-            resp[c] = make_float2((float) v.x, (float) v.y);
+            resp[c % nb * nq + c / nb] = make_float2((float) v.x, (float) v.y);
         }
     } else {
-        const int N = jb.npts, P = N < RZW_PMAX ? N : RZW_PMAX, M = N / P;
-        const int logP = 31 - __clz(P);
-        double2 *y = sm;                                        // [P]
-        double *xb = reinterpret_cast<double *>(sm + P);        // [P]
-        const double dt = 1.0 / (double) N, amp = 2.0 * dt;
-        const int fbar = N / 4;
-        const double f = ((double) fbar + jb.roffset) - 0.5 * jb.z + jb.w / 12.0;
-        const double fd = (jb.z - 0.5 * jb.w) / 2.0, fdd = jb.w / 6.0;
-        // first kept output g0 = fbar nb - numkern / 2, a multiple of nb
-        const long long kbase = (long long) fbar - numkern / (2 * nb);
-        const long long sP = RZW_NMAX / ((long long) nb * P), sN = RZW_NMAX / N;
-        double2 *acc = (M > 1) ? acc_all + jb.acc_off : nullptr;
-        for (int b = 0; b < M; b++) {
-            for (int q = threadIdx.x; q < P; q += blockDim.x) {
-                const double t = (double) (q * M + b) * dt;
-                xb[q] = amp * cospi(2.0 * (t * (t * (t * fdd + fd) + f)));
-            }
-            for (int s = 0; s < nb; s++) {
-                // same q per thread as above: xb[q] is this thread's own write
-                for (int q = threadIdx.x; q < P; q += blockDim.x) {
-                    const double2 w = tw_at(tw, (long long) s * q * sP);
-                    y[q] = make_double2(xb[q] * w.x, xb[q] * w.y);
-                }
-                __syncthreads();
-                fft_pow2(y, P, logP, tw);
-                double2 wsb = make_double2(1.0, 0.0);
-                if (M > 1 && s * b != 0) {
-                    double sn, cs;
-                    sincospi(-2.0 * (double) (s * b) / ((double) nb * (double) N), &sn, &cs);
-                    wsb = make_double2(cs, sn);
-                }
-                // outputs c = s, s + nb, ...: g = g0 + c = nb (kbase + (c - s) / nb) + s
-                for (int c = s + nb * (int) threadIdx.x; c < numkern; c += nb * (int) blockDim.x) {
-                    const long long k = kbase + (c - s) / nb;
-                    double2 v = y[k & (P - 1)];
-                    if (M == 1) {
-                        resp[c] = make_float2((float) v.x, (float) v.y);
-                    } else {
-                        v = cmul64(v, cmul64(tw_at(tw, ((k * b) & (N - 1)) * sN), wsb));
-                        if (b > 0) v = make_double2(acc[c].x + v.x, acc[c].y + v.y);
-                        if (b == M - 1) resp[c] = make_float2((float) v.x, (float) v.y);
-                        else acc[c] = v;
-                    }
-                }
-                __syncthreads();            // y and xb are rewritten next
-            }
-        }
+        double2 *acc = acc_all + jb.acc_off;
+        if (jb.npts >= RZW_PMAX) chirp_response<4096>(jb, tw, sm, resp, acc);
+        else if (jb.npts == 2048) chirp_response<2048>(jb, tw, sm, resp, acc);
+        else if (jb.npts == 1024) chirp_response<1024>(jb, tw, sm, resp, acc);
+        else chirp_response<RZW_PMIN>(jb, tw, sm, resp, acc);
     }
     __syncthreads();                        // the response is visible to the whole CTA
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     for (int o = warp; o < jb.nout; o += nwarp) {
         const long long j = out_j[jb.j_off + o];
-        const long long i0 = j >= 0 ? (j + nb - 1) / nb : -((-j) / nb);
+        // response point nb i - j = nb (i - a) + s, a = ceil(j / nb)
+        const long long a = j >= 0 ? (j + nb - 1) / nb : -((-j) / nb);
+        const float2 *r = resp + (nb * a - j) * nq - a;
         const long long i1 = (numkern - 1 + j) / nb;
         double ar = 0.0, ai = 0.0;
-        for (long long i = i0 + lane; i <= i1; i += 32) {
+        for (long long i = a + lane; i <= i1; i += 32) {
             const long long bi = jb.beginbin + i;
             if (bi < 0 || bi >= numdata) continue;
-            const float2 d = data[bi], p = resp[nb * i - j];
+            const float2 d = data[bi], p = r[i];
             ar += (double) d.x * p.x + (double) d.y * p.y;
             ai += (double) d.y * p.x - (double) d.x * p.y;
         }
@@ -246,7 +370,7 @@ cudaError_t launch_rzw_jobs(const RzwJob *jobs, int njobs, const float2 *data, l
                             float2 *out_amp, cudaStream_t st)
 {
     if (njobs <= 0) return cudaSuccess;
-    const size_t smem = (size_t) RZW_PMAX * (sizeof(double2) + sizeof(double));
+    const size_t smem = (size_t) (RZW_PMAX + RZW_PMAX / 16) * sizeof(double2) + RZW_PMAX * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(k_rzw_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int) smem);
     if (e != cudaSuccess) return e;
@@ -311,7 +435,7 @@ struct Plan {
     }
     void check_chirp(const RzwJob &jb)
     {
-        if (jb.npts > RZW_NMAX || (jb.npts / 4) * jb.nb < jb.numkern / 2) {
+        if (jb.npts > RZW_NMAX || jb.npts < RZW_PMIN || (jb.npts / 4) * jb.nb < jb.numkern / 2) {
             bad = true;
             snprintf(msg, sizeof msg, "response (z %.1f, w %.1f) needs %d chirp samples, "
                      "above %lld", jb.z, jb.w, jb.npts, RZW_NMAX);

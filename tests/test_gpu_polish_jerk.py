@@ -137,3 +137,20 @@ def test_device_noharmpolish_jerk(ctx, ablib, oracle, jerk_case):
             dd = d["derivs"][ii]
             assert abs(dd[0] - rd.pow) <= 1e-4 * rd.pow
             assert abs(dd[6] - rd.locpow) <= 1e-4 * rd.locpow
+
+
+@pytest.mark.parametrize("z,w", [(4.0, 20.0), (-101.0, 60.0), (301.0, -140.0), (-598.0, 100.0), (901.0, 260.0)])
+def test_device_rzw_chirp_lengths(ctx, ablib, oracle, jerk_case, z, w):
+    """Responses from chirps of 512, 1024, 2048, 4096 and 8192 samples (one transform, several phases
+    at a time, and one of two interleaved parts), the mirrored phases among them."""
+    ft, _ = jerk_case
+    obs = _obs(ablib, ft.size, zmax=1000, wmax=300, numharm=1)
+    r = ft.size / 2 + 17.25
+    dev = ctx.optimize_cands(obs, ft, [(0.0, 0.0, 1, r, z, w)])
+    orc = oracle.optimize_cands_w(ft, 0, [(1, r, z, w)], jerk=True, nthreads=os.cpu_count() or 1)
+    for k in ("hirs", "hizs", "hiws"):
+        np.testing.assert_array_equal(dev[0][k], orc[0][k])
+    # noise cells: amplitudes are sums of some 1000 products with responses rounded
+    # to float on both sides
+    assert np.allclose(dev[0]["pows"], orc[0]["pows"], rtol=1e-4)
+    assert np.allclose(dev[0]["derivs"][:, 6], orc[0]["derivs"][:, 6], rtol=1e-4)
