@@ -128,17 +128,17 @@ int  ab_ctx_set_hbm_budget(ab_ctx *ctx, size_t bytes);
 int  ab_ctx_set_corr_path(ab_ctx *ctx, int path);
 
 /* Transform schedule (no counterpart in the reference, whose FFT length per
- * harmonic is calc_fftlen's, src/accel_utils.c:137-150).  The whole-spectrum
- * search correlates each bank with a device FFT of length L (512..8192) that
- * serves m consecutive blocks (1..8, only where the reference's own transform
- * does not wrap); L and m minimise the correlation cost per block under a
- * process-wide table of costs per template and transform, indexed by log2 L
- * (AB_COST_SLOTS = 16 entries; a length whose entry is <= 0 is not used for
- * superblocks).  The library starts with a table measured on B200 for 512 to
- * 4096 points; ab_autotune re-measures those on the context's device and
- * installs them (costs_out may be NULL).  Set the table before creating the
- * banks a search, ab_bank_geometry or ab_fderivs_vol_noalloc rely on: the
- * template length follows it. */
+ * harmonic is calc_fftlen's, src/accel_utils.c:137-150): the template length
+ * L (512..8192) of ab_bank_geometry, ab_bank_kernel and
+ * ab_fderivs_vol_noalloc.  L and a number of blocks m (1..8, only where the
+ * reference's own transform does not wrap) minimise the correlation cost per
+ * block if m blocks shared a transform, under a process-wide table of costs per
+ * template and transform, indexed by log2 L (AB_COST_SLOTS = 16 entries; a
+ * length whose entry is <= 0 is not used for m > 1).  The library starts
+ * with a table measured on B200 for 512 to 4096 points; ab_autotune
+ * re-measures those on the context's device and installs them (costs_out may
+ * be NULL).  Set the table before asking for templates: their length follows
+ * it.  Searches and plane calls correlate segments of their own choice. */
 int  ab_set_transform_costs(const double *costs, int n);
 int  ab_get_transform_costs(double *costs, int n);
 int  ab_autotune(ab_ctx *ctx, double *costs_out, int n);
@@ -149,7 +149,7 @@ int ab_obs_init(const ab_params *p, ab_obs *obs);
 /* Template-bank geometry of obs in the reference's harmonic order (host
  * only).  info[9*k ..] = numharm, harmnum, numkern_zdim, numkern_wdim,
  * reference fftlen, device FFT length, kernel half width, largest numrs,
- * blocks per device transform in the whole-spectrum search. */
+ * blocks that the cost table would have share a transform of that length. */
 int ab_bank_geometry(const ab_obs *obs, int *nbanks, int *info, int maxbanks);
 
 /* Number of blocks of the main search loop (src/accelsearch.c:187-224). */
@@ -258,8 +258,8 @@ int ab_block_stage_sums(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft_h
 int ab_gen_response(ab_ctx *ctx, double roffset, int numbetween, double z, double w,
                     int numkern, ab_fcomplex *out);
 
-/* The FFT'd template (w index wi, z index zi) of bank (numharm, harmnum)
- * as stored on the device, and its device FFT length. */
+/* The FFT'd template (w index wi, z index zi) of bank (numharm, harmnum) on
+ * ab_bank_geometry's device FFT length, and that length. */
 int ab_bank_kernel(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int wi, int zi,
                    ab_fcomplex *out, int maxlen, int *fftlen_dev);
 

@@ -278,7 +278,7 @@ def num_blocks(obs):
 
 def bank_geometry(obs):
     """Per template bank: dict(numharm, harmnum, nz, nw, fftlen_ref, L, hw, numrs_max,
-    sbm = blocks per device transform in the whole-spectrum search)."""
+    sbm = blocks that the cost table would have share a transform of L points)."""
     n = C.c_int()
     rc = lib().ab_bank_geometry(C.byref(obs), C.byref(n), None, 0)
     if rc:
@@ -308,8 +308,8 @@ def get_transform_costs():
 
 
 def set_transform_costs(costs):
-    """Install a cost table (by log2 L); it chooses transform lengths and
-    superblock heights of banks built afterwards."""
+    """Install a cost table (by log2 L); it chooses the template lengths of
+    bank_geometry, bank_kernel and the allocation-free entry point."""
     c = (C.c_double * COST_SLOTS)(*[float(x) for x in list(costs)[:COST_SLOTS]])
     rc = lib().ab_set_transform_costs(c, COST_SLOTS)
     if rc:

@@ -1,0 +1,422 @@
+// ab_corr.cu -- template correlation of the searches and plane calls: the
+// f-fdot planes of subharm_fderivs_vol (src/accel_utils.c:1025-1210) as a
+// sliding correlation over segments of the spectrum.
+//
+// A bank's sub-planes of consecutive blocks lie side by side on one half-bin
+// column grid, and a cell depends on the bins within its template's half
+// width only, so the columns need not be correlated block by block.  They are
+// cut into segments of V = 2048 - 4 hw columns, whatever the blocks, each from
+// one 1024-bin window of the spectrum, hw being the widest half width of a
+// class of templates: wide templates get short segments, narrow ones long
+// ones.  (Transforms over one block or a few whole ones spend a third to a
+// half of their length on overlap: all templates pay for the widest one's, and
+// block lengths do not fit the transform's.  zmax = 600 with 16 harmonics at
+// N = 2^23: 4.5 million transforms of 4096 points, 134 ms; now 22 million
+// pairs of 1024 points, 120 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
+// 225 ms.)  Each block keeps its own normalisation: a segment
+// is transformed with its first block's and a column's powers are scaled by
+// its own block's over that, squared.
+//
+// Banks whose reference transform wraps into valid cells, and the local-power
+// normalisation (a factor per bin and block), need every block's own data:
+// their segments are cut from one block's window, periodic as in the
+// reference's circular correlation.
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include "ab_fft.cuh"
+#include "ab_index.h"
+#include "ab_kernels.h"
+#include "ab_norm.cuh"
+
+namespace ab {
+
+constexpr int SEG_H = AB_SEG_BINS;          // bins of a segment's window
+constexpr int SEG_WARPS = 8;                // warps per CTA, two to a template
+constexpr int SEG_MAXBLK = 256;             // blocks that share one segment
+constexpr int SEG_P = 34;                   // exchange row stride (points): 16-byte rows, no conflicts
+
+// ---------------------------------------------------------------------------
+// radix 32 in registers
+// ---------------------------------------------------------------------------
+// a exp(2 pi i M / 32)
+template <int M> __device__ __forceinline__ float2 tw32(float2 a)
+{
+    constexpr int m = M & 31;
+    if constexpr (m == 0) {
+        return a;
+    } else if constexpr (m % 8 == 0) {
+        return m == 8 ? mul_i<1>(a) : m == 16 ? make_float2(-a.x, -a.y) : mul_i<-1>(a);
+    } else {
+        // cos and sin of pi k / 16
+        constexpr double C[9] = {1.0, 0.98078528040323044913, 0.92387953251128675613,
+                                 0.83146961230254523708, 0.70710678118654752440,
+                                 0.55557023301960222474, 0.38268343236508977173,
+                                 0.19509032201612826785, 0.0};
+        constexpr int q = m / 8, k = m % 8;
+        constexpr double c0 = C[k], s0 = C[8 - k];
+        constexpr float c = (float) (q == 0 ? c0 : q == 1 ? -s0 : q == 2 ? -c0 : s0);
+        constexpr float s = (float) (q == 0 ? s0 : q == 1 ? c0 : q == 2 ? -s0 : -c0);
+        return cmul(a, make_float2(c, s));
+    }
+}
+
+// x[n2 + 8 K1] *= w32^(n2 K1)
+template <int K1> __device__ __forceinline__ void tw32_row(float2 (&x)[32])
+{
+    x[8 * K1 + 1] = tw32<1 * K1>(x[8 * K1 + 1]);
+    x[8 * K1 + 2] = tw32<2 * K1>(x[8 * K1 + 2]);
+    x[8 * K1 + 3] = tw32<3 * K1>(x[8 * K1 + 3]);
+    x[8 * K1 + 4] = tw32<4 * K1>(x[8 * K1 + 4]);
+    x[8 * K1 + 5] = tw32<5 * K1>(x[8 * K1 + 5]);
+    x[8 * K1 + 6] = tw32<6 * K1>(x[8 * K1 + 6]);
+    x[8 * K1 + 7] = tw32<7 * K1>(x[8 * K1 + 7]);
+}
+
+// Inverse (+i) DFT of 32 points in place: n = 8 n1 + n2, k = k1 + 4 k2; bin k
+// is left in x[bin32(k)].
+__device__ __forceinline__ void dft32(float2 (&x)[32])
+{
+#pragma unroll
+    for (int n2 = 0; n2 < 8; n2++) dft4v<1>(x[n2], x[8 + n2], x[16 + n2], x[24 + n2]);
+    tw32_row<1>(x);
+    tw32_row<2>(x);
+    tw32_row<3>(x);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++) dft8<1>(x + 8 * k1);
+}
+__host__ __device__ constexpr int bin32(int k) { return 8 * (k & 3) + (k >> 2); }
+
+// Spectra, twiddles and templates are laid out for lanes that hold points
+// l + 32 m of 1024: points 64 p + l and 64 p + 32 + l side by side, 16 bytes a
+// lane.
+__host__ __device__ constexpr int seg_place(int k) { return (k & ~63) + 2 * (k & 31) + ((k >> 5) & 1); }
+
+// ---------------------------------------------------------------------------
+// columns and normalisations
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ ab_hgeom seg_geom(const SearchConsts &sc, const ab_bank &b, double startr)
+{
+    return ab_harm_geom(startr, startr + sc.rstep - AB_DR, b.numharm, b.harmnum, sc.obs_zlo, sc.obs_wlo,
+                        sc.corr_uselen);
+}
+
+// Per (bank, block): the block's columns and its normalisation (1 / sqrt of
+// the median power / ln 2 of its own window, or photon counts).  A window
+// with a value that is not finite, or a median of zero, makes every cell of
+// the block NaN in the block's own transform: its normalisation is NaN, and
+// the bad bins count as zero for the blocks beside it (k_seg_fwd), whose
+// windows do not hold them.  Blocks of banks correlated by their own data
+// get theirs from k_prep_time.
+__global__ void __launch_bounds__(256) k_seg_cols(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
+                                                  const float2 *fft, SegCols *cols, double *norms)
+{
+    extern __shared__ float spw[];
+    __shared__ double s_norm;
+    const ab_bank b = banks[blockIdx.y];
+    const int j = blockIdx.x;
+    const ab_hgeom g = seg_geom(sc, b, bb.startr[j]);
+    const long long at = (long long) blockIdx.y * bb.nblk + j;
+    if (threadIdx.x == 0) {
+        long long lim = sc.inmem ? g.numrs : min(g.numrs, b.numrs_max);
+        if (sc.inmem && j >= bb.npre0) lim = min(lim, sc.clip_col - g.rlo * AB_RDR);
+        cols[at] = SegCols{g.rlo * AB_RDR, (int) max(lim, 0ll), 0};
+    }
+    if (b.own_data) return;
+    const long long lobin = g.rlo - b.hw0;
+    const int numdata = b.fftlen_ref / AB_NUMBETWEEN;
+    bool bad = false;
+    for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
+        const long long bin = lobin + i - sc.obs_lobin;
+        if (bin >= 0 && bin < sc.numbins) {
+            const float2 v = fft[bin];
+            bad |= !(isfinite(v.x) && isfinite(v.y));
+        }
+    }
+    bad = __syncthreads_or(bad);
+    const double n = block_norm(sc, lobin, numdata, fft, spw, &s_norm);
+    if (threadIdx.x == 0) norms[at] = (bad || !isfinite(n)) ? (double) NAN : n;
+}
+
+__device__ __forceinline__ const SegGroup &group_of_unit(const SegGroup *g, int ng, int unit)
+{
+    int lo = 0, hi = ng - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (g[mid].unit0 <= unit) lo = mid;
+        else hi = mid - 1;
+    }
+    return g[lo];
+}
+
+__device__ __forceinline__ const SegGroup &group_of_cta(const SegGroup *g, int ng, int cta)
+{
+    int lo = 0, hi = ng - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (g[mid].cta0 <= cta) lo = mid;
+        else hi = mid - 1;
+    }
+    return g[lo];
+}
+
+// first block of [0, n) whose columns reach past column q
+__device__ __forceinline__ int first_block(const SegCols *c, int n, long long q)
+{
+    int lo = 0, hi = n - 1;                     // last block that starts at or before q
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (c[mid].c0 <= q) lo = mid;
+        else hi = mid - 1;
+    }
+    while (lo > 0 && c[lo - 1].c0 + c[lo - 1].lim > q) lo--;
+    return lo;
+}
+
+// The normalisation a unit's data carry: of its first block, or of the first
+// one after it that has one.
+__device__ __forceinline__ double unit_norm(const double *nm, int j0, int n)
+{
+    for (int j = j0; j < n && j < j0 + SEG_MAXBLK; j++)
+        if (nm[j] > 0.0 && isfinite(nm[j])) return nm[j];
+    return 1.0;
+}
+
+// Forward transforms of the units' windows, four per CTA.
+__global__ void __launch_bounds__(256) k_seg_fwd(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
+                                                 const SegGroup *groups, int ngroups, int nunits,
+                                                 const SegCols *cols, const double *norms, const float2 *fft,
+                                                 const float2 *dtime, long long dt_per_block, float2 *xhat)
+{
+    using SH = FftShape<SEG_H>;
+    extern __shared__ float2 fsm[];
+    const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
+    const int unit = blockIdx.x * SH::G + grp;
+    const bool ok = unit < nunits;
+    const SegGroup g = group_of_unit(groups, ngroups, ok ? unit : nunits - 1);
+    const ab_bank b = banks[g.bank];
+    const int u = (ok ? unit : nunits - 1) - g.unit0;
+    float2 v[16];
+    if (g.nsub) {
+        const int j = g.blk0 + u / g.nsub, off = u % g.nsub * (g.V / 2) + b.hw0 - g.hw;
+        const int numdata = b.fftlen_ref / AB_NUMBETWEEN;
+        const float2 *d = dtime + j * dt_per_block + b.dtime_off;
+#pragma unroll
+        for (int m = 0; m < 16; m++) v[m] = d[(off + t + SH::NT * m) % numdata];
+    } else {
+        const SegCols *c = cols + (long long) g.bank * bb.nblk + g.blk0;
+        const long long q = c[0].c0 + (long long) u * g.V;
+        const int j0 = first_block(c, g.nblk, q);
+        const double norm = unit_norm(norms + (long long) g.bank * bb.nblk + g.blk0, j0, g.nblk);
+        const long long bin0 = q / 2 - g.hw - sc.obs_lobin;
+#pragma unroll
+        for (int m = 0; m < 16; m++) {
+            const long long bin = bin0 + t + SH::NT * m;
+            float2 x = make_float2(0.f, 0.f);
+            if (bin >= 0 && bin < sc.numbins) {
+                const float2 a = fft[bin];
+                if (isfinite(a.x) && isfinite(a.y))
+                    x = make_float2((float) ((double) a.x * norm), (float) ((double) a.y * norm));
+            }
+            v[m] = x;
+        }
+    }
+    FftTw<SEG_H, -1> tw;
+    tw.init(t);
+    fft_run<SEG_H, -1>(v, fsm + grp * SH::SMEM, t, tw);
+    if (!ok) return;
+    float2 *o = xhat + (long long) unit * SEG_H;
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const int k = t + SH::NT * m;
+        o[seg_place(k)] = v[m];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// correlation
+// ---------------------------------------------------------------------------
+constexpr int TW_OFF = SEG_H;                                   // float2
+constexpr int EX_OFF = 2 * SEG_H;
+constexpr size_t SEG_SMEM = sizeof(float2) * (EX_OFF + SEG_WARPS * 32 * SEG_P);
+
+// One CTA: one unit (segment) and a tile of its class's templates.  A warp
+// takes one of a template's two 1024-point inverse transforms (even or odd
+// columns), 32 points a lane: radix 32 over the points 32 apart, the twiddles,
+// one exchange through the warp's own shared memory, radix 32 again -- no
+// barrier between warps and 8 bytes of exchange each way per point, where
+// radix 16 needs two exchanges behind CTA barriers at 4096 points.
+// Measured (B200, N = 2^20, zmax = 200): 5.4 to 5.7 ns per template and segment;
+// shared memory and L1 data path 58 % busy, FP32 pipe 38 %, issue 47 %: held by
+// latencies at the 16 warps that 128 registers leave an SM.  Both transforms
+// of a template in one warp's paired FP32 instructions halve the issue but
+// leave 8 warps: 20 % slower.  Prefetching the next template into L1: 3 % slower;
+// loads and butterflies interleaved by hand, or one body for both passes: the
+// same.
+__global__ void __launch_bounds__(32 * SEG_WARPS, 2)
+    k_corr_seg(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
+               const SegCols *cols, const double *norms, const float2 *xhat, const float2 *tmpl,
+               const int *perm, float *planes, long long plane_per_block)
+{
+    extern __shared__ __align__(16) float2 fsm[];
+    __shared__ int4 s_blk[SEG_MAXBLK];          // first column, columns, offset, scale of a block here
+    __shared__ int4 s_first[32];                // the first block of each group of 64 columns
+    __shared__ unsigned char s_jlo[32], s_more[32];
+    __shared__ float *s_out;
+    __shared__ long long s_pitch;
+    __shared__ unsigned s_any;                  // bit k: group k of 64 columns has further blocks
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const SegGroup g = group_of_cta(groups, ngroups, blockIdx.x);
+    const int r0 = blockIdx.x - g.cta0, u = r0 % g.nunits, tile = r0 / g.nunits;
+    const ab_bank b = banks[g.bank];
+    {
+        const float4 *src = reinterpret_cast<const float4 *>(xhat + (long long) (g.unit0 + u) * SEG_H);
+        float4 *dst = reinterpret_cast<float4 *>(fsm);
+        for (int i = threadIdx.x; i < SEG_H / 2; i += blockDim.x) dst[i] = src[i];
+        // twiddles exp(2 pi i l s / 1024) of lane l, bin s
+        for (int i = threadIdx.x; i < SEG_H; i += blockDim.x) {
+            double s, c;
+            sincospi((double) (((i & 31) * (i >> 5)) & (SEG_H - 1)) * (2.0 / SEG_H), &s, &c);
+            fsm[TW_OFF + seg_place(i)] = make_float2((float) c, (float) s);
+        }
+    }
+    // the blocks whose columns this unit holds, in transform columns
+    const SegCols *c = cols + (long long) g.bank * bb.nblk + g.blk0;
+    const double *nm = norms + (long long) g.bank * bb.nblk + g.blk0;
+    const int j0 = g.nsub ? u / g.nsub : first_block(c, g.nblk, c[0].c0 + (long long) u * g.V);
+    const long long q = g.nsub ? c[j0].c0 + (long long) (u % g.nsub) * g.V : c[0].c0 + (long long) u * g.V;
+    int nj = 1;
+    if (!g.nsub)
+        while (nj < SEG_MAXBLK && j0 + nj < g.nblk && c[j0 + nj].c0 < q + g.V) nj++;
+    const double ref = g.nsub ? 1.0 : unit_norm(nm, j0, g.nblk);
+    for (int j = threadIdx.x; j < nj; j += blockDim.x) {
+        const int tc0 = (int) (c[j0 + j].c0 - q) + 2 * g.hw;
+        const int lo = max(tc0, 2 * g.hw), hi = min(tc0 + c[j0 + j].lim, 2 * g.hw + g.V);
+        // element of this block's transform column 0, from the first block's
+        const long long off = sc.inmem ? c[j0 + j].c0 - c[j0].c0 - tc0 : (long long) j * plane_per_block - tc0;
+        const double r = nm[j0 + j] / ref;
+        s_blk[j] = make_int4(lo, max(hi - lo, 0), (int) off,
+                             __float_as_int((float) (r * r) * (1.0f / ((float) SEG_H * SEG_H))));
+    }
+    if (threadIdx.x == 0) {
+        s_out = planes + (sc.inmem ? c[j0].c0 : (long long) (g.blk0 + j0) * plane_per_block + b.plane_off);
+        s_pitch = sc.inmem ? sc.rlen : b.numrs_max;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int k0 = 64 * threadIdx.x;
+        int a = 0, n = 0;
+        for (int j = 0; j < nj; j++) {
+            const int4 e = s_blk[j];
+            if (e.y > 0 && e.x < k0 + 64 && e.x + e.y > k0) {
+                if (n == 0) a = j;
+                n = j - a + 1;
+            }
+        }
+        s_first[threadIdx.x] = n ? s_blk[a] : make_int4(0, 0, 0, 0);
+        s_jlo[threadIdx.x] = (unsigned char) a;
+        s_more[threadIdx.x] = (unsigned char) (n > 1 ? n - 1 : 0);
+        const unsigned any = __ballot_sync(0xffffffffu, n > 1);
+        if (threadIdx.x == 0) s_any = any;
+    }
+    __syncthreads();
+    const float4 *xs = reinterpret_cast<const float4 *>(fsm) + lane;
+    const float4 *tws = reinterpret_cast<const float4 *>(fsm + TW_OFF) + lane;
+    float2 *ex = fsm + EX_OFF + warp * 32 * SEG_P;
+    const float4 *ex4 = reinterpret_cast<const float4 *>(ex + lane * SEG_P);
+    const int par = warp & 1;
+    const float4 *k0 = reinterpret_cast<const float4 *>(tmpl + b.seg_tmpl_off + par * SEG_H) + lane;
+    const int *tp = perm + g.t_lo + tile * g.tile + (warp >> 1);
+    const int *tend = perm + g.t_lo + min(g.nt, (tile + 1) * g.tile);
+    for (; tp < tend; tp += SEG_WARPS / 2) {
+        const int tl = *tp;
+        const float4 *kp = k0 + (long long) tl * SEG_H;
+        float2 v[32];
+#pragma unroll
+        for (int p = 0; p < 16; p++) {
+            const float4 k = __ldg(kp + 32 * p);
+            v[2 * p] = make_float2(k.x, k.y);
+            v[2 * p + 1] = make_float2(k.z, k.w);
+        }
+#pragma unroll
+        for (int p = 0; p < 16; p++) {
+            const float4 x = xs[32 * p];
+            v[2 * p] = cmulc(make_float2(x.x, x.y), v[2 * p]);
+            v[2 * p + 1] = cmulc(make_float2(x.z, x.w), v[2 * p + 1]);
+        }
+        dft32(v);
+#pragma unroll
+        for (int p = 0; p < 16; p++) {
+            const float4 w = tws[32 * p];
+            const float2 y = v[bin32(2 * p)];
+            ex[(2 * p) * SEG_P + lane] = p ? cmul(y, make_float2(w.x, w.y)) : y;
+            ex[(2 * p + 1) * SEG_P + lane] = cmul(v[bin32(2 * p + 1)], make_float2(w.z, w.w));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 16; p++) {
+            const float4 y = ex4[p];
+            v[2 * p] = make_float2(y.x, y.y);
+            v[2 * p + 1] = make_float2(y.z, y.w);
+        }
+        __syncwarp();
+        dft32(v);
+        float *row = s_out + tl * s_pitch;
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+            float2 &y = v[bin32(k)];
+            y.x = fmaf(y.x, y.x, y.y * y.y);
+            const int col = 64 * k + 2 * lane + par;
+            const int4 e = s_first[k];
+            if ((unsigned) (col - e.x) < (unsigned) e.y) row[e.z + col] = y.x * __int_as_float(e.w);
+        }
+        if (const unsigned more = s_any) {
+#pragma unroll
+            for (int k = 0; k < 32; k++) {
+                if (!((more >> k) & 1u)) continue;
+                const int col = 64 * k + 2 * lane + par;
+                for (int j = s_jlo[k] + 1, n = s_more[k]; n > 0; n--, j++) {
+                    const int4 f = s_blk[j];
+                    if ((unsigned) (col - f.x) < (unsigned) f.y)
+                        row[f.z + col] = v[bin32(k)].x * __int_as_float(f.w);
+                }
+            }
+        }
+    }
+}
+
+cudaError_t launch_seg_cols(const ab_bank *banks_dev, int nbanks, const SearchConsts &sc, const BlockBatch &bb,
+                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, cudaStream_t st)
+{
+    const size_t smem = sizeof(float) * (size_t) numdata_max;
+    if (smem > 48 * 1024) return cudaErrorInvalidValue;
+    k_seg_cols<<<dim3((unsigned) bb.nblk, (unsigned) nbanks), 256, smem, st>>>(banks_dev, sc, bb, fft, cols, norms);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_seg_fwd(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                           const SegGroup *groups, int ngroups, int nunits, const SegCols *cols,
+                           const double *norms, const float2 *fft, const float2 *dtime, long long dt_per_block,
+                           float2 *xhat, cudaStream_t st)
+{
+    using SH = FftShape<SEG_H>;
+    if (nunits <= 0) return cudaSuccess;
+    k_seg_fwd<<<(unsigned) ((nunits + SH::G - 1) / SH::G), SH::CTA, (size_t) SH::G * SH::SMEM * sizeof(float2), st>>>(
+        banks_dev, sc, bb, groups, ngroups, nunits, cols, norms, fft, dtime, dt_per_block, xhat);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_corr_seg(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                            const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
+                            const double *norms, const float2 *xhat, const float2 *tmpl, const int *perm,
+                            float *planes, long long plane_per_block, cudaStream_t st)
+{
+    if (nctas <= 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k_corr_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SEG_SMEM);
+    if (e != cudaSuccess) return e;
+    k_corr_seg<<<(unsigned) nctas, 32 * SEG_WARPS, SEG_SMEM, st>>>(banks_dev, sc, bb, groups, ngroups, cols, norms,
+                                                                  xhat, tmpl, perm, planes, plane_per_block);
+    return cudaGetLastError();
+}
+
+}  // namespace ab

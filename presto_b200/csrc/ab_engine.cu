@@ -67,7 +67,11 @@ struct ab_ctx {
     ab_bankset bs{};
     bool have_banks = false;
     // template banks: entries of the device-wide cache (shared by every
-    // context on the device); tmpl_p points into the current one
+    // context on the device)
+    // templates of one bank with half widths up to hw, perm[t_lo .. t_lo + nt)
+    struct SegClass {
+        int bank, hw, t_lo, nt;
+    };
     // operands of the tensor-core correlation for one bank set: templates
     // sorted by half-width into tiles, packed split-BF16 taps per tile
     struct TcBank {
@@ -83,7 +87,9 @@ struct ab_ctx {
     };
     struct BankEntry {
         ab_bankset bs;
-        DevBuf<float2> tmpl;
+        DevBuf<float2> tmpl;                // segment templates (ab_corr.cu), natural order
+        DevBuf<int> perm;                   // template indices, by class
+        std::vector<SegClass> classes;      // bank-major, widest first
         unsigned long long used = 0;
         TcBank tc;
         int refs = 0;                       // contexts whose current banks these are
@@ -96,13 +102,15 @@ struct ab_ctx {
     DevBuf<float2> blu_a, blu_b;            // Bluestein work and chirp-kernel transform
     DevBuf<float> dd_x, dd_sub, dd_out;     // dedispersion: spectra, subbands, DM trials
     DevBuf<float2> dd_fft;                  // spectrum of one DM trial (ab_search_dedispersed)
-    DevBuf<int> bidx;                       // bank lists of the grouped preparation launches
+    DevBuf<SegGroup> seg_groups;            // correlation segments: groups, columns, normalisations
+    DevBuf<SegCols> seg_cols;
+    DevBuf<double> seg_norms;
+    std::vector<SegGroup> hgroups;
     DevBuf<int> dd_cd, dd_off;              // dedispersion delays
     long long blu_M = 0;                    // the length blu_b was built for
     DevBuf<int4> dered_runs;                 // runs of equal de-reddening blocks
     DevBuf<float> dered_means;
     DevBuf<TcItem> titems;
-    float2 *tmpl_p = nullptr;
     DevBuf<ab_bank> dbanks;
     DevBuf<double2> tw64;
     DevBuf<double2> tw_rzw;                 // exp(-2 pi i m / 2^RZW_NMAX_LOG2), jerk polishing
@@ -114,11 +122,9 @@ struct ab_ctx {
     long long fft_bins = 0;
     bool fft_valid = false;
     DevBuf<float2> xhat;
-    DevBuf<double> norms;                    // [block][bank] of superblock banks
     DevBuf<float> planes;
     DevBuf<float> fullplane;
     DevBuf<double> startr;
-    DevBuf<CorrItem> items;
     DevBuf<float> dbg;
     DevBuf<float> tmpa, tmpb;
     DevBuf<unsigned> errw;                   // device error word
@@ -230,6 +236,7 @@ static SharedBanks g_banks[kMaxDevices];
 static void free_entry(ab_ctx::BankEntry *e)
 {
     e->tmpl.release();
+    e->perm.release();
     e->tc.dtiles.release();
     e->tc.dperm.release();
     e->tc.pack[0].release();
@@ -244,7 +251,7 @@ static bool same_templates(const ab_bankset &a, const ab_bankset &b)
     for (int i = 0; i < a.nbanks; i++) {
         const ab_bank &x = a.b[i], &y = b.b[i];
         if (x.numharm != y.numharm || x.harmnum != y.harmnum || x.zmax != y.zmax ||
-            x.wmax != y.wmax || x.L != y.L)
+            x.wmax != y.wmax)
             return false;
     }
     return true;
@@ -260,6 +267,32 @@ static int ensure_tw64(ab_ctx *ctx)
     launch_twiddle64(ctx->tw64.p, 1 << kTwLog2, -1, ctx->stream);
     CK(cudaGetLastError());
     return AB_OK;
+}
+
+// Templates of every bank sorted by half width (widest first) and cut into
+// classes whose half widths lie within a step of the class's widest: an
+// eighth of the range (a class's segments are at most 4 steps columns shorter
+// than its narrowest template could use), at least 24.
+static void build_classes(const ab_bankset &bs, std::vector<int> &perm, std::vector<ab_ctx::SegClass> &classes)
+{
+    perm.clear();
+    classes.clear();
+    for (int k = 0; k < bs.nbanks; k++) {
+        const ab_bank &b = bs.b[k];
+        std::vector<int> hw(b.ntmpl), order(b.ntmpl);
+        for (int t = 0; t < b.ntmpl; t++) {
+            hw[t] = ab_resp_halfwidth((double) (-b.zmax + t % b.nz * AB_DZ), (double) (-b.wmax + t / b.nz * AB_DW));
+            order[t] = t;
+        }
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hw[x] > hw[y]; });
+        const int step = std::max(24, (b.hw0 - AB_NUMFINTBINS + 7) / 8);
+        for (int i = 0; i < b.ntmpl;) {
+            const int w = hw[order[i]], i0 = i;
+            while (i < b.ntmpl && hw[order[i]] > w - step) i++;
+            classes.push_back(ab_ctx::SegClass{k, w, b.perm_off + i0, i - i0});
+        }
+        perm.insert(perm.end(), order.begin(), order.end());
+    }
 }
 
 // Makes the template banks of obs current: from the device-wide cache when a
@@ -295,11 +328,18 @@ static int ensure_banks(ab_ctx *ctx, const ab_obs *obs)
         hit->tc.ready = false;                  // a reused entry's operands are stale
         hit->tc.pack_ready[0] = hit->tc.pack_ready[1] = false;
         if (!hit->ready) CK(cudaEventCreateWithFlags(&hit->ready, cudaEventDisableTiming));
-        CK(hit->tmpl.ensure((size_t) nb.tmpl_total));
+        CK(hit->tmpl.ensure((size_t) nb.seg_tmpl_total));
+        std::vector<int> perm;
+        build_classes(nb, perm, hit->classes);
+        CK(hit->perm.ensure(perm.size()));
+        CK(cudaMemcpyAsync(hit->perm.p, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice,
+                           ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));       // perm is a host vector
         for (int i = 0; i < nb.nbanks; i++) {
             tick(ctx, 0, true);
-            cudaError_t e = launch_templates(&nb.b[i], hit->tmpl.p + nb.b[i].tmpl_off, nullptr,
-                                             ctx->tw64.p, kTwLog2, nullptr, 0, ctx->stream);
+            cudaError_t e = launch_templates(&nb.b[i], 0, nb.b[i].ntmpl, 0,
+                                             hit->tmpl.p + nb.b[i].seg_tmpl_off,
+                                             ctx->tw64.p, kTwLog2, ctx->stream);
             tick(ctx, 0, false);
             ctx->launches++;
             if (e != cudaSuccess)
@@ -313,7 +353,6 @@ static int ensure_banks(ab_ctx *ctx, const ab_obs *obs)
         hit->refs++;
     }
     hit->used = ++sb.clock;
-    ctx->tmpl_p = hit->tmpl.p;
     ctx->cur_bank = hit;
     ctx->bs = nb;
     ctx->have_banks = true;
@@ -346,75 +385,113 @@ static SearchConsts make_consts(const ab_obs *obs, const ab_bankset &bs)
     return sc;
 }
 
-// Correlation work items of one batch of nblk blocks, grouped by FFT length.
-struct CorrPlan {
-    std::vector<CorrItem> items;
-    int Ls[8];
-    int off[8], cnt[8];
-    int nL = 0;
+// ---- correlation ------------------------------------------------------------
+// The segments of one batch (ab_corr.cu): per class of templates of banks
+// [bank_lo, bank_hi), units over the columns of blocks [0, nmain) and, in the
+// in-memory mode, of the pre-pass blocks [nmain, nmain + npre) behind them;
+// start is their start frequencies.  Group bank indices count from bank_lo.
+struct SegPlan {
+    int nunits = 0, nctas = 0;
+    bool own_data = false;
+    int numdata_max = 0;
 };
 
-// With sc.superblocks, a bank of superblock height m > 1 has one transform
-// unit per m consecutive blocks of the batch (CorrItem.bi is the unit).
-static void build_corr_plan(const ab_bankset &bs, const SearchConsts &sc, int nblk, int bank_lo,
-                            int bank_hi, CorrPlan &p)
+static SegPlan build_seg_plan(ab_ctx *ctx, const ab_obs *obs, const double *start, int nmain, int npre,
+                              int bank_lo, int bank_hi)
 {
-    p.items.clear();
-    p.nL = 0;
-    for (int L = 512; L <= 8192; L <<= 1) {
-        int start = (int) p.items.size();
-        const int G = L >= 4096 ? 1 : 4096 / L, tile = 16 * G;
-        for (int k = bank_lo; k < bank_hi; k++) {
-            const ab_bank &b = bs.b[k];
-            if (b.L != L) continue;
-            const int units = corr_units(b, sc, nblk);
-            for (int t0 = 0; t0 < b.ntmpl; t0 += tile)
-                for (int bi = 0; bi < units; bi++)
-                    p.items.push_back(CorrItem{bi, k, t0, std::min(tile, b.ntmpl - t0)});
-        }
-        int n = (int) p.items.size() - start;
-        if (n > 0) {
-            p.Ls[p.nL] = L;
-            p.off[p.nL] = start;
-            p.cnt[p.nL] = n;
-            p.nL++;
+    SegPlan p;
+    std::vector<SegGroup> &out = ctx->hgroups;
+    out.clear();
+    long long work = 0;
+    for (const ab_ctx::SegClass &c : ctx->cur_bank->classes) {
+        if (c.bank < bank_lo || c.bank >= bank_hi) continue;
+        const ab_bank &b = ctx->bs.b[c.bank];
+        p.own_data |= b.own_data != 0;
+        p.numdata_max = std::max(p.numdata_max, b.fftlen_ref / AB_NUMBETWEEN);
+        for (int pass = 0; pass < 2; pass++) {
+            const int blk0 = pass ? nmain : 0, n = pass ? npre : nmain;
+            if (n == 0) continue;
+            SegGroup g{};
+            g.bank = c.bank - bank_lo;
+            g.hw = c.hw;
+            g.V = 2 * AB_SEG_BINS - 4 * c.hw;
+            g.t_lo = c.t_lo;
+            g.nt = c.nt;
+            g.blk0 = blk0;
+            g.nblk = n;
+            g.unit0 = p.nunits;
+            if (b.own_data) {
+                g.nsub = (b.numrs_max + g.V - 1) / g.V;
+                g.nunits = g.nsub * n;
+            } else {
+                const double r0 = start[blk0], r1 = start[blk0 + n - 1];
+                const ab_hgeom a = ab_harm_geom(r0, r0 + obs->rstep - AB_DR, b.numharm, b.harmnum, obs->zlo,
+                                                obs->wlo, obs->corr_uselen);
+                const ab_hgeom z = ab_harm_geom(r1, r1 + obs->rstep - AB_DR, b.numharm, b.harmnum, obs->zlo,
+                                                obs->wlo, obs->corr_uselen);
+                const long long w = AB_RDR * (z.rlo - a.rlo) + z.numrs;
+                g.nunits = (int) ((w + g.V - 1) / g.V);
+            }
+            p.nunits += g.nunits;
+            work += (long long) g.nunits * g.nt;
+            out.push_back(g);
         }
     }
-}
-
-static int run_corr(ab_ctx *ctx, const SearchConsts &sc, const BlockBatch &bb, const CorrPlan &p,
-                    const CorrItem *ditems, float *planes, long long ppb, float *fullplane)
-{
-    for (int i = 0; i < p.nL; i++) {
-        tick(ctx, 2, true);
-        cudaError_t e = launch_corr(p.Ls[i], ctx->dbanks.p, sc, bb, ditems + p.off[i], p.cnt[i],
-                                    ctx->xhat.p, ctx->bs.xhat_per_block, ctx->tmpl_p, planes,
-                                    ppb, fullplane, ctx->stream);
-        tick(ctx, 2, false);
-        ctx->launches++;
-        if (e != cudaSuccess)
-            return fail(ctx, AB_ERR_CUDA, "correlation launch failed: %s", cudaGetErrorString(e));
+    // templates per CTA: 64 (the CTA's set-up is a template's work) while that
+    // leaves six CTAs per SM, fewer for a small batch: one block's four planes at
+    // zmax = 50 take 61 us in tiles of 8, 140 us in CTAs of 16 templates
+    const long long per = work / (148 * 6) / 8 * 8;
+    const int tile = (int) std::max<long long>(8, std::min<long long>(64, per));
+    for (SegGroup &g : out) {
+        g.tile = tile;
+        g.cta0 = p.nctas;
+        p.nctas += g.nunits * ((g.nt + tile - 1) / tile);
     }
-    return AB_OK;
+    return p;
 }
 
-static int run_prep(ab_ctx *ctx, const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                    int bank_lo, int bank_hi)
+// Data spectra and correlation of one batch of blocks [0, bb.nblk) (bb.npre0 of
+// them main-loop blocks, the rest pre-pass blocks): planes of the standard
+// mode, or the in-memory plane.
+static int run_corr(ab_ctx *ctx, const ab_obs *obs, const SearchConsts &sc, const BlockBatch &bb,
+                    const double *start, const float2 *fft, int bank_lo, int bank_hi, float *planes,
+                    long long ppb)
 {
+    const ab_bankset &bs = ctx->bs;
+    const int nbanks = bank_hi - bank_lo;
+    const SegPlan p = build_seg_plan(ctx, obs, start, bb.npre0, bb.nblk - bb.npre0, bank_lo, bank_hi);
+    CK(ctx->seg_groups.ensure(ctx->hgroups.size()));
+    CK(ctx->seg_cols.ensure((size_t) nbanks * bb.nblk));
+    CK(ctx->seg_norms.ensure((size_t) nbanks * bb.nblk));
+    CK(ctx->xhat.ensure((size_t) p.nunits * AB_SEG_BINS));
+    if (p.own_data) CK(ctx->dtime.ensure((size_t) bb.nblk * bs.dtime_per_block));
+    CK(cudaMemcpyAsync(ctx->seg_groups.p, ctx->hgroups.data(), sizeof(SegGroup) * ctx->hgroups.size(),
+                       cudaMemcpyHostToDevice, ctx->stream));
+    const ab_bank *db = ctx->dbanks.p + bank_lo;
+    const int ng = (int) ctx->hgroups.size();
     tick(ctx, 1, true);
-    CK(ctx->bidx.ensure((size_t) std::max(1, bank_hi - bank_lo)));
-    cudaError_t e = launch_prep(ctx->dbanks.p + bank_lo, ctx->bs.b + bank_lo, bank_hi - bank_lo,
-                                sc, bb, fft, ctx->xhat.p, ctx->bs.xhat_per_block, ctx->bidx.p,
-                                ctx->stream);
-    tick(ctx, 1, false);
-    {
-        // one launch per distinct transform length
-        unsigned seen = 0;
-        for (int k = bank_lo; k < bank_hi; k++) seen |= 1u << (31 - __builtin_clz((unsigned) ctx->bs.b[k].L));
-        ctx->launches += __builtin_popcount(seen);
+    cudaError_t e = launch_seg_cols(db, nbanks, sc, bb, fft, p.numdata_max, ctx->seg_cols.p, ctx->seg_norms.p,
+                                    ctx->stream);
+    ctx->launches++;
+    for (int k = bank_lo; k < bank_hi && e == cudaSuccess && p.own_data; k++) {
+        if (!bs.b[k].own_data) continue;
+        e = launch_prep_time(ctx->dbanks.p + k, bs.b + k, 1, sc, bb, fft, ctx->dtime.p, bs.dtime_per_block,
+                             ctx->seg_norms.p + (size_t) (k - bank_lo) * bb.nblk, ctx->stream);
+        ctx->launches++;
     }
+    if (e == cudaSuccess)
+        e = launch_seg_fwd(db, sc, bb, ctx->seg_groups.p, ng, p.nunits, ctx->seg_cols.p, ctx->seg_norms.p, fft,
+                           ctx->dtime.p, bs.dtime_per_block, ctx->xhat.p, ctx->stream);
+    tick(ctx, 1, false);
     if (e != cudaSuccess)
-        return fail(ctx, AB_ERR_CUDA, "prep launch failed: %s", cudaGetErrorString(e));
+        return fail(ctx, AB_ERR_CUDA, "data preparation failed: %s", cudaGetErrorString(e));
+    tick(ctx, 2, true);
+    e = launch_corr_seg(db, sc, bb, ctx->seg_groups.p, ng, p.nctas, ctx->seg_cols.p, ctx->seg_norms.p,
+                        ctx->xhat.p, ctx->cur_bank->tmpl.p, ctx->cur_bank->perm.p, planes, ppb, ctx->stream);
+    tick(ctx, 2, false);
+    ctx->launches += 2;
+    if (e != cudaSuccess)
+        return fail(ctx, AB_ERR_CUDA, "correlation launch failed: %s", cudaGetErrorString(e));
     return AB_OK;
 }
 
@@ -554,7 +631,7 @@ static int run_tc(ab_ctx *ctx, const SearchConsts &sc, const BlockBatch &bb, con
     const ab_ctx::TcBank &tb = ctx->cur_bank->tc;
     tick(ctx, 1, true);
     cudaError_t e = launch_prep_time(ctx->dbanks.p + bank_lo, ctx->bs.b + bank_lo, bank_hi - bank_lo,
-                                     sc, bb, fft, ctx->dtime.p, ctx->bs.dtime_per_block, ctx->stream);
+                                     sc, bb, fft, ctx->dtime.p, ctx->bs.dtime_per_block, nullptr, ctx->stream);
     tick(ctx, 1, false);
     ctx->launches++;
     if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "data preparation failed: %s", cudaGetErrorString(e));
@@ -800,55 +877,34 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
             if (rc) return rc;
             CK(ctx->dtime.ensure((size_t) std::max<long long>(std::max(npre, nmain), 1) *
                                  bs.dtime_per_block));
-        } else {
-            CK(ctx->xhat.ensure((size_t) std::max<long long>(nall, 1) * bs.xhat_per_block));
-        }
-        // both passes' work items are built first and uploaded once, each pass
-        // reading its own part, so the passes follow each other on the stream
-        CorrPlan plan[2];
-        std::vector<TcItem> tplan[2];
-        size_t ioff[2] = {0, 0}, itotal = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            const long long nb = pass == 0 ? npre : nmain;
-            ioff[pass] = itotal;
-            if (nb == 0) continue;
-            if (tcp) {
+            // both passes' work items are built first and uploaded once, each pass
+            // reading its own part, so the passes follow each other on the stream
+            std::vector<TcItem> tplan[2];
+            size_t ioff[2] = {0, 0}, itotal = 0;
+            for (int pass = 0; pass < 2; pass++) {
+                const long long nb = pass == 0 ? npre : nmain;
+                ioff[pass] = itotal;
+                if (nb == 0) continue;
                 build_tc_plan(ctx->cur_bank->tc, bs, (int) nb, 0, 1, tplan[pass]);
                 itotal += tplan[pass].size();
-            } else {
-                build_corr_plan(bs, sc, (int) nb, 0, 1, plan[pass]);
-                itotal += plan[pass].items.size();
             }
-        }
-        if (tcp) {
             CK(ctx->titems.ensure(std::max<size_t>(itotal, 1)));
             for (int pass = 0; pass < 2; pass++)
                 if (!tplan[pass].empty())
                     CK(cudaMemcpyAsync(ctx->titems.p + ioff[pass], tplan[pass].data(),
                                        sizeof(TcItem) * tplan[pass].size(), cudaMemcpyHostToDevice,
                                        ctx->stream));
-        } else {
-            CK(ctx->items.ensure(std::max<size_t>(itotal, 1)));
-            for (int pass = 0; pass < 2; pass++)
-                if (!plan[pass].items.empty())
-                    CK(cudaMemcpyAsync(ctx->items.p + ioff[pass], plan[pass].items.data(),
-                                       sizeof(CorrItem) * plan[pass].items.size(),
-                                       cudaMemcpyHostToDevice, ctx->stream));
-        }
-        for (int pass = 0; pass < 2; pass++) {
-            long long nb = pass == 0 ? npre : nmain;
-            if (nb == 0) continue;
-            BlockBatch bb{ctx->startr.p + (pass == 0 ? nmain : 0), 0, (int) nb, pass == 0};
-            if (tcp) {
+            for (int pass = 0; pass < 2; pass++) {
+                const long long nb = pass == 0 ? npre : nmain;
+                if (nb == 0) continue;
+                BlockBatch bb{ctx->startr.p + (pass == 0 ? nmain : 0), 0, (int) nb, pass == 0 ? 0 : (int) nb};
                 rc = run_tc(ctx, sc, bb, dfft, 0, 1, ctx->titems.p + ioff[pass], (int) tplan[pass].size(),
                             nullptr, 0, ctx->fullplane.p);
                 if (rc) return rc;
-                continue;
             }
-            rc = run_prep(ctx, sc, bb, dfft, 0, 1);
-            if (rc) return rc;
-            rc = run_corr(ctx, sc, bb, plan[pass], ctx->items.p + ioff[pass], nullptr, 0,
-                          ctx->fullplane.p);
+        } else if (nall > 0) {
+            BlockBatch bb{ctx->startr.p, 0, (int) nall, (int) nmain};
+            rc = run_corr(ctx, obs, sc, bb, ctx->hstart.data(), dfft, 0, 1, ctx->fullplane.p, 0);
             if (rc) return rc;
         }
         // the sums run in chunks of blocks through the ring of hit sets, so the
@@ -861,7 +917,7 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
             const int set = k % ab_ctx::kHitSets;
             HitSet h = hitset(ctx, set);
             CK(cudaMemsetAsync(h.count, 0, sizeof(unsigned), ctx->stream));
-            BlockBatch bb{ctx->startr.p + c0, c0, nb, 0};
+            BlockBatch bb{ctx->startr.p + c0, c0, nb, nb};
             HitBuf hb{h.keys, h.pows, h.count, ctx->hit_cap};
             const bool dump = dbg_block >= c0 && dbg_block < c0 + nb;
             tick(ctx, 3, true);
@@ -895,7 +951,7 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
         if (rc) return rc;
     }
     const size_t per_block = (size_t) bs.plane_per_block * sizeof(float) +
-                             (size_t) (tcp ? bs.dtime_per_block : bs.xhat_per_block) * sizeof(float2);
+                             (size_t) bs.dtime_per_block * sizeof(float2);
     long long B = (long long) (ctx->scratch_budget / std::max<size_t>(per_block, 1));
     if (B < 1) B = 1;
     if (B > 512) B = 512;
@@ -903,7 +959,6 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
     if (count >= 8 && B > (count + 7) / 8) B = (count + 7) / 8;
     if (B > count) B = std::max<long long>(count, 1);
     CK(ctx->planes.ensure((size_t) B * bs.plane_per_block));
-    CorrPlan full, tail;
     std::vector<TcItem> tfull, ttail;
     long long rem = count % B;
     if (tcp) {
@@ -916,19 +971,6 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
         if (rem)
             CK(cudaMemcpyAsync(ctx->titems.p + tfull.size(), ttail.data(), sizeof(TcItem) * ttail.size(),
                                cudaMemcpyHostToDevice, ctx->stream));
-    } else {
-        CK(ctx->xhat.ensure((size_t) B * bs.xhat_per_block));
-        sc.superblocks = 1;
-        CK(ctx->norms.ensure((size_t) B * bs.nbanks));
-        sc.norms = ctx->norms.p;
-        build_corr_plan(bs, sc, (int) B, 0, bs.nbanks, full);
-        if (rem) build_corr_plan(bs, sc, (int) rem, 0, bs.nbanks, tail);
-        CK(ctx->items.ensure(full.items.size() + tail.items.size()));
-        CK(cudaMemcpyAsync(ctx->items.p, full.items.data(), sizeof(CorrItem) * full.items.size(),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        if (rem)
-            CK(cudaMemcpyAsync(ctx->items.p + full.items.size(), tail.items.data(),
-                               sizeof(CorrItem) * tail.items.size(), cudaMemcpyHostToDevice, ctx->stream));
     }
     int k = 0;
     for (long long b0 = first; b0 < first + count; b0 += B, k++) {
@@ -936,7 +978,7 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
         const int set = k % ab_ctx::kHitSets;
         HitSet h = hitset(ctx, set);
         CK(cudaMemsetAsync(h.count, 0, sizeof(unsigned), ctx->stream));
-        BlockBatch bb{ctx->startr.p + b0, b0, nb, 0};
+        BlockBatch bb{ctx->startr.p + b0, b0, nb, nb};
         if (tcp) {
             const TcItem *di = ctx->titems.p + ((nb == B) ? 0 : tfull.size());
             const int ni = (int) ((nb == B) ? tfull.size() : ttail.size());
@@ -944,19 +986,8 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
                         nullptr);
             if (rc) return rc;
         } else {
-            tick(ctx, 1, true);
-            CK(ctx->bidx.ensure((size_t) std::max(1, bs.nbanks)));
-            cudaError_t en = launch_norms(ctx->dbanks.p, bs.b, bs.nbanks, sc, bb, dfft, ctx->bidx.p,
-                                          ctx->stream);
-            tick(ctx, 1, false);
-            ctx->launches++;
-            if (en != cudaSuccess)
-                return fail(ctx, AB_ERR_CUDA, "normalisation launch failed: %s", cudaGetErrorString(en));
-            rc = run_prep(ctx, sc, bb, dfft, 0, bs.nbanks);
-            if (rc) return rc;
-            const CorrPlan &p = (nb == B) ? full : tail;
-            const CorrItem *di = ctx->items.p + ((nb == B) ? 0 : full.items.size());
-            rc = run_corr(ctx, sc, bb, p, di, ctx->planes.p, bs.plane_per_block, nullptr);
+            rc = run_corr(ctx, obs, sc, bb, ctx->hstart.data() + b0, dfft, 0, bs.nbanks, ctx->planes.p,
+                          bs.plane_per_block);
             if (rc) return rc;
         }
         int dbi = (dbg_block >= b0 && dbg_block < b0 + nb) ? (int) (dbg_block - b0) : -1;
@@ -1135,7 +1166,6 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->planes.release();
     ctx->fullplane.release();
     ctx->startr.release();
-    ctx->items.release();
     ctx->dbg.release();
     ctx->tmpa.release();
     ctx->tmpb.release();
@@ -1150,13 +1180,14 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->dd_sub.release();
     ctx->dd_out.release();
     ctx->dd_fft.release();
-    ctx->bidx.release();
+    ctx->seg_groups.release();
+    ctx->seg_cols.release();
+    ctx->seg_norms.release();
     ctx->dd_cd.release();
     ctx->dd_off.release();
     ctx->dered_runs.release();
     ctx->dered_means.release();
     ctx->titems.release();
-    ctx->norms.release();
     ctx->keys.release();
     ctx->pows.release();
     ctx->count.release();
@@ -1249,12 +1280,12 @@ int ab_autotune(ab_ctx *ctx, double *costs_out, int n)
                             ctx->stream);
             cudaMemcpyAsync(items.p, it.data(), sizeof(CorrItem) * it.size(), cudaMemcpyHostToDevice,
                             ctx->stream);
-            BlockBatch bb{startr.p, 0, kBlocks, 0};
+            BlockBatch bb{startr.p, 0, kBlocks, kBlocks};
             float best = 1e30f;
             for (int rep = 0; rep < 4 && e == cudaSuccess; rep++) {
                 cudaEventRecord(e0, ctx->stream);
                 e = launch_corr(L, dbank.p, sc, bb, items.p, (int) it.size(), xhat.p, L / 2, tmpl.p,
-                                planes.p, (long long) kTmpl * b.numrs_max, nullptr, ctx->stream);
+                                planes.p, (long long) kTmpl * b.numrs_max, ctx->stream);
                 cudaEventRecord(e1, ctx->stream);
                 if (e == cudaSuccess) e = cudaEventSynchronize(e1);
                 float ms = 0.f;
@@ -1869,7 +1900,7 @@ int ab_subharm_fderivs_vol(ab_ctx *ctx, const ab_obs *obs, int numharm, int harm
     CK(ctx->startr.ensure(1));
     CK(cudaMemcpyAsync(ctx->startr.p, &fullrlo, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(ctx->planes.ensure((size_t) ctx->bs.plane_per_block));
-    BlockBatch bb{ctx->startr.p, 0, 1, 0};
+    BlockBatch bb{ctx->startr.p, 0, 1, 1};
     if (ctx->corr_path != AB_CORR_FFT) {
         rc = ensure_tc(ctx);
         if (rc) return rc;
@@ -1883,15 +1914,7 @@ int ab_subharm_fderivs_vol(ab_ctx *ctx, const ab_obs *obs, int numharm, int harm
                     ctx->bs.plane_per_block, nullptr);
         if (rc) return rc;
     } else {
-        CK(ctx->xhat.ensure((size_t) ctx->bs.xhat_per_block));
-        rc = run_prep(ctx, sc, bb, ctx->fft.p, k, k + 1);
-        if (rc) return rc;
-        CorrPlan plan;
-        build_corr_plan(ctx->bs, sc, 1, k, k + 1, plan);
-        CK(ctx->items.ensure(plan.items.size()));
-        CK(cudaMemcpyAsync(ctx->items.p, plan.items.data(), sizeof(CorrItem) * plan.items.size(),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        rc = run_corr(ctx, sc, bb, plan, ctx->items.p, ctx->planes.p, ctx->bs.plane_per_block, nullptr);
+        rc = run_corr(ctx, obs, sc, bb, &fullrlo, ctx->fft.p, k, k + 1, ctx->planes.p, ctx->bs.plane_per_block);
         if (rc) return rc;
     }
     CK(cudaMemcpy2DAsync(out->powers, sizeof(float) * g.numrs, ctx->planes.p + b.plane_off,
@@ -2141,8 +2164,13 @@ int ab_bank_kernel(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int
     if (wi < 0 || wi >= b.nw || zi < 0 || zi >= b.nz) return fail(ctx, AB_ERR_ARG, "template index");
     if (!out) return AB_OK;
     if (maxlen < b.L) return fail(ctx, AB_ERR_OVERFLOW, "need %d", b.L);
-    CK(cudaMemcpyAsync(out, ctx->tmpl_p + b.tmpl_off + (long long) (wi * b.nz + zi) * b.L,
-                       sizeof(float2) * b.L, cudaMemcpyDeviceToHost, ctx->stream));
+    if ((rc = ensure_tw64(ctx))) return rc;
+    CK(ctx->resp.ensure((size_t) b.L));
+    const int t = wi * b.nz + zi;
+    cudaError_t e = launch_templates(&b, t, t + 1, b.L, ctx->resp.p, ctx->tw64.p, kTwLog2, ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "template generation failed: %s", cudaGetErrorString(e));
+    ctx->launches++;
+    CK(cudaMemcpyAsync(out, ctx->resp.p, sizeof(float2) * b.L, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     harvest(ctx);
     return AB_OK;

@@ -389,7 +389,8 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
                 pairs[n][0] = 1 << s; pairs[n][1] = h; n++;
             }
     long long nblocks = ab_num_blocks(obs), npre = ab_num_preblocks(obs);
-    long long tmpl = 0, plane = 0, xhat = 0, dtime = 0;
+    long long tmpl = 0, plane = 0, xhat = 0, dtime = 0, seg = 0;
+    int perm = 0;
     for (int i = 0; i < n; i++) {
         ab_bank *b = &bs->b[i];
         b->numharm = pairs[i][0];
@@ -480,6 +481,11 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
         free(rlo);
         free(nrs);
         b->sbm = sbm;
+        b->own_data = obs->norm_type != 0 || need > b->fftlen_ref;
+        b->seg_tmpl_off = seg;
+        b->perm_off = perm;
+        seg += (long long) b->ntmpl * 2048;
+        perm += b->ntmpl;
         b->L = L;
         b->log2L = twon_to_index(L);
         b->tmpl_off = tmpl;
@@ -493,6 +499,8 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
     }
     bs->nbanks = n;
     bs->tmpl_total = tmpl;
+    bs->seg_tmpl_total = seg;
+    bs->perm_total = perm;
     bs->plane_per_block = plane;
     bs->xhat_per_block = xhat;
     bs->dtime_per_block = dtime;

@@ -22,16 +22,21 @@ typedef struct {
     int zmax, wmax;               /* calc_required_z/w of the search maxima */
     int nz, nw, ntmpl;            /* numkern_zdim, numkern_wdim, numkern */
     int fftlen_ref;               /* the reference's FFT length (calc_fftlen) */
-    int L, log2L;                 /* device FFT length (power of two) */
+    int L, log2L;                 /* template length of ab_bank_kernel and the
+                                     allocation-free entry point (power of two) */
     int hw0;                      /* kern[0][0].kern_half_width (binoffset) */
     int numrs_max;                /* largest numrs over all blocks (row stride) */
-    long long tmpl_off;           /* complex offset of the bank's templates */
+    long long tmpl_off;           /* complex offset of the bank's templates of L points */
+    long long seg_tmpl_off;       /* offset of its segment templates (ab_corr.cu) */
+    int perm_off;                 /* offset of its templates in the order by half width */
+    int own_data;                 /* correlated by each block's own window (the reference's
+                                     transform wraps into valid cells, or -locpow) */
     long long plane_off;          /* float offset inside one block's plane scratch */
     long long xhat_off;           /* complex offset inside one block's spectrum scratch */
     long long dtime_off;          /* complex offset of the block's normalised data
                                      (tensor-core correlation) */
-    int sbm;                      /* blocks per device transform in the standard
-                                     search (superblock height, >= 1) */
+    int sbm;                      /* blocks that the cost table would have share a
+                                     transform of L points (>= 1; reported only) */
     int index;                    /* position in the bank set */
 } ab_bank;
 
@@ -42,6 +47,8 @@ typedef struct {
     int nbanks;
     ab_bank b[AB_MAX_BANKS];
     long long tmpl_total;         /* complex elements over all banks */
+    long long seg_tmpl_total;     /* complex elements of the segment templates */
+    int perm_total;               /* templates over all banks */
     long long plane_per_block;    /* floats of plane scratch per block */
     long long xhat_per_block;     /* complex elements of spectrum scratch per block */
     long long dtime_per_block;    /* complex elements of normalised data per block */
@@ -52,7 +59,7 @@ typedef struct {
 int ab_bankset_init(const ab_obs *obs, ab_bankset *bs);
 /* The same with measured per-template transform costs by log2 L
  * (AB_COST_SLOTS entries, <= 0 for unknown), which choose each bank's
- * transform length and superblock height. */
+ * template length L and sbm. */
 int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_bankset *bs);
 
 /* Number of blocks of the main loop (src/accelsearch.c:187-224) and of the

@@ -3,12 +3,13 @@
 //   (a) k_templates   FP64 response templates (gen_w/z/r_response,
 //                     src/responses.c:159-418), placed (place_complex_kernel,
 //                     src/corr_prep.c:92-114) and FFT'd in FP64, stored FP32.
-//   (b) k_prep        per (block, harmonic): amplitudes with zero padding
+//   (b) k_prep        one block and harmonic: amplitudes with zero padding
 //                     (src/accel_utils.c:993-1022), block-median
 //                     normalisation (:1079-1099), spread (src/corr_prep.c:62-74)
-//                     and forward FFT (:1117-1121).
+//                     and forward FFT (:1117-1121); k_prep_time the data alone.
 //       k_corr<L>     template correlation: data * conj(kernel), inverse FFT,
-//                     |.|^2 / L^2 over the valid cells (:1140-1193).
+//                     |.|^2 / L^2 over the valid cells (:1140-1193).  (The
+//                     searches' correlation is in ab_corr.cu.)
 //   (c)+(d) k_harmsum_*  harmonic sums (add_ffdotpows :1261-1282,
 //                     inmem_add_ffdotpows :1312-1361) fused with the threshold
 //                     of search_ffdotpows (:1412-1452), hits compacted with
@@ -21,8 +22,6 @@
 #include "ab_index.h"
 #include "ab_kernels.h"
 
-#include <algorithm>
-#include <vector>
 #include "ab_norm.cuh"
 #include "ab_resp.cuh"
 #include "ab_select.cuh"
@@ -73,10 +72,34 @@ __device__ void fft64_tab(double2 *x, int n, const double2 *tw, int nmax)
     }
 }
 
+// ---------------------------------------------------------------------------
+// segment templates of the searches' correlation (ab_corr.cu)
+// ---------------------------------------------------------------------------
+// The 2 H-column inverse transform of X K* (X repeated, the data being on
+// every second column) as two of H = 1024 points: the even columns take X with
+// the transform of the even taps, (K[i] + K[i + H]) / 2, the odd ones with
+// (K[i] - K[i + H]) / 2 exp(-2 pi i i / 2H).  `placed` holds K in FP64.
+// Points as ab_corr.cu's lanes read them.
+__device__ void store_seg_template(const double2 *placed, float2 *out)
+{
+    constexpr int H = AB_SEG_BINS;
+    for (int i = threadIdx.x; i < H; i += blockDim.x) {
+        const double2 a = placed[i], b = placed[i + H];
+        const double dr = 0.5 * (a.x - b.x), di = 0.5 * (a.y - b.y);
+        double s, c;
+        sincospi(-(double) i / (double) H, &s, &c);
+        const int o = (i & ~63) + 2 * (i & 31) + ((i >> 5) & 1);
+        out[o] = make_float2((float) (0.5 * (a.x + b.x)), (float) (0.5 * (a.y + b.y)));
+        out[H + o] = make_float2((float) (dr * c - di * s), (float) (dr * s + di * c));
+    }
+}
+
 // One CTA per template.  mode 0: bank template (placed, FFT'd, FP32 into
 // out + t*L).  mode 1: raw response of numkern points into out.  mode 2:
 // raw response of bank template t (numkern = 4 halfwidth points) into
-// out + t*L, L being the row stride (taps of the tensor-core path).
+// out + t*L, L being the row stride (taps of the tensor-core path).  mode 3:
+// bank template placed on L = 2048 columns, stored for ab_corr.cu into
+// out + 2 t AB_SEG_BINS.
 // Dynamic shared memory: (L + nfft_max) double2.
 struct TmplArgs {
     int mode, zmax, wmax, nz, L, t_base;
@@ -109,14 +132,15 @@ __global__ void __launch_bounds__(256) k_templates(TmplArgs a)
     if (a.mode != 1 && numkern > a.L) return;       // host validates; keeps stores in range
     float2 *raw = (a.mode == 2) ? a.out + (size_t) t * a.L : a.out;
     const int L = a.L, half = numkern / 2;
-    double2 *placed = dsm;              // [L]   (mode 0)
-    double2 *chirp = dsm + (a.mode == 0 ? L : 0);   // [nfft]
-    if (a.mode == 0)
+    const bool place = a.mode == 0 || a.mode == 3;
+    double2 *placed = dsm;              // [L]   (modes 0 and 3)
+    double2 *chirp = dsm + (place ? L : 0);         // [nfft]
+    if (place)
         for (int i = threadIdx.x; i < L; i += blockDim.x) placed[i] = make_double2(0.0, 0.0);
     if (fabs(w) < 1E-4) {
         for (int c = threadIdx.x; c < numkern; c += blockDim.x) {
             double2 v = z_resp_point(roffset, numbetween, z, numkern, c);
-            if (a.mode == 0) placed[c >= half ? c - half : L - half + c] = v;
+            if (place) placed[c >= half ? c - half : L - half + c] = v;
             else raw[c] = make_float2((float) v.x, (float) v.y);
         }
         __syncthreads();
@@ -144,13 +168,17 @@ __global__ void __launch_bounds__(256) k_templates(TmplArgs a)
         int first = fbar * numbetween - numkern / 2;
         for (int c = threadIdx.x; c < numkern; c += blockDim.x) {
             double2 v = chirp[first + c];
-            if (a.mode == 0) placed[c >= half ? c - half : L - half + c] = v;
+            if (place) placed[c >= half ? c - half : L - half + c] = v;
             else raw[c] = make_float2((float) v.x, (float) v.y);
         }
         __syncthreads();
     }
-    if (a.mode == 0) {
+    if (place) {
         fft64_tab(placed, L, a.tw, a.nmax);
+        if (a.mode == 3) {
+            store_seg_template(placed, a.out + (size_t) t * 2 * AB_SEG_BINS);
+            return;
+        }
         float2 *o = a.out + (size_t) t * L;
         for (int i = threadIdx.x; i < L; i += blockDim.x)
             o[i] = make_float2((float) placed[i].x, (float) placed[i].y);
@@ -165,41 +193,40 @@ static int chirp_len(double z, double w, int numkern, int numbetween)
     return n * numbetween;
 }
 
-cudaError_t launch_templates(const ab_bank *b, float2 *bank_out, const double2 *tw_place,
-                             const double2 *tw_all, int max_log2, double2 *scratch,
-                             size_t scratch_elems, cudaStream_t st)
+// Templates [t_lo, t_hi) of a bank.  L > 0: each as the transform of its taps
+// placed on L columns, out + (t - t_lo) L; L = 0: as ab_corr.cu reads them, out
+// + 2 AB_SEG_BINS t.
+cudaError_t launch_templates(const ab_bank *b, int t_lo, int t_hi, int L, float2 *out, const double2 *tw_all,
+                             int max_log2, cudaStream_t st)
 {
-    (void) tw_place;
-    (void) scratch;
-    (void) scratch_elems;
+    const bool seg = L == 0;
+    if (seg) L = 2 * AB_SEG_BINS;
     int nfft_max = 0;
-    for (int wi = 0; wi < b->nw; wi++) {
-        double w = -b->wmax + wi * AB_DW;
-        for (int zi = 0; zi < b->nz; zi++) {
-            double z = -b->zmax + zi * AB_DZ;
-            int nk = 2 * AB_NUMBETWEEN * ab_resp_halfwidth(z, w);
-            int n = chirp_len(z, w, nk, AB_NUMBETWEEN);
-            if (n > nfft_max) nfft_max = n;
-        }
+    for (int t = t_lo; t < t_hi; t++) {
+        const double w = -b->wmax + t / b->nz * AB_DW, z = -b->zmax + t % b->nz * AB_DZ;
+        int nk = 2 * AB_NUMBETWEEN * ab_resp_halfwidth(z, w);
+        int n = chirp_len(z, w, nk, AB_NUMBETWEEN);
+        if (nk > L) return cudaErrorInvalidValue;
+        if (n > nfft_max) nfft_max = n;
     }
     int nmax = 1 << max_log2;
-    if (nfft_max > nmax || b->L > nmax) return cudaErrorInvalidValue;
-    size_t smem = (size_t) (b->L + nfft_max) * sizeof(double2);
+    if (nfft_max > nmax || L > nmax) return cudaErrorInvalidValue;
+    size_t smem = (size_t) (L + nfft_max) * sizeof(double2);
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
     cudaFuncSetAttribute(k_templates, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     TmplArgs a{};
-    a.mode = 0;
+    a.mode = seg ? 3 : 0;
     a.zmax = b->zmax;
     a.wmax = b->wmax;
     a.nz = b->nz;
-    a.L = b->L;
+    a.L = L;
     a.tw = tw_all;
     a.nmax = nmax;
-    a.out = bank_out;
+    a.out = seg ? out : out - (size_t) t_lo * L;
     const int chunk = 65535;
-    for (int t0 = 0; t0 < b->ntmpl; t0 += chunk) {
+    for (int t0 = t_lo; t0 < t_hi; t0 += chunk) {
         a.t_base = t0;
-        int n = b->ntmpl - t0 < chunk ? b->ntmpl - t0 : chunk;
+        int n = t_hi - t0 < chunk ? t_hi - t0 : chunk;
         k_templates<<<n, 256, smem, st>>>(a);
     }
     return cudaGetLastError();
@@ -277,77 +304,23 @@ __device__ __forceinline__ void block_geom(const SearchConsts &sc, const ab_bank
                       sc.obs_wlo, sc.corr_uselen);
 }
 
-// Block normalisation 1/sqrt(median(|X|^2)/ln 2) of the numdata bins from
-// lobin (zero outside the spectrum), or 1/sqrt(nph) when nph is given
-// (src/accel_utils.c:1079-1099).  The median is taken over float POWER()
-// values without FMA, sorted exactly; even counts average the two central
-// values (GSL semantics).  pw: shared scratch of numdata floats.
-// Called by every thread of the CTA.
-// The block's normalisation (src/accel_utils.c:1079-1113): 1/sqrt(nph) with
-// -photon, else 1/sqrt(median/ln 2) of the window's powers.  With -locpow
-// (sc.norm_type 1) it leaves the window's powers in pw for locpow_invsqrt
-// and returns 0 (the factor is per bin).
-__device__ double block_norm(const SearchConsts &sc, long long lobin, int numdata, const float2 *fft,
-                             float *pw, double *s_norm)
-{
-    if (sc.nph > 0.0f) {
-        if (threadIdx.x == 0) *s_norm = 1.0 / sqrt((double) sc.nph);
-    } else if (sc.norm_type == 1) {
-        for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
-            long long bin = lobin + i - sc.obs_lobin;
-            float2 v = (bin >= 0 && bin < sc.numbins) ? fft[bin] : make_float2(0.f, 0.f);
-            pw[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
-        }
-        if (threadIdx.x == 0) *s_norm = 0.0;
-    } else {
-        // block median of |X|^2 in float (POWER(), no FMA), src/accel_utils.c:1087-1099
-        for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
-            long long bin = lobin + i - sc.obs_lobin;
-            float2 v = (bin >= 0 && bin < sc.numbins) ? fft[bin] : make_float2(0.f, 0.f);
-            pw[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
-        }
-        __syncthreads();
-        // the two central order statistics (equal for odd counts), as a sort gives them
-        __shared__ unsigned s_hist[256], s_res[2];
-        const float lo = select_rank(pw, numdata, (numdata - 1) / 2, s_hist, s_res);
-        const float hi = (numdata & 1) ? lo : select_rank(pw, numdata, numdata / 2, s_hist, s_res);
-        if (threadIdx.x == 0) {
-            double m = (numdata & 1) ? (double) lo : 0.5 * ((double) lo + (double) hi);
-            float med = (float) m;
-            *s_norm = 1.0 / sqrt((double) med / 0.69314718055994530942);
-        }
-    }
-    __syncthreads();
-    return *s_norm;
-}
-
-// blockIdx.x: bank (bidx[blockIdx.x] when a list is given), blockIdx.y:
-// transform unit; rows past a bank's units (a launch covers banks of one
-// transform length with different superblock heights) return at once
+// The data spectrum of one block and bank for k_corr.
 template <int LH>
-__global__ void __launch_bounds__(256) k_prep(const ab_bank *banks, const int *bidx, SearchConsts sc,
-                                              BlockBatch bb, const float2 *fft, float2 *xhat,
-                                              long long xhat_per_block)
+__global__ void __launch_bounds__(256) k_prep(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
+                                              const float2 *fft, float2 *xhat)
 {
     using SH = FftShape<LH>;
     extern __shared__ float2 fsm[];
     __shared__ double s_norm;
-    const int bank = bidx ? bidx[blockIdx.x] : blockIdx.x, bi = blockIdx.y;
-    const ab_bank b = banks[bank];
-    // superblock: the window of its first block, the normalisation of that
-    // block (computed by k_norms), the data unrepeated over L/2 bins
-    const bool sb = sc.superblocks && b.sbm > 1;
-    const int blk = sb ? bi * b.sbm : bi;
-    if (blk >= bb.nblk) return;
+    const ab_bank b = banks[0];
     ab_hgeom g;
-    block_geom(sc, b, bb.startr[blk], &g);
+    block_geom(sc, b, bb.startr[0], &g);
     const long long lobin = g.rlo - b.hw0;
-    const int numdata = sb ? LH : b.fftlen_ref / AB_NUMBETWEEN;
-    const double norm = sb ? sc.norms[(long long) blk * sc.nbanks + b.index]
-                           : block_norm(sc, lobin, numdata, fft, reinterpret_cast<float *>(fsm), &s_norm);
+    const int numdata = b.fftlen_ref / AB_NUMBETWEEN;
+    const double norm = block_norm(sc, lobin, numdata, fft, reinterpret_cast<float *>(fsm), &s_norm);
     // -locpow: per-bin factors from the window's powers that block_norm left in
-    // shared memory (superblocks are never formed with it)
-    const bool locpow = !sb && sc.nph <= 0.0f && sc.norm_type == 1;
+    // shared memory
+    const bool locpow = sc.nph <= 0.0f && sc.norm_type == 1;
     const float *pw = reinterpret_cast<const float *>(fsm);
     // spread data d[i] = norm * x[i mod numdata] at even samples: the
     // reference's window of numdata bins repeated with period fftlen_ref, so
@@ -380,9 +353,8 @@ __global__ void __launch_bounds__(256) k_prep(const ab_bank *banks, const int *b
     __syncthreads();                    // pw aliases the FFT scratch
     fft_run<LH, -1>(v, sm, t, tw);
     if (grp == 0) {
-        float2 *o = xhat + (long long) bi * xhat_per_block + b.xhat_off;
 #pragma unroll
-        for (int m = 0; m < 16; m++) o[t + SH::NT * m] = v[m];
+        for (int m = 0; m < 16; m++) xhat[t + SH::NT * m] = v[m];
     }
 }
 
@@ -394,15 +366,15 @@ static size_t prep_smem(const ab_bank &b)
     return fftsm > (size_t) n2 * sizeof(float) ? fftsm : (size_t) n2 * sizeof(float);
 }
 
-static cudaError_t launch_prep_one(int LH, dim3 grid, size_t smem, const ab_bank *bp, const int *bidx,
-                                   const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                                   float2 *xhat, long long xhat_per_block, cudaStream_t st)
+cudaError_t launch_prep(const ab_bank *bank_dev, const ab_bank &b, const SearchConsts &sc, const BlockBatch &bb,
+                        const float2 *fft, float2 *xhat, cudaStream_t st)
 {
-    switch (LH) {
+    const size_t smem = prep_smem(b);
+    switch (b.L / 2) {
 #define AB_PREP_CASE(N)                                                                       \
     case N:                                                                                   \
         cudaFuncSetAttribute(k_prep<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-        k_prep<N><<<grid, 256, smem, st>>>(bp, bidx, sc, bb, fft, xhat, xhat_per_block);      \
+        k_prep<N><<<1, 256, smem, st>>>(bank_dev, sc, bb, fft, xhat);                         \
         break;
         AB_PREP_CASE(256)
         AB_PREP_CASE(512)
@@ -413,97 +385,6 @@ static cudaError_t launch_prep_one(int LH, dim3 grid, size_t smem, const ab_bank
         default:
             return cudaErrorInvalidValue;
     }
-    return cudaSuccess;
-}
-
-cudaError_t launch_prep(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
-                        const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                        float2 *xhat, long long xhat_per_block, int *bidx, cudaStream_t st)
-{
-    cudaError_t e;
-    if (!bidx) {
-        // one launch per bank (a 1-bank grid by offsetting the bank pointer)
-        for (int k = 0; k < nbanks; k++) {
-            const ab_bank &b = banks_host[k];
-            e = launch_prep_one(b.L / 2, dim3(1, corr_units(b, sc, bb.nblk)), prep_smem(b),
-                                banks_dev + k, nullptr, sc, bb, fft, xhat, xhat_per_block, st);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaGetLastError();
-    }
-    // one launch per transform length over the banks listed in bidx: the
-    // separate launches of a batch's banks are small grids that leave most of
-    // the GPU idle and run one after another
-    std::vector<int> order;
-    std::vector<int> starts;
-    for (int LH = 256; LH <= 4096; LH *= 2) {
-        starts.push_back((int) order.size());
-        for (int k = 0; k < nbanks; k++)
-            if (banks_host[k].L / 2 == LH) order.push_back(k);
-    }
-    starts.push_back((int) order.size());
-    if ((int) order.size() != nbanks) return cudaErrorInvalidValue;
-    e = cudaMemcpyAsync(bidx, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    int gi = 0;
-    for (int LH = 256; LH <= 4096; LH *= 2, gi++) {
-        const int lo = starts[gi], hi = starts[gi + 1];
-        if (hi == lo) continue;
-        int units = 0;
-        size_t smem = 0;
-        for (int i = lo; i < hi; i++) {
-            const ab_bank &b = banks_host[order[i]];
-            units = std::max(units, corr_units(b, sc, bb.nblk));
-            smem = std::max(smem, prep_smem(b));
-        }
-        e = launch_prep_one(LH, dim3(hi - lo, units), smem, banks_dev, bidx + lo, sc, bb, fft,
-                            xhat, xhat_per_block, st);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaGetLastError();
-}
-
-// Block normalisations of one superblock bank: sc.norms[block * nbanks +
-// bank index] = 1/sqrt(median/ln 2) over the block's own window of
-// fftlen_ref / 2 bins (src/accel_utils.c:1079-1099).
-__global__ void __launch_bounds__(256) k_norms(const ab_bank *banks, const int *bidx, SearchConsts sc,
-                                               BlockBatch bb, const float2 *fft, double *norms)
-{
-    extern __shared__ float2 fsm[];
-    __shared__ double s_norm;
-    const ab_bank b = banks[bidx[blockIdx.x]];
-    const int bi = blockIdx.y;
-    ab_hgeom g;
-    block_geom(sc, b, bb.startr[bi], &g);
-    const double n = block_norm(sc, g.rlo - b.hw0, b.fftlen_ref / AB_NUMBETWEEN, fft,
-                                reinterpret_cast<float *>(fsm), &s_norm);
-    if (threadIdx.x == 0) norms[(long long) bi * sc.nbanks + b.index] = n;
-}
-
-cudaError_t launch_norms(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
-                         const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                         int *bidx, cudaStream_t st)
-{
-    if (!sc.superblocks) return cudaSuccess;
-    // every superblock bank of the batch in one launch
-    std::vector<int> list;
-    size_t smem = 0;
-    for (int k = 0; k < nbanks; k++) {
-        const ab_bank &b = banks_host[k];
-        if (b.sbm <= 1) continue;
-        int numdata = b.fftlen_ref / AB_NUMBETWEEN, n2 = 1;
-        while (n2 < numdata) n2 <<= 1;
-        smem = std::max(smem, (size_t) n2 * sizeof(float));
-        list.push_back(k);
-    }
-    if (list.empty()) return cudaSuccess;
-    if (smem > 200 * 1024 || !bidx) return cudaErrorInvalidValue;
-    cudaError_t e = cudaMemcpyAsync(bidx, list.data(), sizeof(int) * list.size(),
-                                    cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-    cudaFuncSetAttribute(k_norms, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_norms<<<dim3((unsigned) list.size(), bb.nblk), 256, smem, st>>>(
-        banks_dev, bidx, sc, bb, fft, const_cast<double *>(sc.norms));
     return cudaGetLastError();
 }
 
@@ -514,7 +395,7 @@ cudaError_t launch_norms(const ab_bank *banks_dev, const ab_bank *banks_host, in
 // which is the reference's circular correlation over fftlen_ref.
 __global__ void __launch_bounds__(256) k_prep_time(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
                                                    const float2 *fft, float2 *dtime,
-                                                   long long dt_per_block)
+                                                   long long dt_per_block, double *flags)
 {
     extern __shared__ float2 fsm[];
     __shared__ double s_norm;
@@ -528,6 +409,7 @@ __global__ void __launch_bounds__(256) k_prep_time(const ab_bank *banks, SearchC
     const bool locpow = sc.nph <= 0.0f && sc.norm_type == 1;
     const float *pw = reinterpret_cast<const float *>(fsm);
     float2 *o = dtime + (long long) bi * dt_per_block + b.dtime_off;
+    bool bad = false;
     for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
         long long bin = lobin + i - sc.obs_lobin;
         float2 x = make_float2(0.f, 0.f);
@@ -540,13 +422,19 @@ __global__ void __launch_bounds__(256) k_prep_time(const ab_bank *banks, SearchC
                 x = make_float2((float) ((double) v.x * norm), (float) ((double) v.y * norm));
             }
         }
+        bad |= !(isfinite(x.x) && isfinite(x.y));
         o[i] = x;
+    }
+    if (flags) {
+        // a value that is not finite spoils every cell of its block
+        bad = __syncthreads_or(bad);
+        if (threadIdx.x == 0) flags[(long long) bank * bb.nblk + bi] = bad ? (double) NAN : 1.0;
     }
 }
 
 cudaError_t launch_prep_time(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
                              const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                             float2 *dtime, long long dt_per_block, cudaStream_t st)
+                             float2 *dtime, long long dt_per_block, double *flags, cudaStream_t st)
 {
     int n2max = 1;
     for (int k = 0; k < nbanks; k++) {
@@ -558,80 +446,39 @@ cudaError_t launch_prep_time(const ab_bank *banks_dev, const ab_bank *banks_host
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     cudaFuncSetAttribute(k_prep_time, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     dim3 grid(nbanks, bb.nblk);
-    k_prep_time<<<grid, 256, smem, st>>>(banks_dev, sc, bb, fft, dtime, dt_per_block);
+    k_prep_time<<<grid, 256, smem, st>>>(banks_dev, sc, bb, fft, dtime, dt_per_block, flags);
     return cudaGetLastError();
 }
 
 // ======================================================================
 // (b) correlation
 // ======================================================================
-// Correlation of one (block, bank) data spectrum with a tile of templates:
-// the data spectrum is staged in shared memory once, templates stream from
-// L2 (each template row is read by every block of the batch).
+// Correlation of one block's data spectrum with a tile of templates of one
+// bank: the data spectrum is staged in shared memory once, templates stream
+// from L2.  The searches and plane calls use ab_corr.cu; this serves
+// ab_fderivs_vol_noalloc, whose caller holds templates of the bank's L points.
 template <int L>
 __global__ void __launch_bounds__(FftShape<L>::CTA, FftShape<L>::MINB) k_corr(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
-                                              const CorrItem *items, const float2 *xhat,
-                                              long long xhat_per_block, const float2 *tmpl,
-                                              float *planes, long long plane_per_block,
-                                              float *fullplane)
+                                              const CorrItem *items, const float2 *xhat, long long xhat_per_block,
+                                              const float2 *tmpl, float *planes, long long plane_per_block)
 {
     using SH = FftShape<L>;
     extern __shared__ float2 fsm[];
-    __shared__ long long s_off[AB_MAX_SBM];
-    __shared__ float s_scale[AB_MAX_SBM];
-    __shared__ int s_c0[AB_MAX_SBM], s_lim[AB_MAX_SBM];
-    __shared__ int s_sblim;                             // superblock: columns < s_sblim may be kept
     float2 *xs = fsm;                                   // [L/2]
-    const CorrItem it = items[blockIdx.x];              // it.bi: transform unit
+    const CorrItem it = items[blockIdx.x];
     const ab_bank b = banks[it.bank];
     const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
     // exchange buffers: one per transform group, a second set where the
     // transform has exactly two exchanges (fewer barriers)
-    constexpr int NBUF = SH::DBUF ? 2 : 1;
     float2 *sm = fsm + L / 2 + grp * SH::SMEM;
     float2 *sm2 = SH::DBUF ? fsm + L / 2 + (SH::G + grp) * SH::SMEM : nullptr;
-    // column -> block map of a superblock: low / high nibble = first / second
-    // block whose sub-plane holds the column (15 = none)
-    unsigned char *cmap = reinterpret_cast<unsigned char *>(fsm + L / 2 + NBUF * SH::G * SH::SMEM);
     const float2 *xsrc = xhat + (long long) it.bi * xhat_per_block + b.xhat_off;
     for (int i = threadIdx.x; i < L / 2; i += blockDim.x) xs[i] = xsrc[i];
-    const bool sb = !sc.inmem && sc.superblocks && b.sbm > 1;
-    const int b0 = sb ? it.bi * b.sbm : it.bi;
     ab_hgeom g;
-    block_geom(sc, b, bb.startr[b0], &g);
+    block_geom(sc, b, bb.startr[it.bi], &g);
     const int offset = 2 * b.hw0;
-    const int numrs = g.numrs;
+    const int lim = min(g.numrs, b.numrs_max);
     const float invL2 = 1.0f / ((float) L * (float) L);
-    if (sb) {
-        // superblock: block j's column kk is transform column 2 (rlo_j - rlo_0) + kk;
-        // its powers scale by (norm_j / norm_0)^2 (the transform used norm_0)
-        const int mb = min(b.sbm, bb.nblk - b0);
-        if ((int) threadIdx.x < mb) {
-            const int j = threadIdx.x;
-            ab_hgeom gj;
-            block_geom(sc, b, bb.startr[b0 + j], &gj);
-            const int c0 = (int) (2 * (gj.rlo - g.rlo));
-            s_c0[j] = c0;
-            s_lim[j] = max(0, min(gj.numrs, b.numrs_max));
-            s_off[j] = (long long) (b0 + j) * plane_per_block + b.plane_off - c0;
-            const double r = sc.norms[(long long) (b0 + j) * sc.nbanks + b.index] /
-                             sc.norms[(long long) b0 * sc.nbanks + b.index];
-            s_scale[j] = (float) (r * r);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int e = 0;
-            for (int j = 0; j < mb; j++) e = max(e, s_c0[j] + s_lim[j]);
-            s_sblim = e;
-        }
-        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
-            unsigned code = 0xFFu;
-            for (int j = 0; j < mb; j++)
-                if ((unsigned) (kk - s_c0[j]) < (unsigned) s_lim[j])
-                    code = ((code & 0x0Fu) == 0x0Fu) ? ((code & 0xF0u) | j) : ((code & 0x0Fu) | (j << 4));
-            cmap[kk] = (unsigned char) code;
-        }
-    }
     FftTw<L, 1> tw;                                     // twiddle bases in registers
     tw.init(t);
     __syncthreads();
@@ -652,47 +499,9 @@ __global__ void __launch_bounds__(FftShape<L>::CTA, FftShape<L>::MINB) k_corr(co
             for (int m = 0; m < 16; m++) v[m] = make_float2(0.f, 0.f);
         }
         fft_run<L, 1>(v, sm, t, tw, sm2);
-        if (valid && sb) {
-            // outputs m of this warp's lanes that can land in a block's
-            // columns [0, s_sblim): a warp spans 32 consecutive t of one
-            // transform, so the range is uniform and the rest is skipped
-            // (superblock outputs cost a column lookup and one or two scaled
-            // stores each; the single-block stores are cheaper than the test,
-            // measured; not at 8192 points, where the bounds would spill)
-            constexpr bool PRUNE = L <= 4096;
-            const int tw0 = t & ~31;
-            const long long row = (long long) tl * b.numrs_max;
-            const int m_lo = PRUNE ? max(0, (offset - tw0 - 31 + SH::NT - 1) / SH::NT) : 0;
-            const int m_hi = PRUNE ? (s_sblim + offset - tw0 - 1) / SH::NT : 15;
-#pragma unroll
-            for (int m = 0; m < 16; m++) {
-                if (m < m_lo || m > m_hi) continue;
-                const int kk = t + SH::NT * m - offset;
-                if (kk >= 0) {
-                    const unsigned code = cmap[kk];
-                    const float pw = fmaf(v[m].x, v[m].x, v[m].y * v[m].y) * invL2;
-                    unsigned j = code & 0x0Fu;
-                    if (j < AB_MAX_SBM) planes[s_off[j] + row + kk] = pw * s_scale[j];
-                    j = code >> 4;
-                    if (j < AB_MAX_SBM) planes[s_off[j] + row + kk] = pw * s_scale[j];
-                }
-            }
-        } else if (valid) {
-            float *out;
-            long long lim = numrs;
-            if (sc.inmem) {
-                // full f-fdot plane row tl (numws = 1), column 2 rlo + kk
-                // (fund_to_ffdotplane, src/accel_utils.c:1219-1233)
-                out = fullplane + (long long) tl * sc.rlen + g.rlo * AB_RDR;
-                if (bb.is_pre) {
-                    long long room = sc.clip_col - g.rlo * AB_RDR;
-                    if (room < lim) lim = room;
-                }
-            } else {
-                out = planes + (long long) it.bi * plane_per_block + b.plane_off +
-                      (long long) tl * b.numrs_max;
-                if (lim > b.numrs_max) lim = b.numrs_max;
-            }
+        if (valid) {
+            float *out = planes + (long long) it.bi * plane_per_block + b.plane_off +
+                         (long long) tl * b.numrs_max;
 #pragma unroll
             for (int m = 0; m < 16; m++) {
                 int kk = t + SH::NT * m - offset;
@@ -705,19 +514,18 @@ __global__ void __launch_bounds__(FftShape<L>::CTA, FftShape<L>::MINB) k_corr(co
 cudaError_t launch_corr(int L, const ab_bank *banks_dev, const SearchConsts &sc,
                         const BlockBatch &bb, const CorrItem *items, int nitems,
                         const float2 *xhat, long long xhat_per_block, const float2 *tmpl,
-                        float *planes, long long plane_per_block, float *fullplane,
-                        cudaStream_t st)
+                        float *planes, long long plane_per_block, cudaStream_t st)
 {
     if (nitems <= 0) return cudaSuccess;
     switch (L) {
 #define AB_CORR_CASE(N)                                                                       \
     case N: {                                                                                 \
         using SH = FftShape<N>;                                                               \
-        const size_t smem = (size_t) (N / 2 + (SH::DBUF ? 2 : 1) * SH::G * SH::SMEM) *      \
-                            sizeof(float2) + (size_t) N;                                     \
+        const size_t smem = (size_t) (N / 2 + (SH::DBUF ? 2 : 1) * SH::G * SH::SMEM) *        \
+                            sizeof(float2);                                                  \
         cudaFuncSetAttribute(k_corr<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
         k_corr<N><<<nitems, SH::CTA, smem, st>>>(banks_dev, sc, bb, items, xhat, xhat_per_block, \
-                                                 tmpl, planes, plane_per_block, fullplane);   \
+                                                 tmpl, planes, plane_per_block);              \
         break;                                                                                \
     }
         AB_CORR_CASE(512)

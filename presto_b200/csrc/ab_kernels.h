@@ -18,8 +18,6 @@ struct SearchConsts {
     float nph;
     float powcut[AB_MAX_STAGES];
     unsigned *err;             // device error word for bounded waits; may be null
-    int superblocks;           // standard search: banks with sbm > 1 share transforms
-    const double *norms;       // [block][bank] normalisations (superblock banks)
     int norm_type;             // 0: block median, 1: local power (-locpow)
 };
 
@@ -28,7 +26,23 @@ struct BlockBatch {
     const double *startr;      // device array [nblk]
     long long block0;          // key ordinal of item 0
     int nblk;
-    int is_pre;                // pre-pass blocks (in-memory mode only)
+    int npre0;                 // first of the pre-pass blocks (in-memory correlation), else nblk
+};
+
+constexpr int AB_SEG_BINS = 1024;   // bins of a correlation segment's window (ab_corr.cu)
+
+// The units (segments) and CTAs of one bank's class of templates in a batch:
+// unit u of blocks [blk0, blk0 + nblk) starts u V columns behind block blk0's
+// first or, nsub > 0 (banks correlated by each block's own data), (u mod nsub) V
+// behind that of block blk0 + u / nsub.  CTA c takes unit c mod nunits and the
+// templates perm[t_lo + tile (c / nunits) ...].
+struct SegGroup {
+    int bank, hw, V, nunits, unit0, cta0, t_lo, nt, tile, blk0, nblk, nsub;
+};
+
+struct SegCols {               // a block's columns in a bank's plane
+    long long c0;              // first, absolute (2 rlo)
+    int lim, pad;              // columns to fill
 };
 
 struct CorrItem {              // one CTA of the correlation kernel
@@ -48,35 +62,33 @@ struct HitBuf {
 
 // kernel set (a): templates
 void launch_twiddle64(double2 *tw, int n, int sign, cudaStream_t st);
-cudaError_t launch_templates(const ab_bank *bank, float2 *bank_out, const double2 *tw_place,
-                             const double2 *tw_chirp_all, int chirp_max_log2,
-                             double2 *scratch, size_t scratch_elems, cudaStream_t st);
+cudaError_t launch_templates(const ab_bank *bank, int t_lo, int t_hi, int L, float2 *out,
+                             const double2 *tw_all, int max_log2, cudaStream_t st);
 cudaError_t launch_response(double roffset, int numbetween, double z, double w, int numkern,
                             float2 *out, const double2 *tw_chirp_all, int chirp_max_log2,
                             double2 *scratch, cudaStream_t st);
 
-// kernel set (b): spectrum preparation and correlation.  bidx (device, room
-// for nbanks ints): banks of one transform length go out in one launch,
-// listed there; NULL: one launch per bank (no upload)
-cudaError_t launch_prep(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
-                        const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                        float2 *xhat, long long xhat_per_block, int *bidx, cudaStream_t st);
-// per-block normalisations of the superblock banks among banks_host[0..nbanks)
-// into sc.norms[block * sc.nbanks + bank index], in one launch listing them in
-// bidx (device, room for nbanks ints)
-cudaError_t launch_norms(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
-                         const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                         int *bidx, cudaStream_t st);
-// transform units (superblocks, or blocks) of a bank in a batch of nblk blocks
-inline int corr_units(const ab_bank &b, const SearchConsts &sc, int nblk)
-{
-    return (sc.superblocks && b.sbm > 1) ? (nblk + b.sbm - 1) / b.sbm : nblk;
-}
+// kernel set (b): correlation of the searches and plane calls.  cols and norms:
+// [bank][block] of the nbanks banks from banks_dev on (group bank indices count
+// from there); planes of the standard mode, or the in-memory plane (sc.inmem)
+cudaError_t launch_seg_cols(const ab_bank *banks_dev, int nbanks, const SearchConsts &sc, const BlockBatch &bb,
+                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, cudaStream_t st);
+cudaError_t launch_seg_fwd(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                           const SegGroup *groups, int ngroups, int nunits, const SegCols *cols,
+                           const double *norms, const float2 *fft, const float2 *dtime, long long dt_per_block,
+                           float2 *xhat, cudaStream_t st);
+cudaError_t launch_corr_seg(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                            const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
+                            const double *norms, const float2 *xhat, const float2 *tmpl, const int *perm,
+                            float *planes, long long plane_per_block, cudaStream_t st);
+
+// one block and bank with caller-held templates (ab_fderivs_vol_noalloc)
+cudaError_t launch_prep(const ab_bank *bank_dev, const ab_bank &b, const SearchConsts &sc, const BlockBatch &bb,
+                        const float2 *fft, float2 *xhat, cudaStream_t st);
 cudaError_t launch_corr(int L, const ab_bank *banks_dev, const SearchConsts &sc,
                         const BlockBatch &bb, const CorrItem *items, int nitems,
                         const float2 *xhat, long long xhat_per_block, const float2 *tmpl,
-                        float *planes, long long plane_per_block, float *fullplane,
-                        cudaStream_t st);
+                        float *planes, long long plane_per_block, cudaStream_t st);
 
 // kernel sets (c)+(d): harmonic summing fused with the threshold search
 cudaError_t launch_harmsum_std(const ab_bank *banks_dev, const SearchConsts &sc,
@@ -126,9 +138,10 @@ cudaError_t launch_tc_raw(const ab_bank *b, int stride, float2 *out, const doubl
 cudaError_t launch_tc_pack(const ab_bank *b, const TcTile *tiles_dev, int ntiles, int nks_max,
                            const int *perm_dev, const float2 *raw, int stride,
                            unsigned char *pack, int fp16, cudaStream_t st);
+// flags (may be null): [bank][block], NaN where a value is not finite, else 1
 cudaError_t launch_prep_time(const ab_bank *banks_dev, const ab_bank *banks_host, int nbanks,
                              const SearchConsts &sc, const BlockBatch &bb, const float2 *fft,
-                             float2 *dtime, long long dt_per_block, cudaStream_t st);
+                             float2 *dtime, long long dt_per_block, double *flags, cudaStream_t st);
 cudaError_t launch_corr_tc(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
                            const TcItem *items, int nitems, const TcTile *tiles, const int *perm,
                            const float2 *dtime, long long dt_per_block, const unsigned char *pack,

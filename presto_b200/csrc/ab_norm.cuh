@@ -3,6 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "ab_kernels.h"
+#include "ab_select.cuh"
+
 namespace ab {
 
 // invsqrtf (src/misc_utils.c:291-302): the published fast inverse square
@@ -33,6 +36,50 @@ __device__ __forceinline__ float locpow_invsqrt(const float *pw, int numdata, in
     const double normal = (double) ((numdata / 2) / 20);
     const float local = (float) (s * normal * (2.0 / (double) numdata));
     return fast_invsqrtf(local);
+}
+
+// Block normalisation 1/sqrt(median(|X|^2)/ln 2) of the numdata bins from
+// lobin (zero outside the spectrum), or 1/sqrt(nph) when nph is given
+// (src/accel_utils.c:1079-1099).  The median is taken over float POWER()
+// values without FMA, sorted exactly; even counts average the two central
+// values (GSL semantics).  pw: shared scratch of numdata floats.
+// Called by every thread of the CTA.
+// The block's normalisation (src/accel_utils.c:1079-1113): 1/sqrt(nph) with
+// -photon, else 1/sqrt(median/ln 2) of the window's powers.  With -locpow
+// (sc.norm_type 1) it leaves the window's powers in pw for locpow_invsqrt
+// and returns 0 (the factor is per bin).
+__device__ __forceinline__ double block_norm(const SearchConsts &sc, long long lobin, int numdata, const float2 *fft,
+                             float *pw, double *s_norm)
+{
+    if (sc.nph > 0.0f) {
+        if (threadIdx.x == 0) *s_norm = 1.0 / sqrt((double) sc.nph);
+    } else if (sc.norm_type == 1) {
+        for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
+            long long bin = lobin + i - sc.obs_lobin;
+            float2 v = (bin >= 0 && bin < sc.numbins) ? fft[bin] : make_float2(0.f, 0.f);
+            pw[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
+        }
+        if (threadIdx.x == 0) *s_norm = 0.0;
+    } else {
+        // block median of |X|^2 in float (POWER(), no FMA), src/accel_utils.c:1087-1099
+        for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
+            long long bin = lobin + i - sc.obs_lobin;
+            float2 v = (bin >= 0 && bin < sc.numbins) ? fft[bin] : make_float2(0.f, 0.f);
+            pw[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
+        }
+        __syncthreads();
+        // the two central order statistics (equal for odd counts), as a sort gives them
+        __shared__ unsigned s_hist[256], s_res[2];
+        const float lo = select_rank(pw, numdata, (numdata - 1) / 2, s_hist, s_res);
+        const float hi = (numdata & 1) ? lo : next_rank(pw, numdata, (numdata - 1) / 2, lo, s_res);
+        if (threadIdx.x == 0) {
+            double m = (numdata & 1) ? (double) lo : 0.5 * ((double) lo + (double) hi);
+            float med = (float) m;
+            *s_norm = 1.0 / sqrt((double) med / 0.69314718055994530942);
+        }
+    }
+    __syncthreads();
+    return *s_norm;
 }
 
 }  // namespace ab

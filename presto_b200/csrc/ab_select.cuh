@@ -66,4 +66,33 @@ __device__ __forceinline__ float select_rank(const float *a, int n, int k, unsig
     return __uint_as_float(prefix);
 }
 
+// The (k + 1)-th smallest, given the k-th (0-based; n > k + 1): v again if
+// more than k + 1 values are at most v, else the smallest above it.  One pass
+// instead of a second select.  Called by every thread of the CTA.
+__device__ __forceinline__ float next_rank(const float *a, int n, int k, float v, unsigned *s_res)
+{
+    if (threadIdx.x == 0) {
+        s_res[0] = 0u;
+        s_res[1] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    const unsigned vb = __float_as_uint(v);
+    unsigned upto = 0, above = 0xFFFFFFFFu;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const unsigned u = __float_as_uint(a[i]);
+        upto += u <= vb;
+        if (u > vb) above = min(above, u);
+    }
+    upto = __reduce_add_sync(0xffffffffu, upto);
+    above = __reduce_min_sync(0xffffffffu, above);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_res[0], upto);
+        atomicMin(&s_res[1], above);
+    }
+    __syncthreads();
+    const float r = s_res[0] > (unsigned) k + 1u ? v : __uint_as_float(s_res[1]);
+    __syncthreads();
+    return r;
+}
+
 }  // namespace ab

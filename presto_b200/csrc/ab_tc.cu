@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(128, 1) k_corr_tc(TcArgs a)
         // src/accel_utils.c:1219-1233); pre-pass blocks stop at clip_col
         rowbase = a.fullplane + g.rlo * AB_RDR;
         rowstride = sc.rlen;
-        if (a.bb.is_pre) {
+        if (a.bb.npre0 == 0) {
             long long room = sc.clip_col - g.rlo * AB_RDR;
             if (room < lim) lim = room;
         }

@@ -1,0 +1,87 @@
+"""The correlation's segments (ab_corr.cu), which run over block boundaries and differ
+per class of templates: a whole search gives the threshold crossings that searches of single
+blocks give, each cut into segments from its own first column.  Both are sums of the
+same products in FP32; a crossing may be missing from one side only within 1e-5 of its
+power cut, and powers agree to 1e-5 (measured differences stay below 2e-6)."""
+import numpy as np
+import pytest
+
+from presto_b200 import synth
+
+pytestmark = pytest.mark.gpu
+DT = 64e-6
+
+
+def _hits(ctx, obs, fft, first=0, count=-1):
+    ctx.search(obs, fft, first_block=first, max_blocks=count)
+    blk, st, wi, zi, ri, pw = ctx.last_hits()
+    return {tuple(k): p for k, p in zip(zip(blk, st, wi, zi, ri), pw)}
+
+
+def _same(one, whole, obs, block):
+    want = {k: p for k, p in whole.items() if k[0] == block}
+    for k in set(one) ^ set(want):
+        cut = obs.powcut[k[1]]
+        assert abs((one.get(k) or want.get(k)) - cut) <= 1e-5 * cut, (k, cut)
+    for k in set(one) & set(want):
+        assert abs(one[k] - want[k]) <= 1e-5 * want[k], (k, one[k], want[k])
+    return len(want)
+
+
+@pytest.mark.parametrize("N,zmax,wmax,numharm,kw", [
+    (1 << 18, 0, 0, 32, {}),                    # one template a bank; 46 blocks to a segment of the narrowest
+    (1 << 18, 50, 0, 32, {}),
+    (1 << 19, 690, 0, 8, {}),                   # the widest templates, segments of 448 columns
+    (300000, 200, 0, 16, {}),
+    (1 << 18, 100, 200, 16, {}),                # a bank whose reference transform wraps
+    (1 << 18, 60, 100, 8, dict(locpow=True)),   # every block's own data
+    (1 << 18, 60, 0, 4, dict(photon=0.7)),
+    (1 << 18, 100, None, 8, {}),                # the in-memory plane, its pre-pass blocks among them
+    (1 << 17, 20, None, 4, dict(rlo=700.5)),
+])
+def test_whole_search_is_its_blocks(ctx, ablib, N, zmax, wmax, numharm, kw):
+    T = N * DT
+    ps = [dict(r=0.013 * N, z=0.3 * zmax, harms=[(0.09, 0.3)] * 6), dict(r=3.1 * T, z=-0.1 * zmax, harms=[(0.07, 1.0)] * 6)]
+    fft = synth.spectrum(synth.time_series(N, N + zmax, ps))
+    obs = ablib.obs_init(ablib.make_params(N, DT, fft.size, zmax=zmax, wmax=wmax, numharm=numharm, sigma=1.0, **kw))
+    whole = _hits(ctx, obs, fft)
+    nb = ablib.num_blocks(obs)
+    busy = sorted({k[0] for k in whole})
+    assert busy
+    for block in sorted({0, nb // 2, nb - 1, *busy[:2], *busy[len(busy) // 2:len(busy) // 2 + 2], busy[-1]}):
+        _same(_hits(ctx, obs, fft, block, 1), whole, obs, block)
+
+
+def test_bad_bins_spoil_their_blocks_alone(ctx, ablib):
+    """A bin that is not a number, an infinite one and a stretch of zeros: every cell of the blocks whose
+    windows hold them crosses (as in the blocks' own transforms), and the others are those of the
+    clean spectrum."""
+    N = 1 << 18
+    fft = synth.spectrum(synth.time_series(N, 5, [dict(r=70001.3, z=3.0, harms=[(0.12, 0.0)])]))
+    obs = ablib.obs_init(ablib.make_params(N, DT, fft.size, zmax=10, wmax=0, numharm=1, sigma=1.0))
+    clean = _hits(ctx, obs, fft)
+    bad = fft.copy()
+    bad[50000] = np.nan
+    bad[52000] = complex(0.0, np.inf)
+    bad[90000:92000] = 0.0
+    got = _hits(ctx, obs, bad)
+    hw, step, numdata = 21, obs.rstep, 1024
+    spoilt = set()
+    for b in range(ablib.num_blocks(obs)):
+        lo = int(obs.rlo) + b * step - hw
+        win = bad[max(lo, 0):lo + numdata]
+        if not np.all(np.isfinite(win)) or np.median(np.abs(win)) == 0.0:
+            spoilt.add(b)
+    assert len(spoilt) >= 4
+    cells = obs.numz * obs.corr_uselen
+    for b in spoilt:
+        assert sum(k[0] == b for k in got) == cells
+    near = {b + d for b in spoilt for d in (-1, 0, 1)} - spoilt
+    for b in range(ablib.num_blocks(obs)):
+        if b in spoilt:
+            continue
+        one = {k: p for k, p in got.items() if k[0] == b}
+        window = bad[max(int(obs.rlo) + b * step - hw, 0):int(obs.rlo) + b * step - hw + numdata]
+        if b in near and np.any(window == 0.0):
+            continue                                    # its own median moved
+        _same(one, clean, obs, b)
