@@ -908,8 +908,13 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
             if (rc) return rc;
         }
         // the sums run in chunks of blocks through the ring of hit sets, so the
-        // host replays chunk k while the device sums the chunks after it
-        const long long nch = std::min<long long>(8, std::max<long long>(1, count / 32));
+        // host replays chunk k while the device sums the chunks after it.  A
+        // chunk costs a launch's latency, the hits' sigmas and a hand-over to
+        // the replay, some 40 us together: chunks of 2^27 harmonic values (about
+        // 100 us of sums) at least.
+        const long long values = (count * obs->corr_uselen * sc.numz) << (nstage - 1);
+        const long long nch = std::min<long long>({8, std::max<long long>(1, count / 32),
+                                                   std::max<long long>(1, values >> 27)});
         const long long csz = (count + nch - 1) / nch;
         int k = 0;
         for (long long c0 = first; count > 0 && c0 < first + count; c0 += csz, k++) {

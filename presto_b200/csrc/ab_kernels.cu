@@ -593,12 +593,14 @@ __device__ __forceinline__ void flush_hits(unsigned mask, const float *sums, lon
 constexpr int harmsum_min_ctas(int stages) { return stages <= 2 ? 1 : stages <= 4 ? 6 : (stages == 5 ? 4 : 3); }
 // The in-memory sum, up to 4 stages, keeps each subharmonic's last value in a
 // register and reads it again only when the subharmonic's row changes with z
-// (a subharmonic f keeps its row for ~1/f consecutive z rows); 5 CTAs per SM
-// leave room for it.  At 5 and 6 stages the 15 / 31 extra registers would go
-// to the stack (measured 2x slower), and in the standard-mode sum the same
-// change measured slower (jerk search 93.5 -> 111 ms), so those read every
+// (a subharmonic f keeps its row for ~1/f consecutive z rows); at 4 stages 3
+// CTAs per SM leave room for two columns' values (4 spill: N = 2^20, zmax = 200
+// search 1.90 ms against 1.03, and 1.52 with one column a thread and each
+// addition behind its load).  At 5 and 6 stages the 15 / 31 extra registers
+// would go to the stack (measured 2x slower), and in the standard-mode sum the
+// same change measured slower (jerk search 93.5 -> 111 ms), so those read every
 // value.
-constexpr int inmem_min_ctas(int stages) { return stages <= 2 ? 1 : stages <= 4 ? 5 : (stages == 5 ? 4 : 3); }
+constexpr int inmem_min_ctas(int stages) { return stages <= 2 ? 1 : stages == 4 || stages == 6 ? 3 : 4; }
 
 template <int STAGES>
 __global__ void __launch_bounds__(256, harmsum_min_ctas(STAGES)) k_harmsum_std(const ab_bank *banks, SearchConsts sc,
@@ -719,27 +721,45 @@ cudaError_t launch_harmsum_std(const ab_bank *banks_dev, const SearchConsts &sc,
 }
 
 // In-memory mode: fundamental and subharmonic powers come from the full
-// f-fdot plane (inmem_add_ffdotpows).  CTA = (block, z tile, r cells).
+// f-fdot plane (inmem_add_ffdotpows), whose columns run on through the blocks
+// (a block's columns end where the next one's begin, and the subharmonics'
+// columns depend on the plane's column alone).  CTA = (tile of columns, z
+// tile); a block's tail does not leave threads idle.  Up to 4 stages a thread
+// takes two columns, HS_RT apart: the row bookkeeping, the same for every
+// thread, serves both, and their sums are paired additions.  A row's new
+// subharmonic values are all asked for before the first is added: with each
+// addition behind its load a row took the latencies one after another.
+template <int STAGES> struct InmemShape {
+    static constexpr int COLS = STAGES <= 4 ? 2 : 1;       // columns per thread
+    static constexpr int TILE = HS_RT * COLS;
+};
+
 template <int STAGES>
 __global__ void __launch_bounds__(256, inmem_min_ctas(STAGES)) k_harmsum_inmem(SearchConsts sc, BlockBatch bb,
                                                        const float *plane, HitBuf hb, float *dbg,
                                                        int dbg_bi)
 {
-    constexpr int NSUB = (1 << (STAGES - 1)) - 1;
-    __shared__ int s_zrow[NSUB > 0 ? NSUB : 1][HS_ZT];
+    constexpr int NSUB = (1 << (STAGES - 1)) - 1, NS1 = NSUB > 0 ? NSUB : 1;
+    constexpr int COLS = InmemShape<STAGES>::COLS;
+    constexpr bool REUSE = STAGES <= 4;
+    __shared__ int s_zrow[NS1][HS_ZT];
     // bit h: subharmonic h reads another row than at the previous z row
     // (subharmonic f keeps its row for ~1/f consecutive z rows; the value read
     // there is kept in a register instead of read again)
     __shared__ unsigned s_new[HS_ZT];
     const int nzt = (sc.numz + HS_ZT - 1) / HS_ZT;
-    const int zt = blockIdx.x % nzt, bi = blockIdx.x / nzt;
-    const int r = blockIdx.y * HS_RT + threadIdx.x, z0 = zt * HS_ZT;
-    const double startr = bb.startr[bi];
-    const ab_hgeom g0 = ab_harm_geom(startr, startr + sc.rstep - AB_DR, 1, 1, sc.obs_zlo,
+    const int zt = blockIdx.x % nzt, z0 = zt * HS_ZT;
+    const ab_hgeom g0 = ab_harm_geom(bb.startr[0], bb.startr[0] + sc.rstep - AB_DR, 1, 1, sc.obs_zlo,
                                      sc.obs_wlo, sc.corr_uselen);
-    const bool ok = r < g0.numrs;
-    const int rlo = (int) g0.rlo;
-    int rind[NSUB > 0 ? NSUB : 1];
+    const long long ncol = (long long) bb.nblk * sc.corr_uselen;
+    const long long c0 = (long long) (blockIdx.x / nzt) * InmemShape<STAGES>::TILE + threadIdx.x;
+    bool ok[COLS];
+    int q[COLS], rind[NS1][COLS];                           // the plane's columns
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+        ok[c] = c0 + c * HS_RT < ncol;
+        q[c] = (int) (g0.rlo * AB_RDR + (ok[c] ? c0 + c * HS_RT : 0));
+    }
     {
         int h = 0;
 #pragma unroll
@@ -747,8 +767,11 @@ __global__ void __launch_bounds__(256, inmem_min_ctas(STAGES)) k_harmsum_inmem(S
 #pragma unroll
             for (int j = 0; j < (1 << (s - 1)); j++, h++) {
                 const double f = (double) (2 * j + 1) / (double) (1 << s);
-                long long ri = ok ? ab_inmem_rind(rlo, r, f) : 0;
-                rind[h] = (int) min(max(ri, 0ll), sc.rlen - 1);
+#pragma unroll
+                for (int c = 0; c < COLS; c++) {
+                    const long long ri = ab_inmem_rind(0, q[c], f);
+                    rind[h][c] = (int) min(max(ri, 0ll), sc.rlen - 1);
+                }
                 for (int zz = threadIdx.x; zz < HS_ZT; zz += blockDim.x) {
                     int z = z0 + zz;
                     int zi = (z < sc.numz) ? ab_inmem_zind(g0.zlo, z, f) : 0;
@@ -757,7 +780,7 @@ __global__ void __launch_bounds__(256, inmem_min_ctas(STAGES)) k_harmsum_inmem(S
             }
     }
     __syncthreads();
-    if (STAGES <= 4) {
+    if (REUSE) {
         for (int zz = threadIdx.x; zz < HS_ZT; zz += blockDim.x) {
             unsigned m = 0;
             for (int h = 0; h < NSUB; h++)
@@ -769,55 +792,72 @@ __global__ void __launch_bounds__(256, inmem_min_ctas(STAGES)) k_harmsum_inmem(S
     float pc[STAGES];
 #pragma unroll
     for (int s = 0; s < STAGES; s++) pc[s] = sc.powcut[s];
-    const long long block = bb.block0 + bi;
     const int zend = min(z0 + HS_ZT, sc.numz);
-    const bool dump = dbg && bi == dbg_bi && ok;
-    constexpr bool REUSE = STAGES <= 4;
-    float sv[REUSE && NSUB > 0 ? NSUB : 1];
-#pragma unroll
-    for (int h = 0; h < (REUSE ? NSUB : 1); h++) sv[h] = 0.f;
+    float2 sv[REUSE ? NS1 : 1];
     for (int z = z0; z < zend; z++) {
         const int zz = z - z0;
-        const unsigned nm = STAGES <= 4 ? s_new[zz] : 0u;
-        float sums[STAGES];
-        float sum = ok ? plane[(long long) z * sc.rlen + (long long) rlo * AB_RDR + r] : 0.f;
+        float2 sums[STAGES];
+        const float *row = plane + (long long) z * sc.rlen;
+        float2 sum = make_float2(row[q[0]], COLS == 2 ? row[q[COLS - 1]] : 0.f);
+        if constexpr (REUSE) {
+            const unsigned nm = s_new[zz];
+#pragma unroll
+            for (int h = 0; h < NSUB; h++)
+                if ((nm >> h) & 1u) {
+                    const float *sub = plane + (long long) s_zrow[h][zz] * sc.rlen;
+                    sv[h] = make_float2(sub[rind[h][0]], sub[rind[h][COLS - 1]]);
+                }
+        }
         sums[0] = sum;
-        unsigned mask = (ok && !(sum <= pc[0])) ? 1u : 0u;
+        bool hit = !(sum.x <= pc[0]) || (COLS == 2 && !(sum.y <= pc[0]));
         int h = 0;
 #pragma unroll
         for (int s = 1; s < STAGES; s++) {
 #pragma unroll
             for (int j = 0; j < (1 << (s - 1)); j++, h++) {
-                if constexpr (REUSE) {
-                    if (ok && ((nm >> h) & 1u))
-                        sv[h] = plane[(long long) s_zrow[h][zz] * sc.rlen + rind[h]];
-                    if (ok) sum += sv[h];
-                } else {
-                    if (ok) sum += plane[(long long) s_zrow[h][zz] * sc.rlen + rind[h]];
-                }
+                if constexpr (REUSE) sum = __fadd2_rn(sum, sv[h]);
+                else sum.x += plane[(long long) s_zrow[h][zz] * sc.rlen + rind[h][0]];
             }
             sums[s] = sum;
-            if (ok && !(sum <= pc[s])) mask |= 1u << s;
+            hit = hit || !(sum.x <= pc[s]) || (COLS == 2 && !(sum.y <= pc[s]));
         }
-        flush_hits<STAGES>(mask, sums, block, 0, z, r, hb);
-        if (dump) {
+        // one warp vote per row; lanes past the last column hold the first one's cells
+        const bool any = __any_sync(0xffffffffu, hit);
+        if (any || dbg) {
 #pragma unroll
-            for (int s = 0; s < STAGES; s++)
-                dbg[((long long) s * sc.numz + z) * g0.numrs + r] = sums[s];
+            for (int c = 0; c < COLS; c++) {
+                const long long col = c0 + c * HS_RT;
+                const int bi = (int) (ok[c] ? col / sc.corr_uselen : 0);
+                const int r = (int) (ok[c] ? col - (long long) bi * sc.corr_uselen : 0);
+#pragma unroll
+                for (int s = 0; s < STAGES; s++) {
+                    const float p = c ? sums[s].y : sums[s].x;
+                    if (any) emit_hit(ok[c] && !(p <= pc[s]), make_key(bb.block0 + bi, s, 0, z, r), p, hb);
+                    if (dbg && ok[c] && bi == dbg_bi)
+                        dbg[((long long) s * sc.numz + z) * sc.corr_uselen + r] = p;
+                }
+            }
         }
     }
+}
+
+template <int STAGES>
+static void launch_inmem(const SearchConsts &sc, const BlockBatch &bb, const float *fullplane, HitBuf hb, float *dbg,
+                         int dbg_bi, cudaStream_t st)
+{
+    const long long nzt = (sc.numz + HS_ZT - 1) / HS_ZT, ncol = (long long) bb.nblk * sc.corr_uselen;
+    const long long nct = (ncol + InmemShape<STAGES>::TILE - 1) / InmemShape<STAGES>::TILE;
+    k_harmsum_inmem<STAGES><<<(unsigned) (nzt * nct), HS_RT, 0, st>>>(sc, bb, fullplane, hb, dbg, dbg_bi);
 }
 
 cudaError_t launch_harmsum_inmem(const SearchConsts &sc, const BlockBatch &bb,
                                  const float *fullplane, HitBuf hb, float *dbg, int dbg_bi,
                                  cudaStream_t st)
 {
-    int nzt = (sc.numz + HS_ZT - 1) / HS_ZT;
-    dim3 grid((unsigned) (bb.nblk * nzt), (sc.corr_uselen + HS_RT - 1) / HS_RT);
     switch (sc.stages) {
 #define AB_HI_CASE(S)                                                                          \
     case S:                                                                                    \
-        k_harmsum_inmem<S><<<grid, HS_RT, 0, st>>>(sc, bb, fullplane, hb, dbg, dbg_bi);        \
+        launch_inmem<S>(sc, bb, fullplane, hb, dbg, dbg_bi, st);                               \
         break;
         AB_HI_CASE(1)
         AB_HI_CASE(2)
