@@ -588,9 +588,9 @@ __device__ __forceinline__ void flush_hits(unsigned mask, const float *sums, lon
 // HS_RT r cells); each thread owns one r cell, keeps its subharmonic r
 // indices (rinds) in registers and walks the z rows.  Plane row offsets of
 // every subharmonic for the tile's rows are staged in shared memory.
-// Latency-bound gathers: the register cap keeps 6 / 4 / 3 CTAs per SM at
-// 3-4 / 5 / 6 stages.
-constexpr int harmsum_min_ctas(int stages) { return stages <= 2 ? 1 : stages <= 4 ? 6 : (stages == 5 ? 4 : 3); }
+// Latency-bound gathers: the register cap keeps 4 / 3 CTAs per SM at 5 / 6
+// stages (the only ones it serves; k_harmsum_pair below for up to 4).
+constexpr int harmsum_min_ctas(int stages) { return stages == 5 ? 4 : 3; }
 // The in-memory sum, up to 4 stages, keeps each subharmonic's last value in a
 // register and reads it again only when the subharmonic's row changes with z
 // (a subharmonic f keeps its row for ~1/f consecutive z rows); at 4 stages 3
@@ -691,6 +691,159 @@ __global__ void __launch_bounds__(256, harmsum_min_ctas(STAGES)) k_harmsum_std(c
     }
 }
 
+// Up to 4 stages: two columns a thread, blockDim.x apart, so that a row's
+// address, read from shared memory, serves two loads and twice the loads are in
+// flight (two neighbouring columns would spread a warp's loads over twice the
+// bytes).  5 CTAs per SM: jerk search (zmax 200, wmax 300, 8 harmonics, N = 2^22)
+// 63.5 ms of sums, 73.2 at 4 and 78.0 at 6 (spills), 93.4 with one column.  At
+// 5 stages two columns leave 3 CTAs and take 49.3 ms against 32.0 (zmax = 600,
+// 16 harmonics, N = 2^23).
+template <int STAGES>
+__global__ void __launch_bounds__(256, 5) k_harmsum_pair(const ab_bank *banks, SearchConsts sc,
+                                                     BlockBatch bb, const float *planes,
+                                                     long long plane_per_block, HitBuf hb,
+                                                     float *dbg, int dbg_bi)
+{
+    constexpr int NSUB = (1 << (STAGES - 1)) - 1;
+    constexpr int NS1 = NSUB > 0 ? NSUB : 1;
+    constexpr int COLS = 2;
+    __shared__ const float *s_row[HS_ZT][NS1 + 1];      // [z][0] fundamental, [z][1+h] subharmonic h
+    __shared__ long long s_rlo[NS1];
+    __shared__ int s_zlo[NS1], s_wind[NS1];
+    const int nzt = (sc.numz + HS_ZT - 1) / HS_ZT;
+    const int rtile = COLS * (int) blockDim.x;
+    const int nrt = (sc.corr_uselen + rtile - 1) / rtile;
+    // r tile fastest: CTAs that share subharmonic row segments at their r
+    // boundaries run together, so the shared sectors come from L2
+    unsigned x = blockIdx.x;
+    const int rt = (int) (x % (unsigned) nrt);
+    x /= (unsigned) nrt;
+    const int zt = (int) (x % (unsigned) nzt);
+    x /= (unsigned) nzt;
+    const int wi = (int) (x % (unsigned) sc.numws);
+    const int bi = (int) (x / (unsigned) sc.numws);
+    const int r0 = rt * rtile + threadIdx.x;
+    const int z0 = zt * HS_ZT;
+    const double startr = bb.startr[bi];
+    const double lastr = startr + sc.rstep - AB_DR;
+    const ab_hgeom g0 = ab_harm_geom(startr, lastr, 1, 1, sc.obs_zlo, sc.obs_wlo, sc.corr_uselen);
+    const float *pb = planes + (long long) bi * plane_per_block;
+    // per-bank plane geometry of this block, once per CTA
+    if (NSUB > 0 && threadIdx.x < NSUB) {
+        const int h = threadIdx.x;
+        const ab_bank &bh = banks[h + 1];
+        const ab_hgeom gh = ab_harm_geom(startr, lastr, bh.numharm, bh.harmnum, sc.obs_zlo,
+                                         sc.obs_wlo, sc.corr_uselen);
+        s_rlo[h] = gh.rlo;
+        s_zlo[h] = gh.zlo;
+        s_wind[h] = min(max(ab_wind(g0.wlo, wi, bh.f, gh.wlo), 0), bh.nw - 1);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < (NSUB + 1) * HS_ZT; e += blockDim.x) {
+        const int h = e / HS_ZT - 1, zz = e % HS_ZT;
+        const int z = min(z0 + zz, sc.numz - 1);
+        if (h < 0) {
+            s_row[zz][0] = pb + banks[0].plane_off +
+                           ((long long) wi * sc.numz + z) * banks[0].numrs_max;
+        } else {
+            const ab_bank &bh = banks[h + 1];
+            int zi = min(max(ab_zind(sc.obs_zlo, z, bh.f, s_zlo[h]), 0), bh.nz - 1);
+            s_row[zz][h + 1] = pb + bh.plane_off + ((long long) s_wind[h] * bh.nz + zi) * bh.numrs_max;
+        }
+    }
+    // subharmonic r indices of this thread's cells (clamped, so every load is in bounds)
+    bool ok[COLS];
+    int rc[COLS], rind[NS1][COLS];
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+        const int r = r0 + c * (int) blockDim.x;
+        ok[c] = r < g0.numrs;
+        rc[c] = ok[c] ? r : 0;
+#pragma unroll
+        for (int h = 0; h < NSUB; h++)
+            rind[h][c] = min(max(ab_rind(startr, rc[c], banks[h + 1].f, s_rlo[h]), 0), banks[h + 1].numrs_max - 1);
+    }
+    __syncthreads();
+    const long long block = bb.block0 + bi;
+    const int zend = min(z0 + HS_ZT, sc.numz);
+    const bool dump = dbg && bi == dbg_bi;
+    for (int z = z0; z < zend; z++) {
+        const int zz = z - z0;
+        float sums[STAGES][COLS], sum[COLS];
+        bool hit = false;
+        const float *row = s_row[zz][0];
+#pragma unroll
+        for (int c = 0; c < COLS; c++) {
+            sum[c] = __ldg(row + rc[c]);
+            sums[0][c] = sum[c];
+            hit = hit || !(sum[c] <= sc.powcut[0]);
+        }
+        int h = 0;
+#pragma unroll
+        for (int s = 1; s < STAGES; s++) {
+#pragma unroll
+            for (int j = 0; j < (1 << (s - 1)); j++, h++) {
+                row = s_row[zz][h + 1];
+#pragma unroll
+                for (int c = 0; c < COLS; c++) sum[c] += __ldg(row + rind[h][c]);
+            }
+#pragma unroll
+            for (int c = 0; c < COLS; c++) {
+                sums[s][c] = sum[c];
+                hit = hit || !(sum[c] <= sc.powcut[s]);
+            }
+        }
+        // one warp vote per row; lanes past the block's end hold its cell 0
+        if (__any_sync(0xffffffffu, hit)) {
+#pragma unroll
+            for (int c = 0; c < COLS; c++)
+#pragma unroll
+                for (int s = 0; s < STAGES; s++)
+                    emit_hit(ok[c] && !(sums[s][c] <= sc.powcut[s]),
+                             make_key(block, s, wi, z, r0 + c * (int) blockDim.x), sums[s][c], hb);
+        }
+        if (dump) {
+#pragma unroll
+            for (int c = 0; c < COLS; c++)
+#pragma unroll
+                for (int s = 0; s < STAGES; s++)
+                    if (ok[c])
+                        dbg[(((long long) s * sc.numws + wi) * sc.numz + z) * g0.numrs + rc[c]] = sums[s][c];
+        }
+    }
+}
+
+// Threads per CTA: the multiple of 32 up to 256 whose tiles overhang the
+// block's columns least (1544 columns in tiles of 512 leave a quarter of the
+// threads idle, in tiles of 320 a thirtieth), the larger of equals.
+static int harmsum_pair_threads(int uselen)
+{
+    int best = 256;
+    long long least = -1;
+    for (int t = 256; t >= 128; t -= 32) {
+        const long long total = (uselen + 2 * t - 1) / (2 * t) * (2LL * t);
+        if (least < 0 || total < least) {
+            least = total;
+            best = t;
+        }
+    }
+    return best;
+}
+
+template <int STAGES>
+static cudaError_t launch_pair(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                               const float *planes, long long plane_per_block, HitBuf hb, float *dbg, int dbg_bi,
+                               cudaStream_t st)
+{
+    const int threads = harmsum_pair_threads(sc.corr_uselen);
+    const long long nzt = (sc.numz + HS_ZT - 1) / HS_ZT, nrt = (sc.corr_uselen + 2 * threads - 1) / (2 * threads);
+    const long long ncta = (long long) bb.nblk * sc.numws * nzt * nrt;
+    if (ncta < 1 || ncta > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+    k_harmsum_pair<STAGES><<<(unsigned) ncta, threads, 0, st>>>(banks_dev, sc, bb, planes, plane_per_block, hb, dbg,
+                                                                dbg_bi);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_harmsum_std(const ab_bank *banks_dev, const SearchConsts &sc,
                                const BlockBatch &bb, const float *planes,
                                long long plane_per_block, HitBuf hb, float *dbg, int dbg_bi,
@@ -702,15 +855,19 @@ cudaError_t launch_harmsum_std(const ab_bank *banks_dev, const SearchConsts &sc,
     if (ncta < 1 || ncta > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned) ncta;
     switch (sc.stages) {
+#define AB_HP_CASE(S)                                                                          \
+    case S:                                                                                    \
+        return launch_pair<S>(banks_dev, sc, bb, planes, plane_per_block, hb, dbg, dbg_bi, st);
+        AB_HP_CASE(1)
+        AB_HP_CASE(2)
+        AB_HP_CASE(3)
+        AB_HP_CASE(4)
+#undef AB_HP_CASE
 #define AB_HS_CASE(S)                                                                          \
     case S:                                                                                    \
         k_harmsum_std<S><<<grid, HS_RT, 0, st>>>(banks_dev, sc, bb, planes, plane_per_block, hb, \
                                                  dbg, dbg_bi);                                  \
         break;
-        AB_HS_CASE(1)
-        AB_HS_CASE(2)
-        AB_HS_CASE(3)
-        AB_HS_CASE(4)
         AB_HS_CASE(5)
         AB_HS_CASE(6)
 #undef AB_HS_CASE

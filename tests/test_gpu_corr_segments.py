@@ -85,3 +85,27 @@ def test_bad_bins_spoil_their_blocks_alone(ctx, ablib):
         if b in near and np.any(window == 0.0):
             continue                                    # its own median moved
         _same(one, clean, obs, b)
+
+
+@pytest.mark.parametrize("numharm", [1, 2, 4, 8, 16, 32])
+@pytest.mark.parametrize("zmax,wmax", [(0, 0), (70, 0), (200, 0), (40, 40)])
+def test_stage_sums_are_the_per_function_sums(ctx, ablib, numharm, zmax, wmax):
+    """The search's sums of a block (one and two columns a thread, tiles that overhang the block) are, bit for
+    bit, the planes of its harmonics added one after another by the per-function kernel."""
+    N = 1 << 17
+    fft = synth.spectrum(synth.time_series(N, 11 + zmax, [dict(r=9000.3, z=0.2 * zmax, harms=[(0.1, 0.0)] * 4)]))
+    obs = ablib.obs_init(ablib.make_params(N, DT, fft.size, zmax=zmax, wmax=wmax, numharm=numharm))
+    block = ablib.num_blocks(obs) // 2
+    got = ctx.block_stage_sums(obs, fft, block)
+    ctx.set_spectrum(obs, fft)
+    lo = obs.rlo + block * obs.rstep
+    hi = lo + obs.rstep - 0.5
+    meta, fund = ctx.subharm_fderivs_vol(obs, 1, 1, lo, hi)
+    np.testing.assert_array_equal(got[0], fund)
+    m, stage = 2, 1
+    while m <= numharm:
+        for h in range(1, m, 2):
+            smeta, sub = ctx.subharm_fderivs_vol(obs, m, h, lo, hi)
+            fund = ctx.add_ffdotpows(obs, meta, fund, smeta, sub, m, h, lo)
+        np.testing.assert_array_equal(got[stage], fund)
+        m, stage = 2 * m, stage + 1
