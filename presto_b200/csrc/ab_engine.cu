@@ -112,6 +112,7 @@ struct ab_ctx {
     DevBuf<float> dered_means;
     DevBuf<TcItem> titems;
     DevBuf<ab_bank> dbanks;
+    ab_bankset dbanks_host{};               // what dbanks holds (nbanks 0: nothing yet)
     DevBuf<double2> tw64;
     DevBuf<double2> tw_rzw;                 // exp(-2 pi i m / 2^RZW_NMAX_LOG2), jerk polishing
     DevBuf<double2> fresnel_tab;            // auxiliary Fresnel functions, acceleration polishing
@@ -128,6 +129,7 @@ struct ab_ctx {
     DevBuf<float> dbg;
     DevBuf<float> tmpa, tmpb;
     DevBuf<unsigned> errw;                   // device error word
+    bool err_armed = false;                  // the last call's kernels may have set it
 
     // hits: a ring of kHitSets sets, so that the device runs up to
     // kHitSets - 1 batches ahead of the host's replay (batches that hold a
@@ -356,8 +358,12 @@ static int ensure_banks(ab_ctx *ctx, const ab_obs *obs)
     ctx->cur_bank = hit;
     ctx->bs = nb;
     ctx->have_banks = true;
-    CK(cudaMemcpyAsync(ctx->dbanks.p, nb.b, sizeof(ab_bank) * nb.nbanks, cudaMemcpyHostToDevice,
-                       ctx->stream));
+    if (ctx->dbanks_host.nbanks != nb.nbanks ||
+        memcmp(ctx->dbanks_host.b, nb.b, sizeof(ab_bank) * (size_t) nb.nbanks)) {
+        CK(cudaMemcpyAsync(ctx->dbanks.p, nb.b, sizeof(ab_bank) * nb.nbanks, cudaMemcpyHostToDevice,
+                           ctx->stream));
+        ctx->dbanks_host = nb;
+    }
     return AB_OK;
 }
 
@@ -815,6 +821,19 @@ static int drain_hitset(ab_ctx *ctx, int i, Replayer *rp)
     return AB_OK;
 }
 
+// The device error word of a search or plane call, for the kernels with
+// bounded waits (the tensor-core correlation's); the others get none.
+static int clear_device_error(ab_ctx *ctx, SearchConsts &sc)
+{
+    sc.err = nullptr;
+    ctx->err_armed = ctx->corr_path != AB_CORR_FFT;
+    if (!ctx->err_armed) return AB_OK;
+    CK(ctx->errw.ensure(1));
+    CK(cudaMemsetAsync(ctx->errw.p, 0, sizeof(unsigned), ctx->stream));
+    sc.err = ctx->errw.p;
+    return AB_OK;
+}
+
 // Core search over main-loop blocks [first, first+count).  All hits are kept
 // in ctx->hkeys/hpows/hsigs; with list != NULL they are also replayed into
 // the candidate list, batch by batch while the device computes the next
@@ -825,9 +844,8 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
 {
     const ab_bankset &bs = ctx->bs;
     SearchConsts sc = make_consts(obs, bs);
-    CK(ctx->errw.ensure(1));
-    CK(cudaMemsetAsync(ctx->errw.p, 0, sizeof(unsigned), ctx->stream));
-    sc.err = ctx->errw.p;
+    int rc = clear_device_error(ctx, sc);
+    if (rc) return rc;
     long long nmain = ab_num_blocks(obs), npre = ab_num_preblocks(obs);
     if (first < 0) first = 0;
     if (count < 0 || first + count > nmain) count = nmain - first;
@@ -841,7 +859,7 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
     CK(ctx->startr.ensure(ctx->hstart.size()));
     CK(cudaMemcpyAsync(ctx->startr.p, ctx->hstart.data(), sizeof(double) * (nmain + npre),
                        cudaMemcpyHostToDevice, ctx->stream));
-    int rc = ensure_hitsets(ctx);
+    rc = ensure_hitsets(ctx);
     if (rc) return rc;
     ctx->hkeys.clear();
     ctx->hpows.clear();
@@ -1047,7 +1065,10 @@ static int fetch_hits(ab_ctx *ctx, long long *nhits)
 static int check_device_error(ab_ctx *ctx)
 {
     unsigned e = 0;
-    if (!ctx->errw.p) return AB_OK;
+    if (!ctx->err_armed) {                  // nothing waited: only drain the stream
+        CK(cudaStreamSynchronize(ctx->stream));
+        return AB_OK;
+    }
     CK(cudaMemcpyAsync(&e, ctx->errw.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (e) return fail(ctx, AB_ERR_CUDA, "device wait timed out (error word 0x%x)", e);
@@ -1899,9 +1920,7 @@ int ab_subharm_fderivs_vol(ab_ctx *ctx, const ab_obs *obs, int numharm, int harm
         return fail(ctx, AB_ERR_OVERFLOW, "plane needs %zu floats", need);
     SearchConsts sc = make_consts(obs, ctx->bs);
     sc.inmem = 0;                              // the block plane, not the full plane
-    CK(ctx->errw.ensure(1));
-    CK(cudaMemsetAsync(ctx->errw.p, 0, sizeof(unsigned), ctx->stream));
-    sc.err = ctx->errw.p;
+    if ((rc = clear_device_error(ctx, sc))) return rc;
     CK(ctx->startr.ensure(1));
     CK(cudaMemcpyAsync(ctx->startr.p, &fullrlo, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(ctx->planes.ensure((size_t) ctx->bs.plane_per_block));
@@ -1922,9 +1941,13 @@ int ab_subharm_fderivs_vol(ab_ctx *ctx, const ab_obs *obs, int numharm, int harm
         rc = run_corr(ctx, obs, sc, bb, &fullrlo, ctx->fft.p, k, k + 1, ctx->planes.p, ctx->bs.plane_per_block);
         if (rc) return rc;
     }
-    CK(cudaMemcpy2DAsync(out->powers, sizeof(float) * g.numrs, ctx->planes.p + b.plane_off,
-                         sizeof(float) * b.numrs_max, sizeof(float) * g.numrs, (size_t) b.nw * b.nz,
-                         cudaMemcpyDeviceToHost, ctx->stream));
+    if (g.numrs == b.numrs_max)
+        CK(cudaMemcpyAsync(out->powers, ctx->planes.p + b.plane_off, sizeof(float) * need, cudaMemcpyDeviceToHost,
+                           ctx->stream));
+    else
+        CK(cudaMemcpy2DAsync(out->powers, sizeof(float) * g.numrs, ctx->planes.p + b.plane_off,
+                             sizeof(float) * b.numrs_max, sizeof(float) * g.numrs, (size_t) b.nw * b.nz,
+                             cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     harvest(ctx);
     return check_device_error(ctx);
@@ -2221,6 +2244,7 @@ int ab_tc_gemm(ab_ctx *ctx, const float *A, const float *B, float *C, int N, int
     CK(b.ensure((size_t) N * K));
     CK(c.ensure((size_t) 128 * N));
     CK(ctx->errw.ensure(1));
+    ctx->err_armed = true;
     CK(cudaMemsetAsync(ctx->errw.p, 0, sizeof(unsigned), ctx->stream));
     CK(cudaMemcpyAsync(a.p, A, sizeof(float) * 128 * K, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b.p, B, sizeof(float) * N * K, cudaMemcpyHostToDevice, ctx->stream));

@@ -864,7 +864,9 @@ static int radix_sort_kv(unsigned long long *keys, unsigned long long *pl, long 
     }
     int bits = 0;
     while (bits < 64 && ((kmax - kmin) >> bits)) bits++;
-    int npasses = (bits + RS_MAXBITS - 1) / RS_MAXBITS;
+    /* a few keys: short digits (a pass clears and scans its 2^digit counts) */
+    const int maxbits = n < 4096 ? 8 : RS_MAXBITS;
+    int npasses = (bits + maxbits - 1) / maxbits;
     if (npasses == 0) return AB_OK;
     const int dbits = (bits + npasses - 1) / npasses;     /* equal digits, at most 14 bits */
     rs_ctx c;
@@ -1293,7 +1295,14 @@ int ab_replay_hits(const ab_obs *obs, unsigned long long *keys, float *pows, flo
     const size_t n = (size_t) nhits;
     /* pl, kb, ob (8 B), fsg, fnh, hcl (4 B), frr, fzz, fww (8 B), idx (8 B), added (1 B) */
     const size_t need = n * (8 * 3 + 4 * 3 + 8 * 3 + 8 + 1) + 64;
-    if (need > l->scr_cap) {
+    if (need > l->scr_cap && need < ((size_t) 1 << 20)) {
+        /* a small batch: a fresh huge page would cost its clearing, 0.4 ms */
+        void *p = malloc(2 * need);
+        if (!p) return AB_ERR_NOMEM;
+        free(l->scr);
+        l->scr = p;
+        l->scr_cap = 2 * need;
+    } else if (need > l->scr_cap) {
         /* 2 MiB-aligned and marked for huge pages: a batch of millions of
            crossings touches hundreds of MB once, and 4 KiB page faults on it
            would cost more than the replay */
