@@ -11,9 +11,9 @@
 // ones.  (Transforms over one block or a few whole ones spend a third to a
 // half of their length on overlap: all templates pay for the widest one's, and
 // block lengths do not fit the transform's.  zmax = 600 with 16 harmonics at
-// N = 2^23: 4.5 million transforms of 4096 points, 134 ms; now 22 million
-// pairs of 1024 points, 120 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
-// 225 ms.)  Each block keeps its own normalisation: a segment
+// N = 2^23: 12.5 million transforms of 4096 points, 134 ms; now 22 million
+// pairs of 1024 points, 119 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
+// 223 ms.)  Each block keeps its own normalisation: a segment
 // is transformed with its first block's and a column's powers are scaled by
 // its own block's over that, squared.
 //
@@ -34,6 +34,7 @@ namespace ab {
 constexpr int SEG_H = AB_SEG_BINS;          // bins of a segment's window
 constexpr int SEG_WARPS = 8;                // warps per CTA, two to a template
 constexpr int SEG_MAXBLK = 256;             // blocks that share one segment
+constexpr int SEG_TILE = AB_SEG_TILE;       // templates of a CTA at most
 constexpr int SEG_P = 34;                   // exchange row stride (points): 16-byte rows, no conflicts
 
 // ---------------------------------------------------------------------------
@@ -250,9 +251,10 @@ constexpr size_t SEG_SMEM = sizeof(float2) * (EX_OFF + SEG_WARPS * 32 * SEG_P);
 // shared memory and L1 data path 58 % busy, FP32 pipe 38 %, issue 47 %: held by
 // latencies at the 16 warps that 128 registers leave an SM.  Both transforms
 // of a template in one warp's paired FP32 instructions halve the issue but
-// leave 8 warps: 20 % slower.  Prefetching the next template into L1: 3 % slower;
+// leave 8 warps: 20 % slower.  Prefetching the next template into L1: 4 % slower;
 // loads and butterflies interleaved by hand, or one body for both passes: the
-// same.
+// same.  Segments of 2048 bins with 4096-point transforms by a whole CTA (radix
+// 16): 14.2 ns each, 16 % slower over the jerk search.
 __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
     k_corr_seg(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
                const SegCols *cols, const double *norms, const float2 *xhat, const float2 *tmpl,
@@ -262,8 +264,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
     __shared__ int4 s_blk[SEG_MAXBLK];          // first column, columns, offset, scale of a block here
     __shared__ int4 s_first[32];                // the first block of each group of 64 columns
     __shared__ unsigned char s_jlo[32], s_more[32];
-    __shared__ float *s_out;
-    __shared__ long long s_pitch;
+    __shared__ float *s_row[SEG_TILE];          // the templates' rows in the first block's plane
     __shared__ unsigned s_any;                  // bit k: group k of 64 columns has further blocks
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const SegGroup g = group_of_cta(groups, ngroups, blockIdx.x);
@@ -298,10 +299,9 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
         s_blk[j] = make_int4(lo, max(hi - lo, 0), (int) off,
                              __float_as_int((float) (r * r) * (1.0f / ((float) SEG_H * SEG_H))));
     }
-    if (threadIdx.x == 0) {
-        s_out = planes + (sc.inmem ? c[j0].c0 : (long long) (g.blk0 + j0) * plane_per_block + b.plane_off);
-        s_pitch = sc.inmem ? sc.rlen : b.numrs_max;
-    }
+    for (int i = threadIdx.x; i < g.tile && tile * g.tile + i < g.nt; i += blockDim.x)
+        s_row[i] = planes + (sc.inmem ? c[j0].c0 : (long long) (g.blk0 + j0) * plane_per_block + b.plane_off) +
+                   perm[g.t_lo + tile * g.tile + i] * (sc.inmem ? sc.rlen : (long long) b.numrs_max);
     __syncthreads();
     if (threadIdx.x < 32) {
         const int k0 = 64 * threadIdx.x;
@@ -325,12 +325,11 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
     float2 *ex = fsm + EX_OFF + warp * 32 * SEG_P;
     const float4 *ex4 = reinterpret_cast<const float4 *>(ex + lane * SEG_P);
     const int par = warp & 1;
-    const float4 *k0 = reinterpret_cast<const float4 *>(tmpl + b.seg_tmpl_off + par * SEG_H) + lane;
-    const int *tp = perm + g.t_lo + tile * g.tile + (warp >> 1);
-    const int *tend = perm + g.t_lo + min(g.nt, (tile + 1) * g.tile);
-    for (; tp < tend; tp += SEG_WARPS / 2) {
-        const int tl = *tp;
-        const float4 *kp = k0 + (long long) tl * SEG_H;
+    // (templates lie in the order of perm)
+    const int nt = min(g.nt - tile * g.tile, g.tile);
+    const float4 *kp = reinterpret_cast<const float4 *>(tmpl + b.seg_tmpl_off + par * SEG_H) + lane +
+                       (long long) (g.t_lo - b.perm_off + tile * g.tile + (warp >> 1)) * SEG_H;
+    for (int ti = warp >> 1; ti < nt; ti += SEG_WARPS / 2, kp += SEG_WARPS / 2 * SEG_H) {
         float2 v[32];
 #pragma unroll
         for (int p = 0; p < 16; p++) {
@@ -361,7 +360,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
         }
         __syncwarp();
         dft32(v);
-        float *row = s_out + tl * s_pitch;
+        float *row = s_row[ti];
 #pragma unroll
         for (int k = 0; k < 32; k++) {
             float2 &y = v[bin32(k)];

@@ -87,7 +87,7 @@ struct ab_ctx {
     };
     struct BankEntry {
         ab_bankset bs;
-        DevBuf<float2> tmpl;                // segment templates (ab_corr.cu), natural order
+        DevBuf<float2> tmpl;                // segment templates (ab_corr.cu), by class
         DevBuf<int> perm;                   // template indices, by class
         std::vector<SegClass> classes;      // bank-major, widest first
         unsigned long long used = 0;
@@ -339,7 +339,8 @@ static int ensure_banks(ab_ctx *ctx, const ab_obs *obs)
         CK(cudaStreamSynchronize(ctx->stream));       // perm is a host vector
         for (int i = 0; i < nb.nbanks; i++) {
             tick(ctx, 0, true);
-            cudaError_t e = launch_templates(&nb.b[i], 0, nb.b[i].ntmpl, 0,
+            cudaError_t e = launch_templates(&nb.b[i], perm.data() + nb.b[i].perm_off,
+                                             hit->perm.p + nb.b[i].perm_off, nb.b[i].ntmpl, 2 * AB_SEG_BINS,
                                              hit->tmpl.p + nb.b[i].seg_tmpl_off,
                                              ctx->tw64.p, kTwLog2, ctx->stream);
             tick(ctx, 0, false);
@@ -447,7 +448,7 @@ static SegPlan build_seg_plan(ab_ctx *ctx, const ab_obs *obs, const double *star
     // leaves six CTAs per SM, fewer for a small batch: one block's four planes at
     // zmax = 50 take 61 us in tiles of 8, 140 us in CTAs of 16 templates
     const long long per = work / (148 * 6) / 8 * 8;
-    const int tile = (int) std::max<long long>(8, std::min<long long>(64, per));
+    const int tile = (int) std::max<long long>(8, std::min<long long>(AB_SEG_TILE, per));
     for (SegGroup &g : out) {
         g.tile = tile;
         g.cta0 = p.nctas;
@@ -2195,7 +2196,7 @@ int ab_bank_kernel(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int
     if ((rc = ensure_tw64(ctx))) return rc;
     CK(ctx->resp.ensure((size_t) b.L));
     const int t = wi * b.nz + zi;
-    cudaError_t e = launch_templates(&b, t, t + 1, b.L, ctx->resp.p, ctx->tw64.p, kTwLog2, ctx->stream);
+    cudaError_t e = launch_templates(&b, &t, nullptr, 1, b.L, ctx->resp.p, ctx->tw64.p, kTwLog2, ctx->stream);
     if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "template generation failed: %s", cudaGetErrorString(e));
     ctx->launches++;
     CK(cudaMemcpyAsync(out, ctx->resp.p, sizeof(float2) * b.L, cudaMemcpyDeviceToHost, ctx->stream));

@@ -98,8 +98,8 @@ __device__ void store_seg_template(const double2 *placed, float2 *out)
 // out + t*L).  mode 1: raw response of numkern points into out.  mode 2:
 // raw response of bank template t (numkern = 4 halfwidth points) into
 // out + t*L, L being the row stride (taps of the tensor-core path).  mode 3:
-// bank template placed on L = 2048 columns, stored for ab_corr.cu into
-// out + 2 t AB_SEG_BINS.
+// bank template which[CTA], placed on L = 2048 columns, as ab_corr.cu reads it
+// into out + CTA * L.
 // Dynamic shared memory: (L + nfft_max) double2.
 struct TmplArgs {
     int mode, zmax, wmax, nz, L, t_base;
@@ -107,13 +107,14 @@ struct TmplArgs {
     int numbetween, numkern1;
     const double2 *tw;                // exp(-2 pi i m / NMAX), m < NMAX/2
     int nmax;
+    const int *which;                 // mode 3
     float2 *out;
 };
 
 __global__ void __launch_bounds__(256) k_templates(TmplArgs a)
 {
     extern __shared__ double2 dsm[];
-    int t = a.t_base + blockIdx.x;
+    int t = a.mode == 3 ? a.which[blockIdx.x] : a.t_base + blockIdx.x;
     double z, w;
     int numbetween, numkern;
     if (a.mode != 1) {
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(256) k_templates(TmplArgs a)
     if (place) {
         fft64_tab(placed, L, a.tw, a.nmax);
         if (a.mode == 3) {
-            store_seg_template(placed, a.out + (size_t) t * 2 * AB_SEG_BINS);
+            store_seg_template(placed, a.out + (size_t) blockIdx.x * L);
             return;
         }
         float2 *o = a.out + (size_t) t * L;
@@ -193,21 +194,19 @@ static int chirp_len(double z, double w, int numkern, int numbetween)
     return n * numbetween;
 }
 
-// Templates [t_lo, t_hi) of a bank.  L > 0: each as the transform of its taps
-// placed on L columns, out + (t - t_lo) L; L = 0: as ab_corr.cu reads them, out
-// + 2 AB_SEG_BINS t.
-cudaError_t launch_templates(const ab_bank *b, int t_lo, int t_hi, int L, float2 *out, const double2 *tw_all,
-                             int max_log2, cudaStream_t st)
+// n templates which[] of a bank (which_dev: the same on the device), as ab_corr.cu
+// reads them, one behind the other; or, which_dev null, the one template which[0]
+// as the transform of its taps placed on L columns.
+cudaError_t launch_templates(const ab_bank *b, const int *which, const int *which_dev, int n, int L, float2 *out,
+                             const double2 *tw_all, int max_log2, cudaStream_t st)
 {
-    const bool seg = L == 0;
-    if (seg) L = 2 * AB_SEG_BINS;
     int nfft_max = 0;
-    for (int t = t_lo; t < t_hi; t++) {
-        const double w = -b->wmax + t / b->nz * AB_DW, z = -b->zmax + t % b->nz * AB_DZ;
+    for (int i = 0; i < n; i++) {
+        const double w = -b->wmax + which[i] / b->nz * AB_DW, z = -b->zmax + which[i] % b->nz * AB_DZ;
         int nk = 2 * AB_NUMBETWEEN * ab_resp_halfwidth(z, w);
-        int n = chirp_len(z, w, nk, AB_NUMBETWEEN);
+        int nf = chirp_len(z, w, nk, AB_NUMBETWEEN);
         if (nk > L) return cudaErrorInvalidValue;
-        if (n > nfft_max) nfft_max = n;
+        if (nf > nfft_max) nfft_max = nf;
     }
     int nmax = 1 << max_log2;
     if (nfft_max > nmax || L > nmax) return cudaErrorInvalidValue;
@@ -215,19 +214,19 @@ cudaError_t launch_templates(const ab_bank *b, int t_lo, int t_hi, int L, float2
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
     cudaFuncSetAttribute(k_templates, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     TmplArgs a{};
-    a.mode = seg ? 3 : 0;
+    a.mode = which_dev ? 3 : 0;
     a.zmax = b->zmax;
     a.wmax = b->wmax;
     a.nz = b->nz;
     a.L = L;
     a.tw = tw_all;
     a.nmax = nmax;
-    a.out = seg ? out : out - (size_t) t_lo * L;
     const int chunk = 65535;
-    for (int t0 = t_lo; t0 < t_hi; t0 += chunk) {
-        a.t_base = t0;
-        int n = t_hi - t0 < chunk ? t_hi - t0 : chunk;
-        k_templates<<<n, 256, smem, st>>>(a);
+    for (int t0 = 0; t0 < n; t0 += chunk) {
+        a.which = which_dev ? which_dev + t0 : nullptr;
+        a.t_base = which[0];
+        a.out = which_dev ? out + (size_t) t0 * L : out - (size_t) which[0] * L;
+        k_templates<<<n - t0 < chunk ? n - t0 : chunk, 256, smem, st>>>(a);
     }
     return cudaGetLastError();
 }

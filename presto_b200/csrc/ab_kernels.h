@@ -29,6 +29,7 @@ struct BlockBatch {
     int npre0;                 // first of the pre-pass blocks (in-memory correlation), else nblk
 };
 
+constexpr int AB_SEG_TILE = 64;     // templates of one of its CTAs at most
 constexpr int AB_SEG_BINS = 1024;   // bins of a correlation segment's window (ab_corr.cu)
 
 // The units (segments) and CTAs of one bank's class of templates in a batch:
@@ -62,7 +63,7 @@ struct HitBuf {
 
 // kernel set (a): templates
 void launch_twiddle64(double2 *tw, int n, int sign, cudaStream_t st);
-cudaError_t launch_templates(const ab_bank *bank, int t_lo, int t_hi, int L, float2 *out,
+cudaError_t launch_templates(const ab_bank *bank, const int *which, const int *which_dev, int n, int L, float2 *out,
                              const double2 *tw_all, int max_log2, cudaStream_t st);
 cudaError_t launch_response(double roffset, int numbetween, double z, double w, int numkern,
                             float2 *out, const double2 *tw_chirp_all, int chirp_max_log2,
