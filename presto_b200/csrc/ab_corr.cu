@@ -12,8 +12,8 @@
 // half of their length on overlap: all templates pay for the widest one's, and
 // block lengths do not fit the transform's.  zmax = 600 with 16 harmonics at
 // N = 2^23: 12.5 million transforms of 4096 points, 134 ms; now 22 million
-// pairs of 1024 points, 119 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
-// 223 ms.)  Each block keeps its own normalisation: a segment
+// pairs of 1024 points, 107 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
+// 201 ms.)  Each block keeps its own normalisation: a segment
 // is transformed with its first block's and a column's powers are scaled by
 // its own block's over that, squared.
 //
@@ -247,14 +247,16 @@ constexpr size_t SEG_SMEM = sizeof(float2) * (EX_OFF + SEG_WARPS * 32 * SEG_P);
 // one exchange through the warp's own shared memory, radix 32 again -- no
 // barrier between warps and 8 bytes of exchange each way per point, where
 // radix 16 needs two exchanges behind CTA barriers at 4096 points.
-// Measured (B200, N = 2^20, zmax = 200): 5.4 to 5.7 ns per template and segment;
-// shared memory and L1 data path 58 % busy, FP32 pipe 38 %, issue 47 %: held by
-// latencies at the 16 warps that 128 registers leave an SM.  Both transforms
+// Measured (B200): 4.8 to 5.1 ns per template and segment (5.3 to 5.7 before the
+// powers were stored past L1, which they had swept of the templates, and with
+// half the templates to a CTA).  At that stage shared memory and L1 data path
+// were 58 % busy, the FP32 pipe 38 %, issue 47 %: held by latencies at the 16
+// warps that 128 registers leave an SM.  Both transforms
 // of a template in one warp's paired FP32 instructions halve the issue but
 // leave 8 warps: 20 % slower.  Prefetching the next template into L1: 4 % slower;
 // loads and butterflies interleaved by hand, or one body for both passes: the
 // same.  Segments of 2048 bins with 4096-point transforms by a whole CTA (radix
-// 16): 14.2 ns each, 16 % slower over the jerk search.
+// 16): 14.2 ns each, 16 % slower over the jerk search than this then was.
 __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
     k_corr_seg(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
                const SegCols *cols, const double *norms, const float2 *xhat, const float2 *tmpl,
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
             y.x = fmaf(y.x, y.x, y.y * y.y);
             const int col = 64 * k + 2 * lane + par;
             const int4 e = s_first[k];
-            if ((unsigned) (col - e.x) < (unsigned) e.y) row[e.z + col] = y.x * __int_as_float(e.w);
+            if ((unsigned) (col - e.x) < (unsigned) e.y) __stcs(row + (e.z + col), y.x * __int_as_float(e.w));
         }
         if (const unsigned more = s_any) {
 #pragma unroll
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
                 for (int j = s_jlo[k] + 1, n = s_more[k]; n > 0; n--, j++) {
                     const int4 f = s_blk[j];
                     if ((unsigned) (col - f.x) < (unsigned) f.y)
-                        row[f.z + col] = v[bin32(k)].x * __int_as_float(f.w);
+                        __stcs(row + (f.z + col), v[bin32(k)].x * __int_as_float(f.w));
                 }
             }
         }

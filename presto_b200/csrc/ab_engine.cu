@@ -444,8 +444,8 @@ static SegPlan build_seg_plan(ab_ctx *ctx, const ab_obs *obs, const double *star
             out.push_back(g);
         }
     }
-    // templates per CTA: 64 (the CTA's set-up is a template's work) while that
-    // leaves six CTAs per SM, fewer for a small batch: one block's four planes at
+    // templates per CTA: 128 (the CTA's set-up is a template's work; 64: 2 % slower
+    // over the jerk search) while that leaves six CTAs per SM, fewer for a small batch: one block's four planes at
     // zmax = 50 take 61 us in tiles of 8, 140 us in CTAs of 16 templates
     const long long per = work / (148 * 6) / 8 * 8;
     const int tile = (int) std::max<long long>(8, std::min<long long>(AB_SEG_TILE, per));

@@ -29,7 +29,7 @@ struct BlockBatch {
     int npre0;                 // first of the pre-pass blocks (in-memory correlation), else nblk
 };
 
-constexpr int AB_SEG_TILE = 64;     // templates of one of its CTAs at most
+constexpr int AB_SEG_TILE = 128;     // templates of one of its CTAs at most
 constexpr int AB_SEG_BINS = 1024;   // bins of a correlation segment's window (ab_corr.cu)
 
 // The units (segments) and CTAs of one bank's class of templates in a batch:
