@@ -33,14 +33,13 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # DRAM bytes moved per byte of f-fdot planes, from one ncu capture of each
-# kernel on the zmax=600 numharm=16 search at N=2^20 (one batch of 49 blocks,
-# 1.87 GB of planes): the 4096-point correlation launch read 0.17 GB and wrote
-# 1.81 GB for its 1.84 GB of planes (profiles/k_corr_4096_accelsearch_zmax600_
-# N2e20.md); the harmonic sum read 1.885 GB and wrote 0.005 GB for the batch's
-# 1.87 GB (profiles/k_harmsum_std5_accelsearch_zmax600_N2e20.md).  Both move
-# bytes in proportion to the planes, so full-size launches scale by their
-# plane bytes.
-CORR_DRAM_PER_PLANE_BYTE = (0.17 + 1.81) / 1.84
+# kernel at N=2^20: the correlation of the zmax=200 search read 0.031 GB and
+# wrote 0.799 GB for its plane of 0.843 GB (profiles/k_corr_seg_accelsearch_
+# zmax200_N2e20.md; the rest was still in L2); the harmonic sum of the zmax=600
+# numharm=16 search read 1.885 GB and wrote 0.005 GB for a batch's 1.87 GB
+# (profiles/k_harmsum_std5_accelsearch_zmax600_N2e20.md).  Both move bytes in
+# proportion to the planes, so full-size launches scale by their plane bytes.
+CORR_DRAM_PER_PLANE_BYTE = (0.031 + 0.799) / 0.843
 HARMSUM_DRAM_PER_PLANE_BYTE = (1.885 + 0.005) / 1.87
 
 WORKLOADS = {
@@ -413,11 +412,11 @@ def run_ours(args):
     else:
         achieved = counts["corr_flops"] / (corr_ms_per_search / 1e3) / 1e12
         fp32_peak = measured_fp32_peak(ctx)
-        roof = {"bound": "fp32", "kernel": "k_corr (template correlation)",
+        roof = {"bound": "fp32", "kernel": "k_corr_seg (template correlation)",
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak, "traffic": corr_traffic,
                 "traffic_unit": "DRAM bytes per launch (average over the search's correlation "
-                                "launches), scaled from profiles/k_corr_4096_accelsearch_zmax600"
+                                "launches), scaled from profiles/k_corr_seg_accelsearch_zmax200"
                                 "_N2e20.md by plane bytes" if corr_traffic else None,
                 "flops_per_search": counts["corr_flops"],
                 "kernel_ms_per_search": corr_ms_per_search,
