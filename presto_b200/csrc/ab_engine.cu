@@ -115,6 +115,9 @@ struct ab_ctx {
     ab_bankset dbanks_host{};               // what dbanks holds (nbanks 0: nothing yet)
     DevBuf<double2> tw64;
     DevBuf<double2> tw_rzw;                 // exp(-2 pi i m / 2^RZW_NMAX_LOG2), jerk polishing
+    RzwWork rzw_work;                       // jerk polishing scratch
+    DevBuf<PolishIn> pol_in;                // acceleration polishing: candidates and results
+    DevBuf<ab_polished> pol_out;
     DevBuf<double2> fresnel_tab;            // auxiliary Fresnel functions, acceleration polishing
     DevBuf<float2> resp;
 
@@ -1187,6 +1190,9 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->tw64.release();
     ctx->tw_rzw.release();
     ctx->fresnel_tab.release();
+    ctx->rzw_work.release();
+    ctx->pol_in.release();
+    ctx->pol_out.release();
     ctx->resp.release();
     ctx->fft.release();
     ctx->xhat.release();
@@ -1373,9 +1379,10 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
             while (c1 < n && (c1 == c0 || nh + cands[c1].numharm <= 4096)) nh += cands[c1++].numharm;
             rc = !obs->noharmpolish
                      ? rzw_optimize(dfft, obs->numbins, obs->lobin, cands + c0, c1 - c0, out + c0,
-                                    ctx->tw_rzw.p, budget, ctx->stream, msg, sizeof msg, &ctx->launches)
+                                    ctx->tw_rzw.p, budget, ctx->stream, ctx->rzw_work, msg, sizeof msg,
+                                    &ctx->launches)
                      : rzw_optimize_each(dfft, obs->numbins, obs->lobin, cands + c0, c1 - c0, out + c0,
-                                         ctx->tw_rzw.p, budget, ctx->stream, msg, sizeof msg,
+                                         ctx->tw_rzw.p, budget, ctx->stream, ctx->rzw_work, msg, sizeof msg,
                                          &ctx->launches);
             if (rc) return fail(ctx, rc, "%s", msg);
             c0 = c1;
@@ -1409,8 +1416,8 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
                            ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));           // tab is a host vector
     }
-    DevBuf<PolishIn> din;
-    DevBuf<ab_polished> dout;
+    DevBuf<PolishIn> &din = ctx->pol_in;
+    DevBuf<ab_polished> &dout = ctx->pol_out;
     cudaError_t e = din.ensure((size_t) nin);
     if (e == cudaSuccess) e = dout.ensure((size_t) nin);
     if (e == cudaSuccess)
@@ -1422,8 +1429,6 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hout, dout.p, sizeof(ab_polished) * nin, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    din.release();
-    dout.release();
     if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "candidate polishing failed: %s", cudaGetErrorString(e));
     if (each) {
         for (long long k = 0; k < n; k++) {

@@ -332,7 +332,7 @@ static int calc_fftlen(int numharm, int harmnum, int zmax, int wmax, const ab_ob
 /* Correlation cost per template and transform (ms), by log2 L, as installed
  * by ab_set_transform_costs (ab_autotune measures it).  The initial table is
  * k_corr measured on a B200 (1965 MHz): 512 to 4096 points.  Lengths whose
- * entry is <= 0 are not used for superblocks; an all-zero table falls back
+ * entry is <= 0 are not used for m > 1; an all-zero table falls back
  * to the radix-16 work L log2 L for lengths up to 4096.  (8192-point
  * transforms run one 512-thread CTA per SM; in whole searches on B200 they
  * cost more than their calibrated figure, so the initial table leaves them
@@ -443,7 +443,7 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
             free(nrs);
             return AB_ERR_ARG;
         }
-        /* Superblocks (standard search only): when the reference's own
+        /* What ab_bank_geometry reports beside L: when the reference's own
          * transform does not wrap into valid cells, m consecutive blocks can
          * share one device transform of length L2 over the first block's
          * window, provided the widest span of m consecutive blocks'

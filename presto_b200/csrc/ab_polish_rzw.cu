@@ -578,22 +578,6 @@ struct CandState {
     int d_idx[AB_POLISH_MAX_HARM][5];
 };
 
-struct DevMem {
-    void *p = nullptr;
-    size_t n = 0;
-    ~DevMem() { if (p) cudaFree(p); }
-    cudaError_t ensure(size_t bytes)
-    {
-        if (bytes <= n) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaMalloc(&p, bytes ? bytes : 1);
-        if (e == cudaSuccess) n = bytes;
-        return e;
-    }
-};
-
 // Runs the jobs of plan in chunks whose responses fit budget bytes; the
 // outputs land in out_amp (plan.outputs() entries).
 cudaError_t run_plan(Plan &plan, const float2 *data, const double2 *tw, size_t budget, DevMem &djobs,
@@ -645,7 +629,7 @@ double radian_phase(double re, double im)      // RADIAN_PHASE, include/presto.h
 
 int rzw_optimize(const float2 *data, long long numdata, long long lobin, const ab_cand *cands,
                  long long n, ab_polished *out, const double2 *tw, size_t budget, cudaStream_t st,
-                 char *err, size_t errlen, long long *launches)
+                 RzwWork &ws, char *err, size_t errlen, long long *launches)
 {
     // every output of the plan is indexed by int: bound the call's volume
     long long nharm = 0;
@@ -716,7 +700,7 @@ int rzw_optimize(const float2 *data, long long numdata, long long lobin, const a
         snprintf(err, errlen, "%s", pv.msg);
         return AB_ERR_ARG;
     }
-    DevMem djobs, dresp, dacc, dj, damp, dsmall;
+    DevMem &djobs = ws.jobs, &dresp = ws.resp, &dacc = ws.acc, &dj = ws.js, &damp = ws.amp, &dsmall = ws.small;
     cudaError_t e = run_plan(pv, data, tw, budget, djobs, dresp, dacc, dj, damp, st, launches);
     // stage 2: summed powers and the best cell (src/maximize_rzw.c:143-174)
     const size_t small = sizeof(int) * ((size_t) n * (3 + 2 * AB_POLISH_MAX_HARM));
@@ -831,7 +815,7 @@ namespace ab {
 // (src/accel_utils.c:585-597).
 int rzw_optimize_each(const float2 *data, long long numdata, long long lobin, const ab_cand *cands,
                       long long n, ab_polished *out, const double2 *tw, size_t budget,
-                      cudaStream_t st, char *err, size_t errlen, long long *launches)
+                      cudaStream_t st, RzwWork &ws, char *err, size_t errlen, long long *launches)
 {
     constexpr int numz = 2 * kInterpFac + 1, ncell = numz * numz * kNumR;
     struct Entry {
@@ -890,7 +874,7 @@ int rzw_optimize_each(const float2 *data, long long numdata, long long lobin, co
         snprintf(err, errlen, "%s", pv.msg);
         return AB_ERR_ARG;
     }
-    DevMem djobs, dresp, dacc, dj, damp, dsmall;
+    DevMem &djobs = ws.jobs, &dresp = ws.resp, &dacc = ws.acc, &dj = ws.js, &damp = ws.amp, &dsmall = ws.small;
     cudaError_t e = run_plan(pv, data, tw, budget, djobs, dresp, dacc, dj, damp, st, launches);
     std::vector<int> best((size_t) ne, 0);
     std::vector<float> bestval((size_t) ne, 0.0f);
