@@ -12,10 +12,12 @@
 // half of their length on overlap: all templates pay for the widest one's, and
 // block lengths do not fit the transform's.  zmax = 600 with 16 harmonics at
 // N = 2^23: 12.5 million transforms of 4096 points, 134 ms; now 22 million
-// pairs of 1024 points, 107 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
-// 201 ms.)  Each block keeps its own normalisation: a segment
+// pairs of 1024 points, 105 ms.  zmax = 200, wmax = 300 with 8 at 2^22: 317 and
+// 200 ms.)  Each block keeps its own normalisation: a segment
 // is transformed with its first block's and a column's powers are scaled by
-// its own block's over that, squared.
+// its own block's over that, squared.  Where blocks of one segment differ so
+// much that FP32 would carry one's values into another's cells (SEG_RANGE),
+// they are correlated one by one (k_corr_apart).
 //
 // Banks whose reference transform wraps into valid cells, and the local-power
 // normalisation (a factor per bin and block), need every block's own data:
@@ -36,6 +38,14 @@ constexpr int SEG_WARPS = 8;                // warps per CTA, two to a template
 constexpr int SEG_MAXBLK = 256;             // blocks that share one segment
 constexpr int SEG_TILE = AB_SEG_TILE;       // templates of a CTA at most
 constexpr int SEG_P = 34;                   // exchange row stride (points): 16-byte rows, no conflicts
+// What a segment over several blocks may hold: no bin brighter than this
+// against the normalisation of a block whose own window does not hold it, and
+// block normalisations within this factor of each other.  A bin of amplitude A
+// leaves FP32 rounding of some 3e-7 A / 32 in every column of its segment (its
+// power spreads over the transform): 1e-5 at 1024, below 1e-5 of any power
+// a search keeps.  Other segments are correlated block by block, each block's
+// data cut to its own window.
+constexpr float SEG_RANGE = 1024.0f;
 
 // ---------------------------------------------------------------------------
 // radix 32 in registers
@@ -107,13 +117,15 @@ __device__ __forceinline__ ab_hgeom seg_geom(const SearchConsts &sc, const ab_ba
 // with a value that is not finite, or a median of zero, makes every cell of
 // the block NaN in the block's own transform: its normalisation is NaN, and
 // the bad bins count as zero for the blocks beside it (k_seg_fwd), whose
-// windows do not hold them.  Blocks of banks correlated by their own data
-// get theirs from k_prep_time.
+// windows do not hold them.  Also the largest part of a value in the window
+// (SEG_RANGE).  Blocks of banks correlated by their own data get their
+// normalisation from k_prep_time.
 __global__ void __launch_bounds__(256) k_seg_cols(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
-                                                  const float2 *fft, SegCols *cols, double *norms)
+                                                  const float2 *fft, SegCols *cols, double *norms, int *apart)
 {
     extern __shared__ float spw[];
     __shared__ double s_norm;
+    __shared__ unsigned s_loud;
     const ab_bank b = banks[blockIdx.y];
     const int j = blockIdx.x;
     const ab_hgeom g = seg_geom(sc, b, bb.startr[j]);
@@ -121,22 +133,34 @@ __global__ void __launch_bounds__(256) k_seg_cols(const ab_bank *banks, SearchCo
     if (threadIdx.x == 0) {
         long long lim = sc.inmem ? g.numrs : min(g.numrs, b.numrs_max);
         if (sc.inmem && j >= bb.npre0) lim = min(lim, sc.clip_col - g.rlo * AB_RDR);
-        cols[at] = SegCols{g.rlo * AB_RDR, (int) max(lim, 0ll), 0};
+        cols[at].c0 = g.rlo * AB_RDR;
+        cols[at].lim = (int) max(lim, 0ll);
+        s_loud = 0u;
+        if (blockIdx.x == 0 && blockIdx.y == 0) apart[0] = 0;
     }
     if (b.own_data) return;
+    __syncthreads();
     const long long lobin = g.rlo - b.hw0;
     const int numdata = b.fftlen_ref / AB_NUMBETWEEN;
     bool bad = false;
+    float loud = 0.f;
     for (int i = threadIdx.x; i < numdata; i += blockDim.x) {
         const long long bin = lobin + i - sc.obs_lobin;
         if (bin >= 0 && bin < sc.numbins) {
             const float2 v = fft[bin];
-            bad |= !(isfinite(v.x) && isfinite(v.y));
+            if (isfinite(v.x) && isfinite(v.y)) loud = fmaxf(loud, fmaxf(fabsf(v.x), fabsf(v.y)));
+            else bad = true;
         }
     }
+    // (not negative: the bits order as the values do)
+    const unsigned lb = __reduce_max_sync(0xffffffffu, __float_as_uint(loud));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_loud, lb);
     bad = __syncthreads_or(bad);
     const double n = block_norm(sc, lobin, numdata, fft, spw, &s_norm);
-    if (threadIdx.x == 0) norms[at] = (bad || !isfinite(n)) ? (double) NAN : n;
+    if (threadIdx.x == 0) {
+        cols[at].loud = __uint_as_float(s_loud);
+        norms[at] = (bad || !isfinite(n)) ? (double) NAN : n;
+    }
 }
 
 __device__ __forceinline__ const SegGroup &group_of_unit(const SegGroup *g, int ng, int unit)
@@ -183,14 +207,92 @@ __device__ __forceinline__ double unit_norm(const double *nm, int j0, int n)
     return 1.0;
 }
 
-// Forward transforms of the units' windows, four per CTA.
+// Blocks of [j0, n) whose columns a unit of V columns from column q holds; all
+// lanes of a warp.
+__device__ __forceinline__ int unit_blocks(const SegCols *c, int j0, int n, long long q, int V)
+{
+    n = min(n, j0 + SEG_MAXBLK);
+    int nj = 1;
+    for (;;) {
+        const int j = j0 + nj + (int) (threadIdx.x & 31);
+        const unsigned in = __ballot_sync(0xffffffffu, j < n && c[j].c0 < q + V);
+        nj += __popc(in);
+        if (in != 0xffffffffu) return nj;
+    }
+}
+
+// Block j's own window, as points [lo, hi) of a segment whose window starts at bin0.
+__device__ __forceinline__ void block_window(const SearchConsts &sc, const ab_bank &b, const SegCols &c, long long bin0,
+                                             int &lo, int &hi)
+{
+    const long long a = c.c0 / 2 - b.hw0 - sc.obs_lobin, e = min(a + b.fftlen_ref / AB_NUMBETWEEN, sc.numbins);
+    lo = (int) min(max(max(a, 0ll) - bin0, 0ll), (long long) SEG_H);
+    hi = (int) max(min(e - bin0, (long long) SEG_H), 0ll);
+}
+
+// The points t + 64 m of a window (x: its point 0) times norm, zero outside
+// points [lo, hi) and where not finite.
+__device__ __forceinline__ void load_window(float2 (&v)[16], const float2 *x, int lo, int hi, int t, double norm)
+{
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const int k = t + FftShape<SEG_H>::NT * m;
+        v[m] = make_float2(0.f, 0.f);
+        if (k >= lo && k < hi) {
+            const float2 a = x[k];
+            if (isfinite(a.x) && isfinite(a.y))
+                v[m] = make_float2((float) ((double) a.x * norm), (float) ((double) a.y * norm));
+        }
+    }
+}
+
+// Whether blocks [j0, j0 + nj) of one unit are to be kept apart (SEG_RANGE), as
+// far as this warp's points of the window (k0, k0 + 64, ... below k1) tell.
+__device__ __forceinline__ bool keep_apart(const SearchConsts &sc, const ab_bank &b, const SegCols *c, const double *nm,
+                                           int j0, int nj, const float2 *x0, long long bin0, int k0, int k1)
+{
+    const int lane = threadIdx.x & 31;
+    float n = 0.f, i = 0.f, a = 0.f;            // largest norm, 1 / norm and part of a value
+    for (int j = j0 + lane; j < j0 + nj; j += 32) {
+        const double x = nm[j];
+        a = fmaxf(a, c[j].loud);
+        if (!(x > 0.0 && isfinite(x))) continue;
+        n = fmaxf(n, (float) x);
+        i = fmaxf(i, (float) (1.0 / x));
+    }
+    n = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(n)));
+    i = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(i)));
+    a = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(a)));
+    if (!(n * i <= SEG_RANGE)) return true;
+    if (n * a <= SEG_RANGE) return false;
+    // which values, against which blocks
+    bool far = false;
+    for (int j = j0; j < j0 + nj; j++) {
+        const double x = nm[j];
+        if (!(x > 0.0 && isfinite(x))) continue;
+        int lo, hi;
+        block_window(sc, b, c[j], bin0, lo, hi);
+        for (int k = k0; k < k1; k += FftShape<SEG_H>::NT) {
+            if ((k >= lo && k < hi) || bin0 + k < 0) continue;
+            const float2 v = x0[k];
+            far |= isfinite(v.x) && isfinite(v.y) && (double) fmaxf(fabsf(v.x), fabsf(v.y)) * x > (double) SEG_RANGE;
+        }
+    }
+    return __any_sync(0xffffffffu, far);
+}
+
+// Forward transforms of the units' windows, four per CTA, and what the
+// correlation needs to know of a unit.  apart: units whose blocks are kept
+// apart, apart[0] of them in any order from apart[1] on.
 __global__ void __launch_bounds__(256) k_seg_fwd(const ab_bank *banks, SearchConsts sc, BlockBatch bb,
                                                  const SegGroup *groups, int ngroups, int nunits,
                                                  const SegCols *cols, const double *norms, const float2 *fft,
-                                                 const float2 *dtime, long long dt_per_block, float2 *xhat)
+                                                 const float2 *dtime, long long dt_per_block, float2 *xhat,
+                                                 SegUnit *units, int *apart)
 {
     using SH = FftShape<SEG_H>;
     extern __shared__ float2 fsm[];
+    __shared__ int s_apart[SH::CTA / 32];
     const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
     const int unit = blockIdx.x * SH::G + grp;
     const bool ok = unit < nunits;
@@ -204,28 +306,31 @@ __global__ void __launch_bounds__(256) k_seg_fwd(const ab_bank *banks, SearchCon
         const float2 *d = dtime + j * dt_per_block + b.dtime_off;
 #pragma unroll
         for (int m = 0; m < 16; m++) v[m] = d[(off + t + SH::NT * m) % numdata];
+        if (t == 0 && ok) units[unit] = SegUnit{1.0, u / g.nsub, 1};
+        if (t == 0) s_apart[2 * grp] = s_apart[2 * grp + 1] = 0;
     } else {
         const SegCols *c = cols + (long long) g.bank * bb.nblk + g.blk0;
-        const long long q = c[0].c0 + (long long) u * g.V;
-        const int j0 = first_block(c, g.nblk, q);
-        const double norm = unit_norm(norms + (long long) g.bank * bb.nblk + g.blk0, j0, g.nblk);
-        const long long bin0 = q / 2 - g.hw - sc.obs_lobin;
-#pragma unroll
-        for (int m = 0; m < 16; m++) {
-            const long long bin = bin0 + t + SH::NT * m;
-            float2 x = make_float2(0.f, 0.f);
-            if (bin >= 0 && bin < sc.numbins) {
-                const float2 a = fft[bin];
-                if (isfinite(a.x) && isfinite(a.y))
-                    x = make_float2((float) ((double) a.x * norm), (float) ((double) a.y * norm));
-            }
-            v[m] = x;
-        }
+        const double *nm = norms + (long long) g.bank * bb.nblk + g.blk0;
+        const long long q = c[0].c0 + (long long) u * g.V, bin0 = q / 2 - g.hw - sc.obs_lobin;
+        const int j0 = first_block(c, g.nblk, q), nj = unit_blocks(c, j0, g.nblk, q, g.V);
+        const double norm = unit_norm(nm, j0, g.nblk);
+        // the windows of its blocks: nothing else is read
+        int lo, hi, lo1, hi0;
+        block_window(sc, b, c[j0], bin0, lo, hi0);
+        block_window(sc, b, c[j0 + nj - 1], bin0, lo1, hi);
+        const bool far = nj > 1 && keep_apart(sc, b, c, nm, j0, nj, fft + bin0, bin0, t, hi);
+        if ((t & 31) == 0) s_apart[threadIdx.x >> 5] = far;
+        if (t == 0 && ok) units[unit] = SegUnit{norm, j0, nj};
+        load_window(v, fft + bin0, lo, hi, t, norm);
     }
     FftTw<SEG_H, -1> tw;
     tw.init(t);
-    fft_run<SEG_H, -1>(v, fsm + grp * SH::SMEM, t, tw);
+    fft_run<SEG_H, -1>(v, fsm + grp * SH::SMEM, t, tw);     // (its barriers order s_apart)
     if (!ok) return;
+    if (t == 0 && (s_apart[2 * grp] | s_apart[2 * grp + 1])) {
+        units[unit].nj = -units[unit].nj;
+        apart[1 + atomicAdd(apart, 1)] = unit;
+    }
     float2 *o = xhat + (long long) unit * SEG_H;
 #pragma unroll
     for (int m = 0; m < 16; m++) {
@@ -240,6 +345,24 @@ __global__ void __launch_bounds__(256) k_seg_fwd(const ab_bank *banks, SearchCon
 constexpr int TW_OFF = SEG_H;                                   // float2
 constexpr int EX_OFF = 2 * SEG_H;
 constexpr size_t SEG_SMEM = sizeof(float2) * (EX_OFF + SEG_WARPS * 32 * SEG_P);
+
+struct SegMap {
+    int4 blk[SEG_MAXBLK];                       // first column, columns, offset, scale of a block here
+    int4 first[32];                             // the first block of each group of 64 columns
+    unsigned char jlo[32], more[32];
+    float *row[SEG_TILE];                       // the templates' rows in the first block's plane
+    unsigned any;                               // bit k: group k of 64 columns has further blocks
+};
+
+// exp(2 pi i l s / 1024) of lane l, bin s
+__device__ __forceinline__ void fill_twiddles(float2 *tw)
+{
+    for (int i = threadIdx.x; i < SEG_H; i += blockDim.x) {
+        double s, c;
+        sincospi((double) (((i & 31) * (i >> 5)) & (SEG_H - 1)) * (2.0 / SEG_H), &s, &c);
+        tw[seg_place(i)] = make_float2((float) c, (float) s);
+    }
+}
 
 // One CTA: one unit (segment) and a tile of its class's templates.  A warp
 // takes one of a template's two 1024-point inverse transforms (even or odd
@@ -257,69 +380,46 @@ constexpr size_t SEG_SMEM = sizeof(float2) * (EX_OFF + SEG_WARPS * 32 * SEG_P);
 // loads and butterflies interleaved by hand, or one body for both passes: the
 // same.  Segments of 2048 bins with 4096-point transforms by a whole CTA (radix
 // 16): 14.2 ns each, 16 % slower over the jerk search than this then was.
-__global__ void __launch_bounds__(32 * SEG_WARPS, 2)
-    k_corr_seg(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
-               const SegCols *cols, const double *norms, const float2 *xhat, const float2 *tmpl,
-               const int *perm, float *planes, long long plane_per_block)
+// The blocks of a unit are looked up once, by k_seg_fwd, and not by each of its
+// CTAs: 107.4 -> 105.0 ms and 201.9 -> 199.6 (the two searches above).
+//
+// Here: tile `tile` of the group's templates against the data spectrum in fsm,
+// normalised with ref, whose columns from q belong to nj blocks (c and nm: the
+// first one's; blk0: its index in the batch).  All threads of the CTA.
+__device__ __forceinline__ void corr_tile(const SegGroup &g, const ab_bank &b, const SearchConsts &sc, const SegCols *c,
+                                          const double *nm, int blk0, int nj, long long q, double ref, int tile,
+                                          const float2 *tmpl, const int *perm, float *planes,
+                                          long long plane_per_block, float2 *fsm, SegMap &m)
 {
-    extern __shared__ __align__(16) float2 fsm[];
-    __shared__ int4 s_blk[SEG_MAXBLK];          // first column, columns, offset, scale of a block here
-    __shared__ int4 s_first[32];                // the first block of each group of 64 columns
-    __shared__ unsigned char s_jlo[32], s_more[32];
-    __shared__ float *s_row[SEG_TILE];          // the templates' rows in the first block's plane
-    __shared__ unsigned s_any;                  // bit k: group k of 64 columns has further blocks
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const SegGroup g = group_of_cta(groups, ngroups, blockIdx.x);
-    const int r0 = blockIdx.x - g.cta0, u = r0 % g.nunits, tile = r0 / g.nunits;
-    const ab_bank b = banks[g.bank];
-    {
-        const float4 *src = reinterpret_cast<const float4 *>(xhat + (long long) (g.unit0 + u) * SEG_H);
-        float4 *dst = reinterpret_cast<float4 *>(fsm);
-        for (int i = threadIdx.x; i < SEG_H / 2; i += blockDim.x) dst[i] = src[i];
-        // twiddles exp(2 pi i l s / 1024) of lane l, bin s
-        for (int i = threadIdx.x; i < SEG_H; i += blockDim.x) {
-            double s, c;
-            sincospi((double) (((i & 31) * (i >> 5)) & (SEG_H - 1)) * (2.0 / SEG_H), &s, &c);
-            fsm[TW_OFF + seg_place(i)] = make_float2((float) c, (float) s);
-        }
-    }
-    // the blocks whose columns this unit holds, in transform columns
-    const SegCols *c = cols + (long long) g.bank * bb.nblk + g.blk0;
-    const double *nm = norms + (long long) g.bank * bb.nblk + g.blk0;
-    const int j0 = g.nsub ? u / g.nsub : first_block(c, g.nblk, c[0].c0 + (long long) u * g.V);
-    const long long q = g.nsub ? c[j0].c0 + (long long) (u % g.nsub) * g.V : c[0].c0 + (long long) u * g.V;
-    int nj = 1;
-    if (!g.nsub)
-        while (nj < SEG_MAXBLK && j0 + nj < g.nblk && c[j0 + nj].c0 < q + g.V) nj++;
-    const double ref = g.nsub ? 1.0 : unit_norm(nm, j0, g.nblk);
     for (int j = threadIdx.x; j < nj; j += blockDim.x) {
-        const int tc0 = (int) (c[j0 + j].c0 - q) + 2 * g.hw;
-        const int lo = max(tc0, 2 * g.hw), hi = min(tc0 + c[j0 + j].lim, 2 * g.hw + g.V);
+        const int tc0 = (int) (c[j].c0 - q) + 2 * g.hw;
+        const int lo = max(tc0, 2 * g.hw), hi = min(tc0 + c[j].lim, 2 * g.hw + g.V);
         // element of this block's transform column 0, from the first block's
-        const long long off = sc.inmem ? c[j0 + j].c0 - c[j0].c0 - tc0 : (long long) j * plane_per_block - tc0;
-        const double r = nm[j0 + j] / ref;
-        s_blk[j] = make_int4(lo, max(hi - lo, 0), (int) off,
+        const long long off = sc.inmem ? c[j].c0 - c[0].c0 - tc0 : (long long) j * plane_per_block - tc0;
+        const double r = nm[j] / ref;
+        m.blk[j] = make_int4(lo, max(hi - lo, 0), (int) off,
                              __float_as_int((float) (r * r) * (1.0f / ((float) SEG_H * SEG_H))));
     }
     for (int i = threadIdx.x; i < g.tile && tile * g.tile + i < g.nt; i += blockDim.x)
-        s_row[i] = planes + (sc.inmem ? c[j0].c0 : (long long) (g.blk0 + j0) * plane_per_block + b.plane_off) +
+        m.row[i] = planes + (sc.inmem ? c[0].c0 : (long long) blk0 * plane_per_block + b.plane_off) +
                    perm[g.t_lo + tile * g.tile + i] * (sc.inmem ? sc.rlen : (long long) b.numrs_max);
     __syncthreads();
     if (threadIdx.x < 32) {
         const int k0 = 64 * threadIdx.x;
         int a = 0, n = 0;
         for (int j = 0; j < nj; j++) {
-            const int4 e = s_blk[j];
+            const int4 e = m.blk[j];
             if (e.y > 0 && e.x < k0 + 64 && e.x + e.y > k0) {
                 if (n == 0) a = j;
                 n = j - a + 1;
             }
         }
-        s_first[threadIdx.x] = n ? s_blk[a] : make_int4(0, 0, 0, 0);
-        s_jlo[threadIdx.x] = (unsigned char) a;
-        s_more[threadIdx.x] = (unsigned char) (n > 1 ? n - 1 : 0);
+        m.first[threadIdx.x] = n ? m.blk[a] : make_int4(0, 0, 0, 0);
+        m.jlo[threadIdx.x] = (unsigned char) a;
+        m.more[threadIdx.x] = (unsigned char) (n > 1 ? n - 1 : 0);
         const unsigned any = __ballot_sync(0xffffffffu, n > 1);
-        if (threadIdx.x == 0) s_any = any;
+        if (threadIdx.x == 0) m.any = any;
     }
     __syncthreads();
     const float4 *xs = reinterpret_cast<const float4 *>(fsm) + lane;
@@ -362,22 +462,22 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
         }
         __syncwarp();
         dft32(v);
-        float *row = s_row[ti];
+        float *row = m.row[ti];
 #pragma unroll
         for (int k = 0; k < 32; k++) {
             float2 &y = v[bin32(k)];
             y.x = fmaf(y.x, y.x, y.y * y.y);
             const int col = 64 * k + 2 * lane + par;
-            const int4 e = s_first[k];
+            const int4 e = m.first[k];
             if ((unsigned) (col - e.x) < (unsigned) e.y) __stcs(row + (e.z + col), y.x * __int_as_float(e.w));
         }
-        if (const unsigned more = s_any) {
+        if (const unsigned more = m.any) {
 #pragma unroll
             for (int k = 0; k < 32; k++) {
                 if (!((more >> k) & 1u)) continue;
                 const int col = 64 * k + 2 * lane + par;
-                for (int j = s_jlo[k] + 1, n = s_more[k]; n > 0; n--, j++) {
-                    const int4 f = s_blk[j];
+                for (int j = m.jlo[k] + 1, n = m.more[k]; n > 0; n--, j++) {
+                    const int4 f = m.blk[j];
                     if ((unsigned) (col - f.x) < (unsigned) f.y)
                         __stcs(row + (f.z + col), v[bin32(k)].x * __int_as_float(f.w));
                 }
@@ -386,37 +486,128 @@ __global__ void __launch_bounds__(32 * SEG_WARPS, 2)
     }
 }
 
+__global__ void __launch_bounds__(32 * SEG_WARPS, 2)
+    k_corr_seg(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
+               const SegCols *cols, const double *norms, const float2 *xhat, const float2 *tmpl,
+               const int *perm, const SegUnit *units, float *planes, long long plane_per_block)
+{
+    extern __shared__ __align__(16) float2 fsm[];
+    __shared__ SegMap s_map;
+    const SegGroup g = group_of_cta(groups, ngroups, blockIdx.x);
+    const int r0 = blockIdx.x - g.cta0, u = r0 % g.nunits, tile = r0 / g.nunits;
+    const SegUnit w = units[g.unit0 + u];
+    if (w.nj < 0) return;                       // k_corr_apart's
+    const ab_bank b = banks[g.bank];
+    {
+        const float4 *src = reinterpret_cast<const float4 *>(xhat + (long long) (g.unit0 + u) * SEG_H);
+        float4 *dst = reinterpret_cast<float4 *>(fsm);
+        for (int i = threadIdx.x; i < SEG_H / 2; i += blockDim.x) dst[i] = src[i];
+        fill_twiddles(fsm + TW_OFF);
+    }
+    const long long at = (long long) g.bank * bb.nblk + g.blk0;
+    const SegCols *c = cols + at;
+    const long long q = g.nsub ? c[w.j0].c0 + (long long) (u % g.nsub) * g.V : c[0].c0 + (long long) u * g.V;
+    corr_tile(g, b, sc, c + w.j0, norms + at + w.j0, g.blk0 + w.j0, w.nj, q, w.norm, tile, tmpl, perm, planes,
+              plane_per_block, fsm, s_map);
+}
+
+// The units whose blocks are kept apart (SEG_RANGE), one block and tile of
+// templates at a time: the block's data cut to its own window, transformed
+// here.  One CTA per SM shares the list, which is all but always empty.
+__global__ void __launch_bounds__(32 * SEG_WARPS, 1)
+    k_corr_apart(const ab_bank *banks, SearchConsts sc, BlockBatch bb, const SegGroup *groups, int ngroups,
+                 const SegCols *cols, const double *norms, const float2 *fft, const float2 *tmpl, const int *perm,
+                 const SegUnit *units, const int *apart, float *planes, long long plane_per_block)
+{
+    using SH = FftShape<SEG_H>;
+    extern __shared__ __align__(16) float2 fsm[];
+    __shared__ SegMap s_map;
+    const int n = apart[0];
+    if (n == 0) return;
+    fill_twiddles(fsm + TW_OFF);
+    long long base = 0;                         // items of the units before this one
+    for (int i = 0; i < n; i++) {
+        const int unit = apart[1 + i];
+        const SegGroup g = group_of_unit(groups, ngroups, unit);
+        const SegUnit w = units[unit];
+        const ab_bank b = banks[g.bank];
+        const long long at = (long long) g.bank * bb.nblk + g.blk0;
+        const long long q = cols[at].c0 + (long long) (unit - g.unit0) * g.V;
+        const long long bin0 = q / 2 - g.hw - sc.obs_lobin;
+        const int ntile = (g.nt + g.tile - 1) / g.tile, items = -w.nj * ntile;
+        for (int k = (int) ((blockIdx.x + gridDim.x - base % gridDim.x) % gridDim.x); k < items; k += (int) gridDim.x) {
+            const int j = w.j0 + k / ntile, tile = k % ntile;
+            const SegCols *c = cols + at + j;
+            const double *nm = norms + at + j;
+            const double ref = unit_norm(nm, 0, 1);
+            __syncthreads();                    // every warp has done with the last item
+            {
+                const int grp = threadIdx.x / SH::NT, t = threadIdx.x - grp * SH::NT;
+                int lo, hi;
+                block_window(sc, b, *c, bin0, lo, hi);
+                float2 v[16];
+                load_window(v, fft + bin0, lo, hi, t, ref);
+                FftTw<SEG_H, -1> tw;
+                tw.init(t);
+                fft_run<SEG_H, -1>(v, fsm + EX_OFF + grp * SH::SMEM, t, tw);
+                if (grp == 0) {                 // (the other groups did the same)
+#pragma unroll
+                    for (int m = 0; m < 16; m++) fsm[seg_place(t + SH::NT * m)] = v[m];
+                }
+            }
+            corr_tile(g, b, sc, c, nm, g.blk0 + j, 1, q, ref, tile, tmpl, perm, planes, plane_per_block, fsm, s_map);
+        }
+        base += items;
+    }
+}
+
 cudaError_t launch_seg_cols(const ab_bank *banks_dev, int nbanks, const SearchConsts &sc, const BlockBatch &bb,
-                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, cudaStream_t st)
+                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, int *apart, cudaStream_t st)
 {
     const size_t smem = sizeof(float) * (size_t) numdata_max;
     if (smem > 48 * 1024) return cudaErrorInvalidValue;
-    k_seg_cols<<<dim3((unsigned) bb.nblk, (unsigned) nbanks), 256, smem, st>>>(banks_dev, sc, bb, fft, cols, norms);
+    k_seg_cols<<<dim3((unsigned) bb.nblk, (unsigned) nbanks), 256, smem, st>>>(banks_dev, sc, bb, fft, cols, norms, apart);
     return cudaGetLastError();
 }
 
 cudaError_t launch_seg_fwd(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
                            const SegGroup *groups, int ngroups, int nunits, const SegCols *cols,
                            const double *norms, const float2 *fft, const float2 *dtime, long long dt_per_block,
-                           float2 *xhat, cudaStream_t st)
+                           float2 *xhat, SegUnit *units, int *apart, cudaStream_t st)
 {
     using SH = FftShape<SEG_H>;
     if (nunits <= 0) return cudaSuccess;
     k_seg_fwd<<<(unsigned) ((nunits + SH::G - 1) / SH::G), SH::CTA, (size_t) SH::G * SH::SMEM * sizeof(float2), st>>>(
-        banks_dev, sc, bb, groups, ngroups, nunits, cols, norms, fft, dtime, dt_per_block, xhat);
+        banks_dev, sc, bb, groups, ngroups, nunits, cols, norms, fft, dtime, dt_per_block, xhat, units, apart);
     return cudaGetLastError();
 }
 
 cudaError_t launch_corr_seg(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
                             const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
                             const double *norms, const float2 *xhat, const float2 *tmpl, const int *perm,
-                            float *planes, long long plane_per_block, cudaStream_t st)
+                            const SegUnit *units, float *planes, long long plane_per_block, cudaStream_t st)
 {
     if (nctas <= 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(k_corr_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SEG_SMEM);
     if (e != cudaSuccess) return e;
     k_corr_seg<<<(unsigned) nctas, 32 * SEG_WARPS, SEG_SMEM, st>>>(banks_dev, sc, bb, groups, ngroups, cols, norms,
-                                                                  xhat, tmpl, perm, planes, plane_per_block);
+                                                                  xhat, tmpl, perm, units, planes, plane_per_block);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_corr_apart(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                              const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
+                              const double *norms, const float2 *fft, const float2 *tmpl, const int *perm,
+                              const SegUnit *units, const int *apart, float *planes, long long plane_per_block,
+                              cudaStream_t st)
+{
+    if (nctas <= 0) return cudaSuccess;
+    static_assert(4 * FftShape<SEG_H>::SMEM <= SEG_WARPS * 32 * SEG_P, "the transforms' exchange");
+    cudaError_t e = cudaFuncSetAttribute(k_corr_apart, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SEG_SMEM);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = (unsigned) (nctas < 148 ? nctas : 148);
+    k_corr_apart<<<grid, 32 * SEG_WARPS, SEG_SMEM, st>>>(banks_dev, sc, bb, groups, ngroups, cols, norms, fft, tmpl,
+                                                        perm, units, apart, planes, plane_per_block);
     return cudaGetLastError();
 }
 

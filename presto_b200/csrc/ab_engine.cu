@@ -105,6 +105,8 @@ struct ab_ctx {
     DevBuf<SegGroup> seg_groups;            // correlation segments: groups, columns, normalisations
     DevBuf<SegCols> seg_cols;
     DevBuf<double> seg_norms;
+    DevBuf<SegUnit> seg_units;
+    DevBuf<int> seg_apart;                  // units whose blocks are kept apart
     std::vector<SegGroup> hgroups;
     DevBuf<int> dd_cd, dd_off;              // dedispersion delays
     long long blu_M = 0;                    // the length blu_b was built for
@@ -402,7 +404,7 @@ static SearchConsts make_consts(const ab_obs *obs, const ab_bankset &bs)
 // start is their start frequencies.  Group bank indices count from bank_lo.
 struct SegPlan {
     int nunits = 0, nctas = 0;
-    bool own_data = false;
+    bool own_data = false, shared = false;  // banks with blocks' own data, segments over several blocks
     int numdata_max = 0;
 };
 
@@ -430,6 +432,8 @@ static SegPlan build_seg_plan(ab_ctx *ctx, const ab_obs *obs, const double *star
             g.blk0 = blk0;
             g.nblk = n;
             g.unit0 = p.nunits;
+            // (segments as long as the fundamental's blocks lie on them)
+            p.shared |= !b.own_data && n > 1 && !(b.numharm == 1 && g.V == obs->corr_uselen);
             if (b.own_data) {
                 g.nsub = (b.numrs_max + g.V - 1) / g.V;
                 g.nunits = g.nsub * n;
@@ -474,6 +478,8 @@ static int run_corr(ab_ctx *ctx, const ab_obs *obs, const SearchConsts &sc, cons
     CK(ctx->seg_cols.ensure((size_t) nbanks * bb.nblk));
     CK(ctx->seg_norms.ensure((size_t) nbanks * bb.nblk));
     CK(ctx->xhat.ensure((size_t) p.nunits * AB_SEG_BINS));
+    CK(ctx->seg_units.ensure((size_t) p.nunits));
+    CK(ctx->seg_apart.ensure((size_t) p.nunits + 1));
     if (p.own_data) CK(ctx->dtime.ensure((size_t) bb.nblk * bs.dtime_per_block));
     CK(cudaMemcpyAsync(ctx->seg_groups.p, ctx->hgroups.data(), sizeof(SegGroup) * ctx->hgroups.size(),
                        cudaMemcpyHostToDevice, ctx->stream));
@@ -481,7 +487,7 @@ static int run_corr(ab_ctx *ctx, const ab_obs *obs, const SearchConsts &sc, cons
     const int ng = (int) ctx->hgroups.size();
     tick(ctx, 1, true);
     cudaError_t e = launch_seg_cols(db, nbanks, sc, bb, fft, p.numdata_max, ctx->seg_cols.p, ctx->seg_norms.p,
-                                    ctx->stream);
+                                    ctx->seg_apart.p, ctx->stream);
     ctx->launches++;
     for (int k = bank_lo; k < bank_hi && e == cudaSuccess && p.own_data; k++) {
         if (!bs.b[k].own_data) continue;
@@ -491,15 +497,23 @@ static int run_corr(ab_ctx *ctx, const ab_obs *obs, const SearchConsts &sc, cons
     }
     if (e == cudaSuccess)
         e = launch_seg_fwd(db, sc, bb, ctx->seg_groups.p, ng, p.nunits, ctx->seg_cols.p, ctx->seg_norms.p, fft,
-                           ctx->dtime.p, bs.dtime_per_block, ctx->xhat.p, ctx->stream);
+                           ctx->dtime.p, bs.dtime_per_block, ctx->xhat.p, ctx->seg_units.p,
+                           ctx->seg_apart.p, ctx->stream);
     tick(ctx, 1, false);
     if (e != cudaSuccess)
         return fail(ctx, AB_ERR_CUDA, "data preparation failed: %s", cudaGetErrorString(e));
     tick(ctx, 2, true);
     e = launch_corr_seg(db, sc, bb, ctx->seg_groups.p, ng, p.nctas, ctx->seg_cols.p, ctx->seg_norms.p,
-                        ctx->xhat.p, ctx->cur_bank->tmpl.p, ctx->cur_bank->perm.p, planes, ppb, ctx->stream);
-    tick(ctx, 2, false);
+                        ctx->xhat.p, ctx->cur_bank->tmpl.p, ctx->cur_bank->perm.p, ctx->seg_units.p, planes, ppb,
+                        ctx->stream);
     ctx->launches += 2;
+    if (e == cudaSuccess && p.shared) {
+        e = launch_corr_apart(db, sc, bb, ctx->seg_groups.p, ng, p.nctas, ctx->seg_cols.p, ctx->seg_norms.p, fft,
+                              ctx->cur_bank->tmpl.p, ctx->cur_bank->perm.p, ctx->seg_units.p, ctx->seg_apart.p,
+                              planes, ppb, ctx->stream);
+        ctx->launches++;
+    }
+    tick(ctx, 2, false);
     if (e != cudaSuccess)
         return fail(ctx, AB_ERR_CUDA, "correlation launch failed: %s", cudaGetErrorString(e));
     return AB_OK;
@@ -1216,6 +1230,8 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->seg_groups.release();
     ctx->seg_cols.release();
     ctx->seg_norms.release();
+    ctx->seg_units.release();
+    ctx->seg_apart.release();
     ctx->dd_cd.release();
     ctx->dd_off.release();
     ctx->dered_runs.release();

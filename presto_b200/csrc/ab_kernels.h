@@ -45,7 +45,14 @@ struct SegGroup {
 
 struct SegCols {               // a block's columns in a bank's plane
     long long c0;              // first, absolute (2 rlo)
-    int lim, pad;              // columns to fill
+    int lim;                   // columns to fill
+    float loud;                // largest part of a value in its window
+};
+
+struct SegUnit {
+    double norm;               // what its data are normalised with
+    int j0, nj;                // the blocks whose columns it holds, from the group's first;
+                               // nj < 0: -nj blocks, correlated one by one
 };
 
 struct CorrItem {              // one CTA of the correlation kernel
@@ -73,17 +80,23 @@ cudaError_t launch_response(double roffset, int numbetween, double z, double w, 
 
 // kernel set (b): correlation of the searches and plane calls.  cols and norms:
 // [bank][block] of the nbanks banks from banks_dev on (group bank indices count
-// from there); planes of the standard mode, or the in-memory plane (sc.inmem)
+// from there); planes of the standard mode, or the in-memory plane (sc.inmem);
+// apart: room for nunits + 1
 cudaError_t launch_seg_cols(const ab_bank *banks_dev, int nbanks, const SearchConsts &sc, const BlockBatch &bb,
-                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, cudaStream_t st);
+                            const float2 *fft, int numdata_max, SegCols *cols, double *norms, int *apart, cudaStream_t st);
 cudaError_t launch_seg_fwd(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
                            const SegGroup *groups, int ngroups, int nunits, const SegCols *cols,
                            const double *norms, const float2 *fft, const float2 *dtime, long long dt_per_block,
-                           float2 *xhat, cudaStream_t st);
+                           float2 *xhat, SegUnit *units, int *apart, cudaStream_t st);
 cudaError_t launch_corr_seg(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
                             const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
                             const double *norms, const float2 *xhat, const float2 *tmpl, const int *perm,
-                            float *planes, long long plane_per_block, cudaStream_t st);
+                            const SegUnit *units, float *planes, long long plane_per_block, cudaStream_t st);
+cudaError_t launch_corr_apart(const ab_bank *banks_dev, const SearchConsts &sc, const BlockBatch &bb,
+                              const SegGroup *groups, int ngroups, int nctas, const SegCols *cols,
+                              const double *norms, const float2 *fft, const float2 *tmpl, const int *perm,
+                              const SegUnit *units, const int *apart, float *planes, long long plane_per_block,
+                              cudaStream_t st);
 
 // one block and bank with caller-held templates (ab_fderivs_vol_noalloc)
 cudaError_t launch_prep(const ab_bank *bank_dev, const ab_bank &b, const SearchConsts &sc, const BlockBatch &bb,

@@ -109,3 +109,82 @@ def test_stage_sums_are_the_per_function_sums(ctx, ablib, numharm, zmax, wmax):
             fund = ctx.add_ffdotpows(obs, meta, fund, smeta, sub, m, h, lo)
         np.testing.assert_array_equal(got[stage], fund)
         m, stage = 2 * m, stage + 1
+
+
+def _hit_arrays(ctx, obs, fft, first=0, count=-1):
+    ctx.search(obs, fft, first_block=first, max_blocks=count)
+    blk, st, wi, zi, ri, pw = (np.asarray(a) for a in ctx.last_hits())
+    key = (((blk.astype(np.int64) * 8 + st) * 128 + wi) * 4096 + zi) * 65536 + ri
+    order = np.argsort(key)
+    return key[order], blk[order], st[order], np.asarray(pw, np.float64)[order]
+
+
+LOUD = [("quiet", 1e-17), ("quiet", 1e-6), ("bright", 1e6), ("bright", 1e8), ("bright", 3e18)]
+PLACES = (20011, 40000, 77777, 100500)
+
+
+def _loud(what, value, pulsars, places=PLACES):
+    """A spectrum with stretches that are quieter than the rest by a large factor or bins that are far brighter
+    (bin 0 too: a series that was not de-reddened), and the bins that were changed."""
+    fft = synth.spectrum(synth.time_series(1 << 18, 5, pulsars)).astype(np.complex64)
+    changed = np.zeros(fft.size, bool)
+    for a in places if what == "quiet" else (0, *places):
+        b = a + (1600 if what == "quiet" else 1)
+        fft[a:b] = fft[a:b] * np.float32(value) if what == "quiet" else value
+        changed[a:b] = True
+    return fft, changed
+
+
+def _clean_blocks(obs, changed, banks):
+    """The blocks none of whose windows (of any bank) holds a changed bin."""
+    import presto_b200 as pb
+    out = []
+    for b in range(pb.num_blocks(obs)):
+        for g in banks:
+            lo = int((obs.rlo + b * obs.rstep) * g["harmnum"] / g["numharm"]) - g["hw"] - 2
+            if np.any(changed[max(lo, 0):lo + g["fftlen_ref"] // 2 + 4]):
+                break
+        else:
+            out.append(b)
+    return out
+
+
+@pytest.mark.parametrize("what,value", LOUD)
+@pytest.mark.parametrize("zmax,wmax,numharm", [(0, 0, 32), (50, 0, 16), (50, 0, 1), (20, 20, 4)])
+def test_loud_and_quiet_blocks_keep_to_themselves(ctx, ablib, what, value, zmax, wmax, numharm):
+    """A segment over several blocks would carry loud bins' rounding, or a scale that overflows, into blocks whose
+    own windows do not hold them.  The crossings of such blocks are those of a search of the block alone, whose
+    windows hold nothing loud."""
+    fft, changed = _loud(what, value, [dict(r=70001.3, z=3.0, harms=[(0.12, 0.0)] * 4)],
+                         PLACES[:1] if numharm == 32 else PLACES)
+    obs = ablib.obs_init(ablib.make_params(1 << 18, DT, fft.size, zmax=zmax, wmax=wmax, numharm=numharm, sigma=1.0))
+    whole = _hit_arrays(ctx, obs, fft)
+    cuts = np.array(list(obs.powcut), np.float64)
+    blocks = _clean_blocks(obs, changed, ablib.bank_geometry(obs))
+    assert len(blocks) > 8
+    for b in blocks:
+        key, blk, st, pw = _hit_arrays(ctx, obs, fft, b, 1)
+        wkey, wst, wpw = (whole[i][whole[1] == b] for i in (0, 2, 3))
+        # missing from one side only within 1e-5 of the cut
+        for k, s, p, other in ((key, st, pw, wkey), (wkey, wst, wpw, key)):
+            lone = ~np.isin(k, other)
+            assert np.all(np.abs(p[lone] - cuts[s[lone]]) <= 1e-5 * cuts[s[lone]]), (b, int(lone.sum()))
+        _, i, j = np.intersect1d(key, wkey, return_indices=True)
+        assert np.all(np.abs(pw[i] - wpw[j]) <= 1e-5 * pw[i]), b
+
+
+@pytest.mark.parametrize("what,value", LOUD)
+@pytest.mark.parametrize("zmax", [0, 50, 200])
+def test_loud_and_quiet_blocks_in_the_plane(ctx, ablib, what, value, zmax):
+    """The same for the in-memory plane: the rows of such a block are those of the standard mode's block alone."""
+    fft, changed = _loud(what, value, [])
+    kw = dict(zmax=zmax, numharm=1)
+    obs = ablib.obs_init(ablib.make_params(1 << 18, DT, fft.size, wmax=None, **kw))
+    std = ablib.obs_init(ablib.make_params(1 << 18, DT, fft.size, wmax=0, **kw))
+    assert obs.inmem and not std.inmem
+    clean = _clean_blocks(std, changed, ablib.bank_geometry(std))
+    near = [b for b in clean if {b - 2, b - 1, b + 1, b + 2} - set(clean)]
+    assert len(near) > 8
+    for b in near:
+        got, want = ctx.block_stage_sums(obs, fft, b)[0], ctx.block_stage_sums(std, fft, b)[0]
+        assert np.all(np.abs(got - want) <= 1e-5 * (want + 1.0)), b
