@@ -24,6 +24,7 @@
 // their segments are cut from one block's window, periodic as in the
 // reference's circular correlation.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 
 #include "ab_fft.cuh"
@@ -395,7 +396,8 @@ __device__ __forceinline__ void corr_tile(const SegGroup &g, const ab_bank &b, c
     for (int j = threadIdx.x; j < nj; j += blockDim.x) {
         const int tc0 = (int) (c[j].c0 - q) + 2 * g.hw;
         const int lo = max(tc0, 2 * g.hw), hi = min(tc0 + c[j].lim, 2 * g.hw + g.V);
-        // element of this block's transform column 0, from the first block's
+        // element of this block's transform column 0, from the first block's (in
+        // 32 bits: launch_corr_seg)
         const long long off = sc.inmem ? c[j].c0 - c[0].c0 - tc0 : (long long) j * plane_per_block - tc0;
         const double r = nm[j] / ref;
         m.blk[j] = make_int4(lo, max(hi - lo, 0), (int) off,
@@ -588,6 +590,8 @@ cudaError_t launch_corr_seg(const ab_bank *banks_dev, const SearchConsts &sc, co
                             const SegUnit *units, float *planes, long long plane_per_block, cudaStream_t st)
 {
     if (nctas <= 0) return cudaSuccess;
+    // corr_tile's offsets between blocks (ab_batch_blocks keeps to this)
+    if (!sc.inmem && bb.nblk > 1 && bb.nblk * plane_per_block > INT_MAX) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_corr_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) SEG_SMEM);
     if (e != cudaSuccess) return e;
     k_corr_seg<<<(unsigned) nctas, 32 * SEG_WARPS, SEG_SMEM, st>>>(banks_dev, sc, bb, groups, ngroups, cols, norms,

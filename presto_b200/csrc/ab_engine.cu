@@ -464,6 +464,25 @@ static SegPlan build_seg_plan(ab_ctx *ctx, const ab_obs *obs, const double *star
     return p;
 }
 
+// Bytes on the device that a block of a batch takes beside its planes: its
+// share of the segments' spectra, or (tensor-core path, banks correlated by
+// blocks' own data) its normalised data.
+static long long batch_bytes(const ab_ctx *ctx, bool tcp)
+{
+    const ab_bankset &bs = ctx->bs;
+    const long long data = bs.dtime_per_block * (long long) sizeof(float2);
+    if (tcp) return data;
+    long long n = 0;
+    bool own = false;
+    for (const ab_ctx::SegClass &c : ctx->cur_bank->classes) {
+        const ab_bank &b = bs.b[c.bank];
+        const long long V = 2 * AB_SEG_BINS - 4 * c.hw, bytes = AB_SEG_BINS * (long long) sizeof(float2);
+        own |= b.own_data != 0;
+        n += b.own_data ? (b.numrs_max + V - 1) / V * bytes : b.numrs_max * bytes / V;
+    }
+    return n + (own ? data : 0);
+}
+
 // Data spectra and correlation of one batch of blocks [0, bb.nblk) (bb.npre0 of
 // them main-loop blocks, the rest pre-pass blocks): planes of the standard
 // mode, or the in-memory plane.
@@ -991,14 +1010,7 @@ static int search_core(ab_ctx *ctx, const ab_obs *obs, const float2 *dfft, long 
         rc = ensure_tc(ctx);
         if (rc) return rc;
     }
-    const size_t per_block = (size_t) bs.plane_per_block * sizeof(float) +
-                             (size_t) bs.dtime_per_block * sizeof(float2);
-    long long B = (long long) (ctx->scratch_budget / std::max<size_t>(per_block, 1));
-    if (B < 1) B = 1;
-    if (B > 512) B = 512;
-    // several batches per search let the replay overlap the device work
-    if (count >= 8 && B > (count + 7) / 8) B = (count + 7) / 8;
-    if (B > count) B = std::max<long long>(count, 1);
+    const long long B = ab_batch_blocks(count, bs.plane_per_block, batch_bytes(ctx, tcp), ctx->scratch_budget);
     CK(ctx->planes.ensure((size_t) B * bs.plane_per_block));
     std::vector<TcItem> tfull, ttail;
     long long rem = count % B;

@@ -320,6 +320,19 @@ void ab_preblock_starts(const ab_obs *obs, double *out, long long n)
     for (long long i = 0; i < n; i++, startr += obs->rstep) out[i] = startr;
 }
 
+long long ab_batch_blocks(long long count, long long plane_floats, long long other_bytes, size_t budget)
+{
+    const long long per = plane_floats * (long long) sizeof(float) + other_bytes;
+    long long b = per > 0 ? (long long) (budget / (size_t) per) : 512;
+    if (b > 512) b = 512;
+    if (plane_floats > 0 && b > INT_MAX / plane_floats) b = INT_MAX / plane_floats;
+    if (count >= 8 && b > (count + 7) / 8) b = (count + 7) / 8;
+    if (b > count) b = count;
+    if (b < 1) return 1;
+    const long long batches = (count + b - 1) / b;
+    return batches > 0 ? (count + batches - 1) / batches : 1;
+}
+
 static int calc_fftlen(int numharm, int harmnum, int zmax, int wmax, const ab_obs *obs)
 {                                                      /* src/accel_utils.c:137-150 */
     double f = (double) harmnum / (double) numharm;

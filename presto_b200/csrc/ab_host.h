@@ -67,6 +67,13 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
 long long ab_num_blocks(const ab_obs *obs);
 long long ab_num_preblocks(const ab_obs *obs);
 
+/* Blocks of one batch of a standard search over count blocks, each with
+ * plane_floats floats of planes and other_bytes more on the device: what
+ * budget bytes hold, at most 512 and, so that the replay overlaps the device
+ * work, an eighth of the blocks; the batches of about one size.  Elements of a
+ * batch's planes are counted in 32 bits (a block's offset in ab_corr.cu). */
+long long ab_batch_blocks(long long count, long long plane_floats, long long other_bytes, size_t budget);
+
 int  ab_w_resp_halfwidth(double z, double w);
 int  ab_dered_plan(long long numbins, int startwidth, int endwidth, double endfreq, double T,
                    int *blocks, long long maxblocks, long long *nblocks);

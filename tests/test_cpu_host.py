@@ -184,3 +184,26 @@ def test_candlist_worklog_lines_for_added_candidates_only():
     assert [c[3] for c in lst.get()] == [1007.5, 3000.25]
     with pytest.raises(pb.AccelError):
         lst.set_worklog(True, 0.0)
+
+
+@pytest.mark.parametrize("count", [0, 1, 7, 8, 100, 3090, 20000])
+@pytest.mark.parametrize("plane", [43, 3372, 38_000_000 // 4, 263_000_000, 300_000_000, 3_000_000_000])
+@pytest.mark.parametrize("other", [0, 8192, 1 << 20])
+@pytest.mark.parametrize("budget", [1 << 20, 1 << 30, 8 << 30, 64 << 30])
+def test_batch_blocks(ablib, count, plane, other, budget):
+    """A batch's planes and segment spectra stay within the budget and its planes within 32-bit element
+    offsets (9 blocks of 263 million floats, a zmax 300, wmax 600 search, fit 16 GB but not those), unless a single
+    block does not; batches of one size that cover the blocks in no more turns than the largest would."""
+    import ctypes as C
+
+    f = ablib.lib().ab_batch_blocks
+    f.argtypes = [C.c_longlong, C.c_longlong, C.c_longlong, C.c_size_t]
+    f.restype = C.c_longlong
+    b = f(count, plane, other, budget)
+    assert 1 <= b <= max(1, min(512, count))
+    if b > 1:
+        assert b * (4 * plane + other) <= budget and b * plane < 1 << 31
+        assert count < 8 or b <= (count + 7) // 8
+    most = max(1, min(512, budget // (4 * plane + other), (2 ** 31 - 1) // plane, count if count < 8 else (count + 7) // 8))
+    assert -(-count // b) == -(-count // most)
+    assert count == 0 or count - (-(-count // b) - 1) * b > 0
