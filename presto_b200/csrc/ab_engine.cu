@@ -1399,7 +1399,7 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
             CK(cudaGetLastError());
         }
         char msg[256] = {0};
-        const size_t budget = std::min<size_t>(ctx->scratch_budget, 1ull << 30);
+        const size_t budget = std::min<size_t>(ctx->scratch_budget, RZW_RESP);
         // candidates in groups of at most 4096 harmonics bound each plan's host
         // memory (about 7000 volume outputs per harmonic)
         for (long long c0 = 0; c0 < n;) {
@@ -1412,10 +1412,11 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
                      : rzw_optimize_each(dfft, obs->numbins, obs->lobin, cands + c0, c1 - c0, out + c0,
                                          ctx->tw_rzw.p, budget, ctx->stream, ctx->rzw_work, msg, sizeof msg,
                                          &ctx->launches);
-            if (rc) return fail(ctx, rc, "%s", msg);
+            if (rc) break;
             c0 = c1;
         }
-        return AB_OK;
+        if (ctx->rzw_work.bytes() > std::min<size_t>(ctx->scratch_budget, RZW_KEEP)) ctx->rzw_work.release();
+        return rc ? fail(ctx, rc, "%s", msg) : AB_OK;
     }
     // -noharmpolish (src/accel_utils.c:585-611): max_rz_arr for each harmonic
     // on its own at (r h, z h); results gathered back per candidate below
@@ -1753,6 +1754,7 @@ int ab_ctx_set_hbm_budget(ab_ctx *ctx, size_t bytes)
     if (!ctx || bytes == 0) return AB_ERR_ARG;
     ctx->hbm_budget = bytes;
     ctx->scratch_budget = std::min<size_t>(8ull << 30, bytes / 4);
+    if (use_device(ctx) == AB_OK) ctx->rzw_work.release();      // allocated anew within the new budget
     return AB_OK;
 }
 

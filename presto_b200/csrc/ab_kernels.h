@@ -231,14 +231,20 @@ struct DevMem {
 };
 // The jobs', responses' and outputs' memory, kept by the context between calls
 // (48 candidates: 7.7 ms; 10.0 and at times 20 with an
-// allocation on each call).
+// allocation on each call) as long as it is at most RZW_KEEP bytes.
 struct RzwWork {
     DevMem jobs, resp, acc, js, amp, small;
+    size_t bytes() const { return jobs.n + resp.n + acc.n + js.n + amp.n + small.n; }
     void release()
     {
         for (DevMem *m : {&jobs, &resp, &acc, &js, &amp, &small}) m->release();
     }
 };
+constexpr size_t RZW_KEEP = 256ull << 20;
+// Responses of one launch: what stays in L2 until its correlations read it.
+// 48 candidates of a zmax = 200, wmax = 300 search, 1 GB of responses: 5.65 ms
+// in one launch, 5.53 at 256 MB, 5.47 at 128 and 64, 5.66 at 32.
+constexpr size_t RZW_RESP = 128ull << 20;
 // max_rzw_arr_harmonics for every candidate (host planning + the two
 // kernels above): data is the device spectrum of numdata bins, tw the FP64
 // table exp(-2 pi i m / 2^RZW_NMAX_LOG2), budget the response scratch per

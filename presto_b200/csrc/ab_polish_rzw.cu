@@ -589,8 +589,11 @@ cudaError_t run_plan(Plan &plan, const float2 *data, const double2 *tw, size_t b
     if (e == cudaSuccess && !plan.js.empty())
         e = cudaMemcpyAsync(dj.p, plan.js.data(), sizeof(long long) * plan.js.size(),
                             cudaMemcpyHostToDevice, st);
-    size_t i = 0;
-    while (e == cudaSuccess && i < plan.jobs.size()) {
+    // the chunks first, so that the scratch is allocated once
+    std::vector<size_t> ends;
+    long long rmax = 0, amax = 0;
+    size_t jmax = 0;
+    for (size_t i = 0; i < plan.jobs.size();) {
         const size_t j0 = i;
         long long roff = 0, aoff = 0;
         while (i < plan.jobs.size()) {
@@ -604,14 +607,20 @@ cudaError_t run_plan(Plan &plan, const float2 *data, const double2 *tw, size_t b
             aoff += na;
             i++;
         }
-        e = djobs.ensure(sizeof(RzwJob) * (i - j0));
-        if (e == cudaSuccess) e = dresp.ensure(sizeof(float2) * (size_t) roff);
-        if (e == cudaSuccess) e = dacc.ensure(sizeof(double2) * (size_t) aoff);
+        rmax = std::max(rmax, roff);
+        amax = std::max(amax, aoff);
+        jmax = std::max(jmax, i - j0);
+        ends.push_back(i);
+    }
+    if (e == cudaSuccess) e = djobs.ensure(sizeof(RzwJob) * jmax);
+    if (e == cudaSuccess) e = dresp.ensure(sizeof(float2) * (size_t) rmax);
+    if (e == cudaSuccess) e = dacc.ensure(sizeof(double2) * (size_t) amax);
+    size_t j0 = 0;
+    for (size_t k = 0; k < ends.size() && e == cudaSuccess; j0 = ends[k++]) {
+        const size_t nj = ends[k] - j0;
+        e = cudaMemcpyAsync(djobs.p, plan.jobs.data() + j0, sizeof(RzwJob) * nj, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(djobs.p, plan.jobs.data() + j0, sizeof(RzwJob) * (i - j0),
-                                cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess)
-            e = launch_rzw_jobs((const RzwJob *) djobs.p, (int) (i - j0), data, plan.numdata, tw,
+            e = launch_rzw_jobs((const RzwJob *) djobs.p, (int) nj, data, plan.numdata, tw,
                                 (float2 *) dresp.p, (double2 *) dacc.p, (const long long *) dj.p,
                                 (float2 *) damp.p, st);
         if (e == cudaSuccess) ++*launches;

@@ -154,3 +154,29 @@ def test_device_rzw_chirp_lengths(ctx, ablib, oracle, jerk_case, z, w):
     # to float on both sides
     assert np.allclose(dev[0]["pows"], orc[0]["pows"], rtol=1e-4)
     assert np.allclose(dev[0]["derivs"][:, 6], orc[0]["derivs"][:, 6], rtol=1e-4)
+
+
+def test_polish_scratch_is_bounded(ablib, jerk_case):
+    """What a context keeps of a polishing's scratch between calls is at most 256 MB, and given back when the budget
+    is set (measured in whole 2 MB pages of several allocations: 24 MB of slack)."""
+    import torch
+
+    ft, cands = jerk_case
+    obs = _obs(ablib, ft.size, zmax=200, numharm=8)
+    rng = np.random.default_rng(1)
+    many = [(0.0, 0.0, 8, r, 0.0, 0.0) for r in rng.uniform(2000.0, 0.05 * ft.size, 48)]
+    c = ablib.Context(0)
+    c.optimize_cands(obs, ft, [(0.0, 0.0, 1, 5000.0, 0.0, 0.0)])       # tables, the spectrum and small scratch
+    assert c.L.ab_ctx_set_hbm_budget(c.ptr, 32 << 30) == 0
+    free0 = torch.cuda.mem_get_info()[0]
+    a = c.optimize_cands(obs, ft, many)
+    assert free0 - torch.cuda.mem_get_info()[0] <= (256 + 24) << 20
+    assert c.L.ab_ctx_set_hbm_budget(c.ptr, 64 << 20) == 0              # 16 MB of scratch
+    assert free0 - torch.cuda.mem_get_info()[0] <= 24 << 20
+    b = c.optimize_cands(obs, ft, many)
+    assert free0 - torch.cuda.mem_get_info()[0] <= (16 + 24) << 20
+    c.close()
+    for x, y in zip(a, b):                                             # and the launches' sizes change nothing
+        for k in ("pows", "hirs", "hizs", "hiws", "derivs"):
+            np.testing.assert_array_equal(x[k], y[k])
+
