@@ -2240,6 +2240,30 @@ int ab_bank_kernel(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int
     return AB_OK;
 }
 
+int ab_seg_template(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int wi, int zi, ab_fcomplex *out)
+{
+    if (!ctx || !obs || !out) return AB_ERR_ARG;
+    int rc = use_device(ctx);
+    if (rc) return rc;
+    rc = ensure_banks(ctx, obs);
+    if (rc) return rc;
+    const int k = find_bank(ctx->bs, numharm, harmnum);
+    if (k < 0) return fail(ctx, AB_ERR_ARG, "no bank %d/%d", harmnum, numharm);
+    const ab_bank &b = ctx->bs.b[k];
+    if (wi < 0 || wi >= b.nw || zi < 0 || zi >= b.nz) return fail(ctx, AB_ERR_ARG, "template index");
+    std::vector<int> perm((size_t) b.ntmpl);
+    CK(cudaMemcpyAsync(perm.data(), ctx->cur_bank->perm.p + b.perm_off, sizeof(int) * perm.size(),
+                       cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    const long long at = std::find(perm.begin(), perm.end(), wi * b.nz + zi) - perm.begin();
+    if (at == b.ntmpl) return fail(ctx, AB_ERR_STATE, "template %d not in the order", wi * b.nz + zi);
+    CK(cudaMemcpyAsync(out, ctx->cur_bank->tmpl.p + b.seg_tmpl_off + at * 2 * AB_SEG_BINS,
+                       sizeof(float2) * 2 * AB_SEG_BINS, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    harvest(ctx);
+    return AB_OK;
+}
+
 int ab_ctx_set_profiling(ab_ctx *ctx, int on)
 {
     if (!ctx) return AB_ERR_ARG;

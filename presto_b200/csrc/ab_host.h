@@ -79,6 +79,10 @@ int  ab_dered_plan(long long numbins, int startwidth, int endwidth, double endfr
                    int *blocks, long long maxblocks, long long *nblocks);
 int  ab_dered_runs(long long numbins, int startwidth, int endwidth, double endfreq, double T, int *runs,
                    int maxruns, int *nruns, long long *nblocks, int *maxlen);
+/* For the tests: the template (w index wi, z index zi) of bank (numharm,
+ * harmnum) as the searches multiply with it, 2 x 1024 points in ab_corr.cu's
+ * order. */
+int  ab_seg_template(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int wi, int zi, ab_fcomplex *out);
 int  ab_next_good_fftlen(int n);
 int  ab_fftlen_from_kernwidth(int kw);
 

@@ -31,7 +31,9 @@ def _same(one, whole, obs, block):
 @pytest.mark.parametrize("N,zmax,wmax,numharm,kw", [
     (1 << 18, 0, 0, 32, {}),                    # one template a bank; 46 blocks to a segment of the narrowest
     (1 << 18, 50, 0, 32, {}),
-    (1 << 19, 690, 0, 8, {}),                   # the widest templates, segments of 448 columns
+    (1 << 19, 690, 0, 8, {}),                   # wide templates, segments of 468 columns
+    (1 << 19, 730, 0, 8, {}),                   # the widest accepted (half width 417), of 380
+    (1 << 18, 730, 0, 1, dict(locpow=True)),
     (300000, 200, 0, 16, {}),
     (1 << 18, 100, 200, 16, {}),                # a bank whose reference transform wraps
     (1 << 18, 60, 100, 8, dict(locpow=True)),   # every block's own data

@@ -94,11 +94,20 @@ def test_responses_match_reference_build(ctx, oracle, kind, nb, z, w):
     assert np.max(np.abs(dev - want)) <= 2e-6 * np.max(np.abs(want))
 
 
+def _placed(oracle, L, numkern, z, w):
+    """The oracle's response with its centre at index 0 of L points (place_complex_kernel), transformed in FP64."""
+    resp = oracle.response("w" if w != 0 else "z", 2, numkern, z=z, w=w)
+    placed = np.zeros(L, np.complex128)
+    half = numkern // 2
+    placed[:half] = resp[half:]
+    placed[L - half:] = resp[:half]
+    return np.fft.fft(placed)
+
+
 def test_fundamental_templates_match_oracle(ctx, oracle, ablib, case):
-    """Device templates against the oracle's: at the reference's fftlen when
-    the device uses it, else the oracle's response placed (centre at index 0,
-    place_complex_kernel) and transformed in FP64 at the device length (a
-    superblock transform serves several blocks)."""
+    """ab_bank_kernel's templates (generated on demand) against the oracle's: at the reference's
+    fftlen when the device uses it, else the oracle's response placed (centre at index 0,
+    place_complex_kernel) and transformed in FP64 at the device length."""
     obs, oobs = case["obs"], case["oobs"]
     bank = oracle.Bank(oobs, 1, 1)
     hwf = ablib.lib().ab_w_resp_halfwidth
@@ -109,14 +118,36 @@ def test_fundamental_templates_match_oracle(ctx, oracle, ablib, case):
                 orc = bank.kernel(wi, zi)
             else:
                 z, w = -bank.zmax + 2.0 * zi, -bank.wmax + 20.0 * wi
-                numkern = 4 * hwf(z, w)
-                resp = oracle.response("w" if w != 0 else "z", 2, numkern, z=z, w=w)
-                placed = np.zeros(dev.size, np.complex128)
-                half = numkern // 2
-                placed[:half] = resp[half:]
-                placed[dev.size - half:] = resp[:half]
-                orc = np.fft.fft(placed)
+                orc = _placed(oracle, dev.size, 4 * hwf(z, w), z, w)
             assert np.max(np.abs(dev - orc)) <= 2e-6 * np.max(np.abs(orc)), (wi, zi, dev.size)
+
+
+@pytest.mark.parametrize("zmax,wmax,numharm", [(0, 0, 1), (60, 0, 4), (200, 0, 16), (730, 0, 1), (100, 200, 2)])
+def test_segment_templates_match_oracle(ctx, oracle, ablib, zmax, wmax, numharm):
+    """The templates the searches multiply with, read back from where they lie by class: their lanes' order undone
+    and the transforms of the even and the odd taps put together again, they are the oracle's response placed on
+    2048 columns.  The narrowest and the widest class (730: the widest half width accepted), w banks.  Two FP32
+    roundings of values up to the largest, and the oracle's taps in FP32: 2e-6 as above."""
+    import ctypes as C
+
+    obs = ablib.obs_init(ablib.make_params(1 << 17, DT, 1 << 16, zmax=zmax, wmax=wmax, numharm=numharm))
+    hwf = ablib.lib().ab_w_resp_halfwidth
+    f = ctx.L.ab_seg_template
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]
+    i = np.arange(1024)
+    place = (i & ~63) + 2 * (i & 31) + ((i >> 5) & 1)
+    raw = np.zeros(2048, np.complex64)
+    for g in ablib.bank_geometry(obs):
+        zm, wm = g["nz"] - 1, 10 * (g["nw"] - 1)
+        for wi in sorted({0, g["nw"] // 2, g["nw"] - 1}):
+            for zi in sorted({0, 1 % g["nz"], g["nz"] // 3, g["nz"] // 2, g["nz"] - 1}):
+                assert f(ctx.ptr, C.byref(obs), g["numharm"], g["harmnum"], wi, zi, raw.ctypes.data) == 0
+                even = raw[:1024][place].astype(np.complex128)
+                odd = raw[1024:][place] * np.exp(1j * np.pi * i / 1024)
+                dev = np.concatenate([even + odd, even - odd])
+                z, w = -zm + 2.0 * zi, -wm + 20.0 * wi
+                orc = _placed(oracle, 2048, 4 * hwf(z, w), z, w)
+                assert np.max(np.abs(dev - orc)) <= 2e-6 * np.max(np.abs(orc)), (g, wi, zi)
 
 
 def _harmonics(obs):
@@ -402,9 +433,59 @@ def test_wrapping_bank_matches_oracle(ctx, ablib, oracle):
         assert ok, (b, worst)
 
 
+def test_8192_point_templates_and_planes(ablib, oracle):
+    """A cost table that makes 8192-point templates cheapest (the four-pass FFT, 512-thread CTAs): ab_bank_kernel's
+    templates and the planes that ab_fderivs_vol_noalloc makes with them match the oracle."""
+    import ctypes as C
+
+    import torch
+
+    c = CASES["std"]
+    fft = _spec(c["N"], c["seed"], c["pulsars"])
+    kw = dict(zmax=c["zmax"], wmax=c["wmax"], numharm=c["numharm"])
+    oobs = oracle.obs_init(oracle.make_params(c["N"], DT, fft.size, **kw))
+    hwf = ablib.lib().ab_w_resp_halfwidth
+    default = ablib.get_transform_costs()
+    table = list(default)
+    table[13] = default[12] * 1.5
+    ablib.set_transform_costs(table)
+    cx = ablib.Context(0)
+    try:
+        obs = ablib.obs_init(ablib.make_params(c["N"], DT, fft.size, **kw))
+        banks = [b for b in ablib.bank_geometry(obs) if b["L"] == 8192]
+        assert banks
+        dfft = torch.from_numpy(fft.view(np.float32).copy()).cuda()
+        for g in banks:
+            m, h = g["numharm"], g["harmnum"]
+            tmpl = np.stack([cx.bank_kernel(obs, m, h, 0, zi) for zi in range(g["nz"])])
+            assert tmpl.shape == (g["nz"], 8192)
+            for zi in (0, g["nz"] // 3, g["nz"] - 1):
+                z = 1.0 - g["nz"] + 2.0 * zi
+                orc = _placed(oracle, 8192, 4 * hwf(z, 0.0), z, 0.0)
+                assert np.max(np.abs(tmpl[zi] - orc)) <= 2e-6 * np.max(np.abs(orc)), (m, h, zi)
+            dtmpl = torch.from_numpy(tmpl.view(np.float32).copy()).cuda()
+            bank = oracle.Bank(oobs, m, h)
+            for k in (0, 9):
+                lo = obs.rlo + k * obs.rstep
+                ometa, orc, _, _ = oracle.subharm_fderivs_vol(oobs, fft, m, h, lo, lo + obs.rstep - 0.5, bank)
+                out = torch.full((orc.size,), -1.0, device="cuda")
+                meta = ablib.accel.FFDotPows()
+                torch.cuda.synchronize()
+                assert cx.L.ab_fderivs_vol_noalloc(C.byref(obs), m, h, lo, dfft.data_ptr(), dtmpl.data_ptr(), tmpl.size,
+                                                   out.data_ptr(), out.numel(), C.c_void_p(0), C.byref(meta)) == 0
+                torch.cuda.synchronize()
+                assert (meta.rlo, meta.numrs) == (ometa["rlo"], ometa["numrs"])
+                ok, worst = _close(out.cpu().numpy().reshape(orc.shape), orc)
+                assert ok, (m, h, k, worst)
+    finally:
+        ablib.set_transform_costs(default)
+        cx.close()
+
+
 def test_search_with_8192_point_transforms(ablib, oracle):
-    """A cost table that makes 8192-point superblock transforms cheapest (the
-    four-pass FFT, 512-thread CTAs): the search still matches the oracle."""
+    """A cost table that makes 8192-point templates cheapest changes what ab_bank_kernel and
+    ab_fderivs_vol_noalloc use (test_8192_point_templates_and_planes) and no search: it still matches the
+    oracle."""
     c = CASES["std"]
     fft = _spec(c["N"], c["seed"], c["pulsars"])
     kw = dict(zmax=c["zmax"], wmax=c["wmax"], numharm=c["numharm"])
