@@ -190,3 +190,39 @@ def test_loud_and_quiet_blocks_in_the_plane(ctx, ablib, what, value, zmax):
     for b in near:
         got, want = ctx.block_stage_sums(obs, fft, b)[0], ctx.block_stage_sums(std, fft, b)[0]
         assert np.all(np.abs(got - want) <= 1e-5 * (want + 1.0)), b
+
+
+def test_plane_of_more_than_2e31_columns(ctx, ablib):
+    """A forced in-memory search of more than 2^30 bins: columns past 2^31.  A line there and one at half its
+    frequency: the stage-0 power is the standard mode's, the stage-1 power the sum of the two lines' (powers of
+    single bins, FP32 roundings)."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB of device memory")
+    numbins, line = (1 << 30) + (1 << 15), (1 << 30) + 20000
+    fft = torch.empty(numbins, dtype=torch.complex64, device="cuda")
+    torch.view_as_real(fft).normal_(0.0, 0.5 ** 0.5, generator=torch.Generator(device="cuda").manual_seed(3))
+    fft[line], fft[line // 2] = 30.0, 20.0
+    torch.cuda.synchronize()
+    kw = dict(zmax=0, numharm=2, sigma=10.0, rlo=1.0, rhi=float(numbins - 1))
+    own = ablib.Context(0)
+    try:
+        got = {}
+        for name, more in (("plane", dict(inmem=True)), ("std", dict(wmax=0))):
+            obs = ablib.obs_init(ablib.make_params(2 * numbins, DT, numbins, **kw, **more))
+            assert obs.inmem == (name == "plane")
+            for bin in (line, line // 2):
+                block = int((bin - obs.rlo) // obs.rstep)
+                own.search(obs, None, first_block=block, max_blocks=1, device_ptr=fft.data_ptr())
+                blk, st, wi, zi, ri, pw = own.last_hits()
+                col = int(2 * (bin - (obs.rlo + block * obs.rstep)))
+                got[name, bin] = {int(s): float(p) for b, s, r, p in zip(blk, st, ri, pw) if b == block and r == col}
+        for bin in (line, line // 2):
+            assert abs(got["plane", bin][0] - got["std", bin][0]) <= 1e-5 * got["std", bin][0]
+        want = got["plane", line][0] + got["plane", line // 2][0]
+        assert abs(got["plane", line][1] - want) <= 1e-6 * want
+    finally:
+        own.close()
+        del fft
+        torch.cuda.empty_cache()
