@@ -26,6 +26,7 @@ using namespace ab;
 namespace {
 
 constexpr int kTwLog2 = 14;                 // FP64 twiddle table for FFTs up to 16384
+constexpr size_t kBankKeep = 256ull << 20;  // of ab_bank_kernel's templates
 constexpr int kNumKinds = 8;   // templates, prep, corr, harmsum (device); host setup, host replay,
                                // hit fetch; dedispersion (device)
 double now_ms()
@@ -122,6 +123,10 @@ struct ab_ctx {
     DevBuf<ab_polished> pol_out;
     DevBuf<double2> fresnel_tab;            // auxiliary Fresnel functions, acceleration polishing
     DevBuf<float2> resp;
+    // ab_bank_kernel: every template of the bank it was last asked for (a
+    // caller asks for them one by one), templates of wmax bk_w, zmax bk_z, length bk_L
+    DevBuf<float2> bank_tmpl;
+    int bk_z = -1, bk_w = -1, bk_L = 0;
 
     // spectrum, scratch, planes
     DevBuf<float2> fft;
@@ -1220,6 +1225,7 @@ void ab_ctx_destroy(ab_ctx *ctx)
     ctx->pol_in.release();
     ctx->pol_out.release();
     ctx->resp.release();
+    ctx->bank_tmpl.release();
     ctx->fft.release();
     ctx->xhat.release();
     ctx->planes.release();
@@ -1754,7 +1760,11 @@ int ab_ctx_set_hbm_budget(ab_ctx *ctx, size_t bytes)
     if (!ctx || bytes == 0) return AB_ERR_ARG;
     ctx->hbm_budget = bytes;
     ctx->scratch_budget = std::min<size_t>(8ull << 30, bytes / 4);
-    if (use_device(ctx) == AB_OK) ctx->rzw_work.release();      // allocated anew within the new budget
+    if (use_device(ctx) == AB_OK) {             // allocated anew when needed
+        ctx->rzw_work.release();
+        ctx->bank_tmpl.release();
+        ctx->bk_L = 0;
+    }
     return AB_OK;
 }
 
@@ -2229,12 +2239,28 @@ int ab_bank_kernel(ab_ctx *ctx, const ab_obs *obs, int numharm, int harmnum, int
     if (!out) return AB_OK;
     if (maxlen < b.L) return fail(ctx, AB_ERR_OVERFLOW, "need %d", b.L);
     if ((rc = ensure_tw64(ctx))) return rc;
-    CK(ctx->resp.ensure((size_t) b.L));
+    // the whole bank, kept for the next call, up to kBankKeep bytes; else the one template
     const int t = wi * b.nz + zi;
-    cudaError_t e = launch_templates(&b, &t, nullptr, 1, b.L, ctx->resp.p, ctx->tw64.p, kTwLog2, ctx->stream);
-    if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "template generation failed: %s", cudaGetErrorString(e));
-    ctx->launches++;
-    CK(cudaMemcpyAsync(out, ctx->resp.p, sizeof(float2) * b.L, cudaMemcpyDeviceToHost, ctx->stream));
+    const bool keep = (size_t) b.ntmpl * b.L * sizeof(float2) <= kBankKeep;
+    const bool have = keep && ctx->bk_z == b.zmax && ctx->bk_w == b.wmax && ctx->bk_L == b.L;
+    if (!have) {
+        std::vector<int> which(keep ? (size_t) b.ntmpl : 1);
+        for (size_t i = 0; i < which.size(); i++) which[i] = keep ? (int) i : t;
+        ctx->bk_L = 0;
+        CK(ctx->bank_tmpl.ensure(which.size() * (size_t) b.L));
+        cudaError_t e = launch_templates(&b, which.data(), nullptr, (int) which.size(), b.L, ctx->bank_tmpl.p,
+                                         ctx->tw64.p, kTwLog2, ctx->stream);
+        if (e != cudaSuccess)
+            return fail(ctx, AB_ERR_CUDA, "template generation failed: %s", cudaGetErrorString(e));
+        ctx->launches++;
+        if (keep) {
+            ctx->bk_z = b.zmax;
+            ctx->bk_w = b.wmax;
+            ctx->bk_L = b.L;
+        }
+    }
+    CK(cudaMemcpyAsync(out, ctx->bank_tmpl.p + (keep ? (size_t) t * b.L : 0), sizeof(float2) * b.L,
+                       cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     harvest(ctx);
     return AB_OK;

@@ -196,8 +196,8 @@ static int chirp_len(double z, double w, int numkern, int numbetween)
 }
 
 // n templates which[] of a bank (which_dev: the same on the device), as ab_corr.cu
-// reads them, one behind the other; or, which_dev null, the one template which[0]
-// as the transform of its taps placed on L columns.
+// reads them, one behind the other; or, which_dev null, the n templates from
+// which[0] on as the transforms of their taps placed on L columns.
 cudaError_t launch_templates(const ab_bank *b, const int *which, const int *which_dev, int n, int L, float2 *out,
                              const double2 *tw_all, int max_log2, cudaStream_t st)
 {
@@ -225,7 +225,7 @@ cudaError_t launch_templates(const ab_bank *b, const int *which, const int *whic
     const int chunk = 65535;
     for (int t0 = 0; t0 < n; t0 += chunk) {
         a.which = which_dev ? which_dev + t0 : nullptr;
-        a.t_base = which[0];
+        a.t_base = which[t0];
         a.out = which_dev ? out + (size_t) t0 * L : out - (size_t) which[0] * L;
         k_templates<<<n - t0 < chunk ? n - t0 : chunk, 256, smem, st>>>(a);
     }

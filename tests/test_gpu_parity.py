@@ -150,6 +150,32 @@ def test_segment_templates_match_oracle(ctx, oracle, ablib, zmax, wmax, numharm)
                 assert np.max(np.abs(dev - orc)) <= 2e-6 * np.max(np.abs(orc)), (g, wi, zi)
 
 
+def test_bank_kernel_over_banks_and_lengths(ctx, oracle, ablib):
+    """ab_bank_kernel keeps a bank's templates between calls: asked in turn for banks of two searches and under two
+    cost tables (two lengths of one bank), and after a new budget, each is the oracle's."""
+    hwf = ablib.lib().ab_w_resp_halfwidth
+    obs = [ablib.obs_init(ablib.make_params(1 << 17, DT, 1 << 16, zmax=z, wmax=w, numharm=2)) for z, w in ((60, 0), (20, 40))]
+    default = ablib.get_transform_costs()
+    table = list(default)
+    table[13] = default[12] * 1.5
+    lengths = set()
+    try:
+        for turn in range(3):
+            ablib.set_transform_costs(table if turn == 1 else default)
+            for o in obs:
+                for g in ablib.bank_geometry(o):
+                    for zi in (g["nz"] - 1, 2):
+                        dev = ctx.bank_kernel(o, g["numharm"], g["harmnum"], 0, zi)
+                        z, w = 1.0 - g["nz"] + 2.0 * zi, -10.0 * (g["nw"] - 1)
+                        orc = _placed(oracle, g["L"], 4 * hwf(z, w), z, w)
+                        assert np.max(np.abs(dev - orc)) <= 2e-6 * np.max(np.abs(orc)), (turn, g, zi)
+                        lengths.add((g["numharm"], g["nz"], g["nw"], g["L"]))
+            assert ctx.L.ab_ctx_set_hbm_budget(ctx.ptr, 32 << 30) == 0
+    finally:
+        ablib.set_transform_costs(default)
+    assert len(lengths) > 4
+
+
 def _harmonics(obs):
     hs = [(1, 1)]
     if not obs.inmem:
