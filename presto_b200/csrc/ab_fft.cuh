@@ -1,10 +1,10 @@
 // ab_fft.cuh -- shared-memory FFTs for sm_100a.
 //
-// FP32 complex FFT of power-of-two length L in [256, 4096], Stockham
+// FP32 complex FFT of power-of-two length L in [256, 8192], Stockham
 // auto-sort with radix-16 passes (plus one radix-2/4/8 pass), computed by a
 // "group" of NT = L/16 threads that each hold 16 points in registers in the
-// strided layout v[m] = x[t + NT*m].  A 256-thread CTA runs 4096/L groups
-// side by side; every group owns (L + L/16) float2 of padded shared memory.
+// strided layout v[m] = x[t + NT*m].  A CTA of 256 threads runs 4096/L groups
+// side by side (8192 points: one group of 512); every group owns (L + L/16) float2 of padded shared memory.
 // Twiddles depend only on the thread, so they are computed once (FP64
 // sincospi, rounded to FP32) and kept in registers across transforms.
 //

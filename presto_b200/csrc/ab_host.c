@@ -402,7 +402,7 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
                 pairs[n][0] = 1 << s; pairs[n][1] = h; n++;
             }
     long long nblocks = ab_num_blocks(obs), npre = ab_num_preblocks(obs);
-    long long tmpl = 0, plane = 0, xhat = 0, dtime = 0, seg = 0;
+    long long plane = 0, dtime = 0, seg = 0;
     int perm = 0;
     for (int i = 0; i < n; i++) {
         ab_bank *b = &bs->b[i];
@@ -501,21 +501,14 @@ int ab_bankset_init_tuned(const ab_obs *obs, const double *cost_by_log2L, ab_ban
         perm += b->ntmpl;
         b->L = L;
         b->log2L = twon_to_index(L);
-        b->tmpl_off = tmpl;
-        tmpl += (long long) b->ntmpl * L;
-        b->xhat_off = xhat;
-        xhat += L / 2;
         b->dtime_off = dtime;
         dtime += b->fftlen_ref / AB_NUMBETWEEN;
         b->plane_off = plane;
         plane += (long long) b->nw * b->nz * b->numrs_max;
     }
     bs->nbanks = n;
-    bs->tmpl_total = tmpl;
     bs->seg_tmpl_total = seg;
-    bs->perm_total = perm;
     bs->plane_per_block = plane;
-    bs->xhat_per_block = xhat;
     bs->dtime_per_block = dtime;
     return AB_OK;
 }

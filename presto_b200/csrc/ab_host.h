@@ -26,13 +26,11 @@ typedef struct {
                                      allocation-free entry point (power of two) */
     int hw0;                      /* kern[0][0].kern_half_width (binoffset) */
     int numrs_max;                /* largest numrs over all blocks (row stride) */
-    long long tmpl_off;           /* complex offset of the bank's templates of L points */
     long long seg_tmpl_off;       /* offset of its segment templates (ab_corr.cu) */
     int perm_off;                 /* offset of its templates in the order by half width */
     int own_data;                 /* correlated by each block's own window (the reference's
                                      transform wraps into valid cells, or -locpow) */
     long long plane_off;          /* float offset inside one block's plane scratch */
-    long long xhat_off;           /* complex offset inside one block's spectrum scratch */
     long long dtime_off;          /* complex offset of the block's normalised data
                                      (tensor-core correlation) */
     int sbm;                      /* blocks that the cost table would have share a
@@ -46,11 +44,8 @@ typedef struct {
 typedef struct {
     int nbanks;
     ab_bank b[AB_MAX_BANKS];
-    long long tmpl_total;         /* complex elements over all banks */
     long long seg_tmpl_total;     /* complex elements of the segment templates */
-    int perm_total;               /* templates over all banks */
     long long plane_per_block;    /* floats of plane scratch per block */
-    long long xhat_per_block;     /* complex elements of spectrum scratch per block */
     long long dtime_per_block;    /* complex elements of normalised data per block */
 } ab_bankset;
 
@@ -75,6 +70,8 @@ long long ab_num_preblocks(const ab_obs *obs);
 long long ab_batch_blocks(long long count, long long plane_floats, long long other_bytes, size_t budget);
 
 int  ab_w_resp_halfwidth(double z, double w);
+/* The block list of deredden, bin by bin as the reference steps; the engine
+ * works from ab_dered_runs, and the tests hold one against the other. */
 int  ab_dered_plan(long long numbins, int startwidth, int endwidth, double endfreq, double T,
                    int *blocks, long long maxblocks, long long *nblocks);
 int  ab_dered_runs(long long numbins, int startwidth, int endwidth, double endfreq, double T, int *runs,

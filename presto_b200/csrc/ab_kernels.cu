@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(FftShape<L>::CTA, FftShape<L>::MINB) k_corr(co
     // transform has exactly two exchanges (fewer barriers)
     float2 *sm = fsm + L / 2 + grp * SH::SMEM;
     float2 *sm2 = SH::DBUF ? fsm + L / 2 + (SH::G + grp) * SH::SMEM : nullptr;
-    const float2 *xsrc = xhat + (long long) it.bi * xhat_per_block + b.xhat_off;
+    const float2 *xsrc = xhat + (long long) it.bi * xhat_per_block;
     for (int i = threadIdx.x; i < L / 2; i += blockDim.x) xs[i] = xsrc[i];
     ab_hgeom g;
     block_geom(sc, b, bb.startr[it.bi], &g);
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(FftShape<L>::CTA, FftShape<L>::MINB) k_corr(co
         const bool valid = tl < it.t0 + it.nt;
         float2 v[16];
         if (valid) {
-            const float2 *kp = tmpl + b.tmpl_off + (long long) tl * L;
+            const float2 *kp = tmpl + (long long) tl * L;
 #pragma unroll
             for (int m = 0; m < 16; m++) {
                 int i = t + SH::NT * m;

@@ -174,9 +174,7 @@ extern "C" int ab_fderivs_vol_noalloc(const ab_obs *obs, int numharm, int harmnu
 
     // The caller's arrays: templates [nw][nz][L] at offset 0, powers
     // [nw][nz][numrs] (row stride numrs), data spectrum at scratch offset 0.
-    b.tmpl_off = 0;
     b.plane_off = 0;
-    b.xhat_off = 0;
     b.numrs_max = g.numrs;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     k_noalloc_setup<<<(nitems + 255) / 256, 256, 0, st>>>(b, fullrlo, b.ntmpl, tile, nitems,
