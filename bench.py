@@ -33,13 +33,14 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # DRAM bytes moved per byte of f-fdot planes, from one ncu capture of each
-# kernel at N=2^20: the correlation of the zmax=200 search read 0.031 GB and
-# wrote 0.799 GB for its plane of 0.843 GB (profiles/k_corr_seg_accelsearch_
-# zmax200_N2e20.md; the rest was still in L2); the harmonic sum of the zmax=600
-# numharm=16 search read 1.885 GB and wrote 0.005 GB for a batch's 1.87 GB
-# (profiles/k_harmsum_std5_accelsearch_zmax600_N2e20.md).  Both move bytes in
-# proportion to the planes, so full-size launches scale by their plane bytes.
-CORR_DRAM_PER_PLANE_BYTE = (0.031 + 0.799) / 0.843
+# kernel on the zmax=600 numharm=16 search at N=2^20 (a batch of 49 blocks,
+# 1.872 GB of planes).  The correlation writes every plane byte once (the part
+# still in L2 when a captured launch ends, 47 MB, is a fixed amount that the
+# next launch writes out) and read 0.151 GB of templates and spectra
+# (profiles/k_corr_seg_accelsearch_zmax600_N2e20.md): the read share of a
+# full-size launch is an estimate from that.  The harmonic sum read 1.885 GB and
+# wrote 0.005 GB (profiles/k_harmsum_std5_accelsearch_zmax600_N2e20.md).
+CORR_DRAM_PER_PLANE_BYTE = 1.0 + 0.151 / 1.872
 HARMSUM_DRAM_PER_PLANE_BYTE = (1.885 + 0.005) / 1.87
 
 WORKLOADS = {
@@ -383,9 +384,8 @@ def run_ours(args):
     # ---- roofline of the dominant kernel (correlation) ----
     corr_ms_per_search = kms[2] / args.steps
     harm_ms = kms[3] / args.steps
-    # DRAM traffic per launch, standard mode: each kernel's measured DRAM bytes
-    # per byte of f-fdot planes (one ncu capture each on the zmax=600 numharm=16
-    # search at N=2^20) times this search's plane bytes per launch
+    # DRAM traffic per launch, standard mode: each kernel's DRAM bytes per byte
+    # of f-fdot planes (above) times this search's plane bytes per launch
     corr_traffic = harm_traffic = None
     if not obs.inmem and not tc and kn[2] and kn[3]:
         planes = counts["harmsum_min_bytes"] * args.steps
@@ -416,8 +416,9 @@ def run_ours(args):
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak, "traffic": corr_traffic,
                 "traffic_unit": "DRAM bytes per launch (average over the search's correlation "
-                                "launches), scaled from profiles/k_corr_seg_accelsearch_zmax200"
-                                "_N2e20.md by plane bytes" if corr_traffic else None,
+                                "launches): plane bytes written once plus the read share of "
+                                "profiles/k_corr_seg_accelsearch_zmax600_N2e20.md, an estimate"
+                                if corr_traffic else None,
                 "flops_per_search": counts["corr_flops"],
                 "kernel_ms_per_search": corr_ms_per_search,
                 "peak_source": "measured in-run FP32 FMA loop (MEASURED_PEAKS.json "

@@ -107,6 +107,10 @@ int  ab_ctx_create(int device, ab_ctx **out);
 void ab_ctx_destroy(ab_ctx *ctx);
 const char *ab_ctx_last_error(const ab_ctx *ctx);
 void *ab_ctx_stream(ab_ctx *ctx);                 /* cudaStream_t of the context */
+/* Device memory the context plans for (0.85 of what is free when it is
+ * created): a quarter of it, at most 8 GiB, bounds a search batch's planes and
+ * the scratch that polishing keeps between calls.  Setting it gives that scratch
+ * and ab_bank_kernel's templates back. */
 int  ab_ctx_set_hbm_budget(ab_ctx *ctx, size_t bytes);
 
 /* Correlation path of the context's searches and drop-ins (replaces the
