@@ -1421,7 +1421,7 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
             if (rc) break;
             c0 = c1;
         }
-        if (ctx->rzw_work.bytes() > std::min<size_t>(ctx->scratch_budget, RZW_KEEP)) ctx->rzw_work.release();
+        if (ctx->rzw_work.bytes() > std::min<size_t>(ctx->scratch_budget, POLISH_KEEP)) ctx->rzw_work.release();
         return rc ? fail(ctx, rc, "%s", msg) : AB_OK;
     }
     // -noharmpolish (src/accel_utils.c:585-611): max_rz_arr for each harmonic
@@ -1464,6 +1464,11 @@ int ab_optimize_cands(ab_ctx *ctx, const ab_obs *obs, const ab_fcomplex *fft, in
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hout, dout.p, sizeof(ab_polished) * nin, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    // kept for the next call as long as they are small
+    if (din.n * sizeof(PolishIn) + dout.n * sizeof(ab_polished) > std::min<size_t>(ctx->scratch_budget, POLISH_KEEP)) {
+        din.release();
+        dout.release();
+    }
     if (e != cudaSuccess) return fail(ctx, AB_ERR_CUDA, "candidate polishing failed: %s", cudaGetErrorString(e));
     if (each) {
         for (long long k = 0; k < n; k++) {
@@ -1762,6 +1767,8 @@ int ab_ctx_set_hbm_budget(ab_ctx *ctx, size_t bytes)
     ctx->scratch_budget = std::min<size_t>(8ull << 30, bytes / 4);
     if (use_device(ctx) == AB_OK) {             // allocated anew when needed
         ctx->rzw_work.release();
+        ctx->pol_in.release();
+        ctx->pol_out.release();
         ctx->bank_tmpl.release();
         ctx->bk_L = 0;
     }

@@ -171,6 +171,8 @@ struct PolishIn {
     int numharm;
     int mode;                   // 0: max_rz_arr_harmonics, 1: max_rz_arr (one harmonic)
 };
+// Device memory of a polishing call that its context may keep for the next.
+constexpr size_t POLISH_KEEP = 256ull << 20;
 // fresnel_tab: fresnel_table's points on the device
 constexpr int POLISH_FRESNEL_TAB = 353;
 void fresnel_table(double2 *out);
@@ -231,7 +233,7 @@ struct DevMem {
 };
 // The jobs', responses' and outputs' memory, kept by the context between calls
 // (48 candidates: 7.7 ms; 10.0 and at times 20 with an
-// allocation on each call) as long as it is at most RZW_KEEP bytes.
+// allocation on each call) as long as it is at most POLISH_KEEP bytes.
 struct RzwWork {
     DevMem jobs, resp, acc, js, amp, small;
     size_t bytes() const { return jobs.n + resp.n + acc.n + js.n + amp.n + small.n; }
@@ -240,7 +242,6 @@ struct RzwWork {
         for (DevMem *m : {&jobs, &resp, &acc, &js, &amp, &small}) m->release();
     }
 };
-constexpr size_t RZW_KEEP = 256ull << 20;
 // Responses of one launch: what stays in L2 until its correlations read it.
 // 48 candidates of a zmax = 200, wmax = 300 search, 1 GB of responses: 5.65 ms
 // in one launch, 5.53 at 256 MB, 5.47 at 128 and 64, 5.66 at 32.

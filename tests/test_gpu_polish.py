@@ -12,6 +12,8 @@ optimizer battery and against the polishing oracle.
   powers within 1e-3 relative or 1e-6 of the peak power.
 * Candidates of a real search (cfg1 recipe at N = 2^19): the same bounds.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -140,3 +142,29 @@ def test_device_polish_teams(ctx, ablib, oracle):
             for k in range(len(base), n):
                 for key in ("pows", "hirs", "hizs"):
                     np.testing.assert_array_equal(dev[k][key], dev[k % len(base)][key])
+
+
+def test_polish_results_are_given_back(ctx, ablib):
+    """A list whose results take more than the context's scratch budget leaves none of them on the device (measured
+    in whole pages of two allocations), and short lists after it give what they gave before."""
+    import torch
+
+    ft = harmonic_signal(R_HARM, 5.0, 4, 1.0, 99)
+    obs = _obs(ablib, ft.size)
+    few = [(0.0, 0.0, 1, R_HARM + 0.1, 4.0, 0.0)] * 3
+    c = ablib.Context(0)
+    try:
+        want = c.optimize_cands(obs, ft, few)
+        size = ctypes.sizeof(ablib.accel.Polished)
+        assert c.L.ab_ctx_set_hbm_budget(c.ptr, 4 << 20) == 0                  # 1 MB of scratch
+        free0 = torch.cuda.mem_get_info()[0]
+        n = (48 << 20) // size
+        many = c.optimize_cands(obs, ft, [few[0]] * n)
+        assert free0 - torch.cuda.mem_get_info()[0] <= 8 << 20
+        for got in (c.optimize_cands(obs, ft, few), many[:3], many[-3:]):
+            for a, b in zip(got, want):
+                np.testing.assert_array_equal(a["pows"], b["pows"])
+                np.testing.assert_array_equal(a["hirs"], b["hirs"])
+    finally:
+        c.close()
+
